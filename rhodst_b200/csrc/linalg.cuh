@@ -6,8 +6,10 @@
 #pragma once
 
 #include <climits>
+#include <type_traits>
 
 #include "kernels.cuh"
+#include "rdst_records.h"
 
 namespace rdst {
 
@@ -202,25 +204,17 @@ struct IluDev {
     int mu_use;             // U slots the backward sweep applies (0: (D + L)^-1 of Gauss-Seidel)
     const int* lu_col;      // [fid] column of each factor slot (-1: empty)
     const int* lu_src;      // [fid] SELL flat slot of the same block in A
-    // task records of the bulk apply (null: not kept).  Each sweep's tasks
-    // (24 rows of one level, in the order the sweep takes them) are laid
-    // out one after the other in rec_f (forward) / rec_b (backward): a
-    // 96-byte header of 24 words (byte offset of the row's record from the
-    // task start | slot count << 24), then the row records: the columns of
-    // the row's L (U) slots, padded to 16 bytes, the blocks (entry 5i+j),
-    // and backward the pivot inverse, each record padded to 16 bytes.
-    // task_f/task_b: (offset in 16-byte units, bytes) per task; part_tf /
-    // part_tb: first task of each part.  The headers and columns are set
-    // once; k_ilu_pack writes the blocks at val_f/val_b (16-byte units) of
-    // every row after each factorisation.
+    // factor records of the apply (rdst_records.h; null: not kept): forward
+    // and backward, their groups, the first group of each part, and the tasks.
+    // Headers and columns are set once, the blocks after each factorisation.
     unsigned char* rec_f;
     unsigned char* rec_b;
-    const uint2* task_f;
-    const uint2* task_b;
-    const int* part_tf;
-    const int* part_tb;
-    const unsigned* val_f;
-    const unsigned* val_b;
+    const RecGroup* grp_f;
+    const RecGroup* grp_b;
+    const int* part_gf;
+    const int* part_gb;
+    const RecTask* task_f;
+    const RecTask* task_b;
     // the direct factorisation's addressing (null: gather + factor
     // instead).  Per update triple (tr_start ranges):
     // fr_trk: where U_kj is read, the flat SELL slot of A_kj (>= 0), factor
@@ -336,7 +330,6 @@ __global__ void __launch_bounds__(ILU_TPB) k_ilu_factor(SellMat<MT> A, MT* __res
 constexpr int ILU_APPLY_TPB = 128;
 constexpr int ILU_APPLY_MINB = 4;      // resident CTAs per SM the register budget is sized for
 constexpr int ILU_MAX_LV = 1023;       // level offsets staged in shared memory up to this many
-constexpr int ILU_LB_MAX = 1024;       // widest level the bulk apply's level buffers hold (2 x 40 KB)
 
 // One row task of a sweep: the factor row's columns, this lane's entries
 // of each slot, its pivot-inverse row (backward sweep) and the starting
@@ -466,198 +459,7 @@ __global__ void __launch_bounds__(ILU_APPLY_TPB, ILU_APPLY_MINB)
     }
 }
 
-// ---- ILU apply with the factor rows of each task brought in by bulk copies
-//
-// Same subdomains, levels and tasks as k_ilu_apply.  What differs is how a
-// task's data reaches the lanes, and the arithmetic (below): the task records
-// (IluDev::rec_f / rec_b, one contiguous byte range per task) are brought
-// in by a single cp.async.bulk (TMA) copy, issued by one thread, into a
-// shared-memory stage whose mbarrier counts the bytes; NS stages keep
-// NS - 1 tasks in flight ahead of the one being computed.  The copies run
-// in the async proxy (no register of the lanes waits on them), the lanes
-// read 16-byte-aligned records from shared memory, and the memory system
-// sees large contiguous requests.  The starting values y0 (b forward, the
-// forward result backward) come by per-lane cp.async.  With LB, the x
-// values of each level also go to one of two shared-memory level buffers
-// (level l to buffer l & 1, row r at r - first row of l, padded to 16
-// bytes for vector loads): the dependencies
-// of a row in the level the sweep took just before are read from there,
-// older ones from global memory.  In breadth-first order (rdst_order.h)
-// nearly all couplings join consecutive levels.
-//
-// A stage is refilled only after the barrier that ends the task that read
-// it.  Each mbarrier wait is bounded (2 s of globaltimer): on expiry the
-// CTA raises bit 2 of *flags (reported as a timeout by the host), waits,
-// again bounded, for its copies in flight and returns.
-__device__ __forceinline__ unsigned long long globaltimer_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// global -> shared bulk copy completing on an mbarrier (no multicast)
-__device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-// true once the phase of parity `parity` has completed; false after 2 s
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-    unsigned long long t0 = 0;
-    for (unsigned it = 0;; ++it) {
-        unsigned ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-        if ((it & 63) == 0) {
-            const unsigned long long now = globaltimer_ns();
-            if (it == 0) t0 = now;
-            else if (now - t0 > 2000000000ull) return false;
-        }
-    }
-}
-__device__ __forceinline__ void cpa8(unsigned dst, const void* src, bool ok) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(ok ? 8 : 0) : "memory");
-}
-__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-// Four warps a subdomain, five lanes a row (one per component), six rows a
-// warp: a task is up to 24 rows of one level.  The lanes multiply in CT,
-// the arithmetic of the factors' storage type: double for 8-byte factors,
-// float for 4- and 2-byte ones (the reduced-precision preconditioner
-// applies its FP32/BF16 factors in FP32; its input b and output x stay
-// FP64 vectors).  Each factor block's product with x_k is summed first
-// (the block-times-vector of the oracle's apply), then subtracted from y,
-// block by block in column order.
-constexpr int ILU_BULK_TPB = 128;
-constexpr int ILU_BULK_RPT = (ILU_BULK_TPB / 32) * 6;   // rows per task (24)
-constexpr int ILU_BULK_HDR = ILU_BULK_RPT * 4;           // task header bytes (96)
-
-__device__ __forceinline__ double to_ct(double v, double) { return v; }
-__device__ __forceinline__ float to_ct(float v, float) { return v; }
-__device__ __forceinline__ float to_ct(__nv_bfloat16 v, float) { return __bfloat162float(v); }
-__device__ __forceinline__ float to_ct(double v, float) { return (float)v; }
-// level-buffer row: five values padded to 16 bytes (6 doubles / 8 floats)
-template <typename CT> constexpr int lb_row() { return sizeof(CT) == 8 ? 6 : 8; }
-__device__ __forceinline__ void lb_load(const double* p, double (&o)[5]) {
-    const double2* q = reinterpret_cast<const double2*>(p);
-    const double2 a0 = q[0], a1 = q[1], a2 = q[2];
-    o[0] = a0.x; o[1] = a0.y; o[2] = a1.x; o[3] = a1.y; o[4] = a2.x;
-}
-__device__ __forceinline__ void lb_load(const float* p, float (&o)[5]) {
-    const float4* q = reinterpret_cast<const float4*>(p);
-    const float4 a0 = q[0], a1 = q[1];
-    o[0] = a0.x; o[1] = a0.y; o[2] = a0.z; o[3] = a0.w; o[4] = a1.x;
-}
-
-// stages the bulk apply keeps (NS - 1 tasks in flight)
-template <typename MT>
-constexpr int ilu_bulk_stages() { return 3; }
 constexpr int ILU_FR_MAXQ = 8;      // lower slots per row the direct factorisation takes
-
-// factor blocks -> task records (after each factorisation): one CTA per 32
-// rows.  The blocks the chunk's rows use are staged through shared memory
-// (loads of the sliced stores contiguous over the rows): the L blocks of the
-// factor store, the U blocks of A (of the factor store for rows whose own
-// blocks take updates), the pivot inverses; then the rows' value areas are
-// written as whole 16-byte chunks, the threads on consecutive chunks of
-// consecutive rows.
-template <typename MT>
-__host__ __device__ constexpr int ilu_pack_tile() { return 25 * 33; }
-
-template <typename MT>
-__global__ void __launch_bounds__(256) k_ilu_pack(int N, SellMat<MT> A, const MT* __restrict__ lu,
-                                                  const MT* __restrict__ dinv, IluDev P) {
-    extern __shared__ __align__(16) unsigned char s_pack[];
-    MT* tiles = reinterpret_cast<MT*>(s_pack);        // [slots][25][33]
-    __shared__ int s_n[2][32], s_pre[33], s_max[2], s_upd[32];
-    __shared__ int s_src[ILU_FR_MAXQ * 2][32];
-    constexpr int TL = ilu_pack_tile<MT>();
-    constexpr int EPC = 16 / (int)sizeof(MT);
-    const int chunk = blockIdx.x, r0 = chunk * 32;
-    const int ms = P.ml + P.mu;
-    if (threadIdx.x < 32) {
-        const int r = r0 + threadIdx.x;
-        const int nlu = r < N ? P.nlu[r] : 0;
-        int nl = nlu & 255, nu = P.mu_use ? (nlu >> 8) & 255 : 0;
-        s_n[0][threadIdx.x] = r < N ? nl : -1;
-        s_n[1][threadIdx.x] = r < N ? nu : -1;
-        s_upd[threadIdx.x] = (nlu >> 16) & 1;
-        for (int o = 16; o > 0; o >>= 1) {
-            nl = max(nl, __shfl_xor_sync(0xffffffffu, nl, o));
-            nu = max(nu, __shfl_xor_sync(0xffffffffu, nu, o));
-        }
-        if (threadIdx.x == 0) { s_max[0] = nl; s_max[1] = nu; }
-    }
-    __syncthreads();
-    // sources of the U blocks: flat SELL slot of A, -1 - fid of the factor
-    // store (rows whose own blocks take updates), or -2 (zero)
-    for (int i = threadIdx.x; i < s_max[1] * 32; i += blockDim.x) {
-        const int u = i >> 5, j = i & 31;
-        const int f = (chunk * ms + P.ml + u) * 32 + j;
-        const int src = r0 + j < N ? P.lu_src[f] : -2;
-        s_src[u][j] = s_upd[j] ? -1 - f : (src >= 0 ? src : -2);     // -2: empty slot or fill, zero
-    }
-    for (int side = 0; side < 2; ++side) {
-        const int nmax = s_max[side];
-        const int ntile = side == 0 ? nmax : nmax + 1;     // backward: U slots, then the pivot inverses
-        __syncthreads();
-        for (int t = 0; t < ntile; ++t) {
-            for (int i = threadIdx.x; i < 800; i += blockDim.x) {
-                const int e = i >> 5, j = i & 31;
-                MT v;
-                if (side == 0) v = lu[(size_t)(chunk * ms + t) * 800 + i];
-                else if (t == nmax) v = dinv[(size_t)chunk * 800 + i];
-                else {
-                    const int src = s_src[t][j];
-                    v = src >= 0 ? A.val[flat_e(src, e)] : (src == -2 ? mt_zero<MT>() : lu[flat_e(-1 - src, e)]);
-                }
-                tiles[t * TL + e * 33 + j] = v;
-            }
-        }
-        // chunks per row, prefix
-        if (threadIdx.x < 32) {
-            const int n = s_n[side][threadIdx.x];
-            const int nel = n < 0 ? 0 : 25 * (side == 0 ? n : n + 1);
-            int c = (nel + EPC - 1) / EPC, x = c;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, x, o);
-                if ((int)threadIdx.x >= o) x += y;
-            }
-            s_pre[threadIdx.x + 1] = x;
-            if (threadIdx.x == 0) s_pre[0] = 0;
-        }
-        __syncthreads();
-        const int total = s_pre[32];
-        for (int g = threadIdx.x; g < total; g += blockDim.x) {
-            int j = 0;
-#pragma unroll
-            for (int st = 16; st > 0; st >>= 1)
-                if (s_pre[j + st] <= g) j += st;
-            const int ch = g - s_pre[j];
-            const int n = s_n[side][j];
-            const int nel = 25 * (side == 0 ? n : n + 1);
-            alignas(16) MT v[EPC];
-#pragma unroll
-            for (int k = 0; k < EPC; ++k) {
-                const int e = ch * EPC + k;
-                const int q = e / 25, ee = e - 25 * q;
-                const int t = (side == 1 && q == n) ? nmax : q;
-                v[k] = e < nel ? tiles[t * TL + ee * 33 + j] : mt_zero<MT>();
-            }
-            uint4* dst = reinterpret_cast<uint4*>(side == 0 ? P.rec_f + (size_t)P.val_f[r0 + j] * 16
-                                                            : P.rec_b + (size_t)P.val_b[r0 + j] * 16);
-            dst[ch] = *reinterpret_cast<const uint4*>(v);
-        }
-    }
-}
 
 // one IKJ update triple of row r: U_kj read from A (us >= 0), the sliced
 // factor store (fid -us - 1) or zero (INT_MIN); L_rk U_kj taken from the
@@ -801,227 +603,503 @@ __global__ void __launch_bounds__(32) k_ilu_factor_direct(SellMat<MT> A, MT* __r
     }
 }
 
-// The apply is specialised by warp: warps 0-3 compute (five lanes a row,
-// six rows a warp), a fifth warp produces.  For each task the producer
-// walks the cursor, publishes the task's rows and level buffers in s_q,
-// starts the bulk copy of its record into a stage and the copies of its y0
-// into the y0 slot, and waits for the latter before the barrier that ends
-// the task being computed; the compute warps only wait for the stage,
-// multiply and store.  All 160 threads take the same barriers.
-constexpr int ILU_BULK_THREADS = ILU_BULK_TPB + 32;
-
-template <typename MT, int NS, bool LB>
-__global__ void __launch_bounds__(ILU_BULK_THREADS, 6)
-    k_ilu_apply_bulk(IluDev P, const double* __restrict__ b, double* x, const int* __restrict__ active,
-                     int lb_rows, int stage_bytes, int off_slots, int task_slots, int* flags) {
-    using CT = typename IluCT<MT>::T;
-    constexpr int T = ILU_BULK_TPB;
-    constexpr int RPT = ILU_BULK_RPT;
-    constexpr int LR = lb_row<CT>();
-    if (active && !*active) return;
-    __shared__ __align__(8) unsigned long long s_bar[NS];
-    __shared__ int s_abort;
-    // per stage: valid, first row, rows, the level's first row, its buffer,
-    // the previous level's first row and width
-    __shared__ int s_q[NS][8];
-    extern __shared__ __align__(128) unsigned char s_dyn[];
-    unsigned char* s_stage = s_dyn;                                                   // [NS][stage_bytes]
-    double* s_y0 = reinterpret_cast<double*>(s_dyn + (size_t)NS * stage_bytes);       // [NS][T]
-    CT* s_lvx = reinterpret_cast<CT*>(s_y0 + NS * T);                                 // [2][lb_rows][LR]
-    uint2* s_task = reinterpret_cast<uint2*>(s_lvx + 2 * LR * lb_rows);               // [task_slots] f then b
-    int* s_off = reinterpret_cast<int*>(s_task + task_slots);                         // [off_slots]
-    const int part = blockIdx.x;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool producer = warp == T / 32;
-    const int rsub = lane / 5, comp = lane - 5 * (lane / 5);
-    const bool lane_ok = !producer && lane < 30;
-    const int i_row = warp * 6 + rsub;
-    const int l0 = P.part_lvl0[part], l1 = P.part_lvl0[part + 1];
-    const bool staged = l1 - l0 < off_slots;
-    if (staged)
-        for (int i = tid; i <= l1 - l0; i += ILU_BULK_THREADS) s_off[i] = P.lvl_off[l0 + i];
-    const int tf0 = P.part_tf[part], ntf = P.part_tf[part + 1] - tf0;
-    const int tb0 = P.part_tb[part], ntb = P.part_tb[part + 1] - tb0;
-    const bool tstaged = ntf + ntb <= task_slots;
-    if (tstaged) {
-        for (int i = tid; i < ntf; i += ILU_BULK_THREADS) s_task[i] = P.task_f[tf0 + i];
-        for (int i = tid; i < ntb; i += ILU_BULK_THREADS) s_task[ntf + i] = P.task_b[tb0 + i];
+// ---- ILU apply with the factor records brought in by bulk copies
+//
+// x = (L U)^-1 b on each subdomain: one CTA walks the subdomain's wavefront
+// levels forward (unit L) and backward (U with the stored pivot inverses).
+// What bounds it is the chain of levels: each one reads the x of the level
+// before, multiplies and hands its own on, and a warp by itself spends three
+// quarters of a task's ~900 cycles on fetching the task.  So everything that
+// does not depend on the previous level is taken off that chain:
+//  * a producer warp brings the records (rdst_records.h), a group of tasks
+//    per cp.async.bulk, into one of two shared-memory stages, and the
+//    starting values (b forward, the forward result backward) of the
+//    group's rows by coalesced cp.async; both complete on the stage's "full"
+//    mbarrier, the compute warps return the stage on its "empty" one;
+//  * the tasks, six rows each, go round the W compute warps, and a warp
+//    brings its next task's columns, block rows (whole 16-byte words,
+//    conflict-free) and starting value into registers while the others walk
+//    the levels before it;
+//  * a level's end is a named barrier (one id per level in turn) on which a
+//    warp only arrives, except for the one level that its next task reads.
+// What is left between two levels is the load of the previous level's x
+// from the level buffers (two, by level parity), five multiply-adds per
+// block, backward the pivot product by shuffles, and the store, without a
+// branch: a row short of NB blocks multiplies zeros with the buffers' row of
+// zeros.
+//
+// Five lanes a row (one per component).  The lanes multiply in CT, the
+// arithmetic of the factors' storage type (FP64 in double, FP32 and BF16 in
+// float); input b and output x stay FP64 vectors.  Each block's product with
+// x_k is summed first, then subtracted from y, block by block in column
+// order.  Blocks beyond the first NB of a row (rare) are read from the stage
+// when they are needed (EXT).
+//
+// TIGHT: three compute warps (two with FP64) and the registers of six CTAs an
+// SM.  Every
+// mbarrier wait is bounded (2 s of globaltimer): on expiry the warp raises
+// bit 2 of *flags (reported as a timeout by the host), takes part in the
+// sweep's remaining level barriers, so that no other warp stays in one, and
+// ends; they find their own waits expired in turn, and the producer waits,
+// again bounded, for its copies in flight.
+__device__ __forceinline__ unsigned long long globaltimer_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// global -> shared bulk copy completing on an mbarrier (no multicast)
+__device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// true once the phase of parity `parity` has completed; false after 2 s
+__device__ __noinline__ bool mbar_wait_slow(unsigned bar, unsigned parity) {
+    const unsigned long long t0 = globaltimer_ns();
+    for (;;) {
+        for (int it = 0; it < 64; ++it)
+            if (mbar_try(bar, parity)) return true;
+        if (globaltimer_ns() - t0 > 2000000000ull) return false;
     }
-    const unsigned bar0 = (unsigned)__cvta_generic_to_shared(&s_bar[0]);
-    const unsigned stage0 = (unsigned)__cvta_generic_to_shared(s_stage);
-    const unsigned y0s = (unsigned)__cvta_generic_to_shared(s_y0);
-    if (tid == 0) {
-        for (int k = 0; k < NS; ++k) mbar_init(bar0 + 8 * k, 1);
-        s_abort = 0;
+}
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
+    return mbar_try(bar, parity) || mbar_wait_slow(bar, parity);
+}
+__device__ __forceinline__ void cpa8(unsigned dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
+}
+// the calling thread's cp.async so far count as one of the arrivals of bar
+__device__ __forceinline__ void cpa_arrive(unsigned bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+
+// Shared-memory loads and stores by 32-bit address.  They are issued in
+// program order (volatile), so a task's loads go out together ahead of the
+// arithmetic; `ok` false: zeros, no load.
+__device__ __forceinline__ uint4 lds4(unsigned a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ unsigned lds1(unsigned a) {
+    unsigned v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ unsigned lds_byte(unsigned a) {
+    unsigned v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ double lds_double(unsigned a) {
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts(unsigned a, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
+__device__ __forceinline__ void sts(unsigned a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+// level-buffer row: five values padded to 16 bytes (6 doubles / 8 floats)
+template <typename CT> constexpr int lb_row_bytes() { return sizeof(CT) == 8 ? 48 : 32; }
+__device__ __forceinline__ void lb_load(unsigned a, double (&o)[5]) {
+    asm volatile("ld.shared.v2.f64 {%0,%1}, [%2];" : "=d"(o[0]), "=d"(o[1]) : "r"(a) : "memory");
+    asm volatile("ld.shared.v2.f64 {%0,%1}, [%2];" : "=d"(o[2]), "=d"(o[3]) : "r"(a + 16) : "memory");
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(o[4]) : "r"(a + 32) : "memory");
+}
+__device__ __forceinline__ void lb_load(unsigned a, float (&o)[5]) {
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]) : "r"(a) : "memory");
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(o[4]) : "r"(a + 16) : "memory");
+}
+// one row of five entries of a record's values: word `idx` of the task's
+// 5 * tot (rdst_records.h)
+__device__ __forceinline__ void rec_load(unsigned v, int tot, int idx, bool ok, double (&o)[5], double) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n mov.f64 %0, 0d0000000000000000;\n"
+                 " mov.f64 %1, %0;\n mov.f64 %2, %0;\n mov.f64 %3, %0;\n mov.f64 %4, %0;\n"
+                 " @p ld.shared.v2.f64 {%0,%1}, [%6];\n @p ld.shared.v2.f64 {%2,%3}, [%7];\n @p ld.shared.f64 %4, [%8];\n}"
+                 : "=&d"(o[0]), "=&d"(o[1]), "=&d"(o[2]), "=&d"(o[3]), "=&d"(o[4])
+                 : "r"((unsigned)ok), "r"(v + 16 * idx), "r"(v + 80 * tot + 16 * idx), "r"(v + 160 * tot + 8 * idx));
+}
+__device__ __forceinline__ void rec_load(unsigned v, int tot, int idx, bool ok, float (&o)[5], float) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n mov.f32 %0, 0f00000000;\n"
+                 " mov.f32 %1, %0;\n mov.f32 %2, %0;\n mov.f32 %3, %0;\n mov.f32 %4, %0;\n"
+                 " @p ld.shared.v4.f32 {%0,%1,%2,%3}, [%6];\n @p ld.shared.f32 %4, [%7];\n}"
+                 : "=&f"(o[0]), "=&f"(o[1]), "=&f"(o[2]), "=&f"(o[3]), "=&f"(o[4])
+                 : "r"((unsigned)ok), "r"(v + 16 * idx), "r"(v + 80 * tot + 4 * idx));
+}
+__device__ __forceinline__ void rec_load(unsigned v, int tot, int idx, bool ok, float (&o)[5], __nv_bfloat16) {
+    unsigned a, b, c;
+    asm volatile("{\n .reg .pred p;\n .reg .u16 h;\n setp.ne.u32 p, %3, 0;\n mov.u32 %0, 0;\n mov.u32 %1, 0;\n"
+                 " mov.u16 h, 0;\n @p ld.shared.v2.u32 {%0,%1}, [%4];\n @p ld.shared.u16 h, [%5];\n cvt.u32.u16 %2, h;\n}"
+                 : "=&r"(a), "=&r"(b), "=&r"(c)
+                 : "r"((unsigned)ok), "r"(v + 8 * idx), "r"(v + 40 * tot + 2 * idx));
+    o[0] = __uint_as_float(a << 16); o[1] = __uint_as_float(a & 0xffff0000u);
+    o[2] = __uint_as_float(b << 16); o[3] = __uint_as_float(b & 0xffff0000u);
+    o[4] = __uint_as_float(c << 16);
+}
+// the same words written by the pack
+__device__ __forceinline__ void rec_store(unsigned char* v, int tot, int idx, const double (&o)[5]) {
+    *reinterpret_cast<double2*>(v + 16 * (size_t)idx) = make_double2(o[0], o[1]);
+    *reinterpret_cast<double2*>(v + 80 * (size_t)tot + 16 * (size_t)idx) = make_double2(o[2], o[3]);
+    *reinterpret_cast<double*>(v + 160 * (size_t)tot + 8 * (size_t)idx) = o[4];
+}
+__device__ __forceinline__ void rec_store(unsigned char* v, int tot, int idx, const float (&o)[5]) {
+    *reinterpret_cast<float4*>(v + 16 * (size_t)idx) = make_float4(o[0], o[1], o[2], o[3]);
+    *reinterpret_cast<float*>(v + 80 * (size_t)tot + 4 * (size_t)idx) = o[4];
+}
+__device__ __forceinline__ void rec_store(unsigned char* v, int tot, int idx, const __nv_bfloat16 (&o)[5]) {
+    uint2 a;
+    a.x = (unsigned)__bfloat16_as_ushort(o[0]) | (unsigned)__bfloat16_as_ushort(o[1]) << 16;
+    a.y = (unsigned)__bfloat16_as_ushort(o[2]) | (unsigned)__bfloat16_as_ushort(o[3]) << 16;
+    *reinterpret_cast<uint2*>(v + 8 * (size_t)idx) = a;
+    *reinterpret_cast<unsigned short*>(v + 40 * (size_t)tot + 2 * (size_t)idx) = __bfloat16_as_ushort(o[4]);
+}
+
+// factor blocks -> records (after each factorisation): a warp per task, lane
+// (position, component) as the apply reads it, so that every store of a slot
+// fills whole sectors of the record; the reads of the sliced stores are 6-row
+// pieces of lines that the neighbouring warps share.  L comes from the factor
+// store, U from A (from the factor store for rows whose own blocks take
+// updates, zero for a fill), backward first the pivot inverse.
+template <typename MT>
+__global__ void __launch_bounds__(256) k_ilu_pack(int nf, int nb, SellMat<MT> A, const MT* __restrict__ lu,
+                                                  const MT* __restrict__ dinv, IluDev P) {
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (w >= nf + nb) return;
+    const bool back = w >= nf;
+    unsigned char* rec = back ? P.rec_b : P.rec_f;
+    const RecTask t = back ? P.task_b[w - nf] : P.task_f[w];
+    const uint4 h = *reinterpret_cast<const uint4*>(rec + (size_t)t.head16 * 16);
+    const uint4 g = *reinterpret_cast<const uint4*>(rec + (size_t)t.head16 * 16 + 16);
+    const int n = (int)(h.y & 255u), S = (int)((h.y >> 8) & 255u), tot = (int)(h.w >> 16);
+    const int pos = lane / 5, comp = lane - 5 * pos;
+    if (lane >= 30 || pos >= n) return;
+    unsigned char* v = rec + (size_t)t.group16 * 16 + 16 * (size_t)(h.x >> 16);
+    const int r = (int)h.z + (int)((pos < 4 ? g.y >> (8 * pos) : g.z >> (8 * (pos - 4))) & 255u);
+    const int ms = P.ml + P.mu;
+    auto copy = [&](const MT* src, int blk) {       // src: entry 0 of the block, entries 32 apart
+        MT o[5];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) o[j] = src ? src[(5 * comp + j) * 32] : mt_zero<MT>();
+        rec_store(v, tot, 5 * blk + comp, o);
+    };
+    if (back) copy(dinv + flat_e(r, 0), pos);
+    const bool own_u = back && ((P.nlu[r] >> 16) & 1);
+    int blk = (back ? n : 0) + pos;
+#pragma unroll 4
+    for (int k = 0; k < S; ++k) {
+        const int nk = k < 4 ? (int)((g.x >> (8 * k)) & 255u) : (int)v[k - 16];
+        if (pos < nk) {
+            const int f = lu_fid(r, back ? P.ml + k : k, ms);
+            const MT* src = lu + flat_e(f, 0);
+            if (back && !own_u) {
+                const int a = P.lu_src[f];
+                src = a >= 0 ? A.val + flat_e(a, 0) : nullptr;
+            }
+            copy(src, blk);
+        }
+        blk += nk;
+    }
+}
+
+template <typename MT, int NB, bool EXT, bool TIGHT>
+__global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TIGHT ? 6 : 2)
+    k_ilu_apply_rec(IluDev P, const double* __restrict__ b, double* x, const int* __restrict__ active,
+                    int stage_bytes, int y0_rows, int lb_rows, int* flags) {
+    using CT = typename IluCT<MT>::T;
+    if (active && !*active) return;
+    __shared__ __align__(8) unsigned long long s_bar[2 * REC_STAGES + 1];     // full, empty, forward done
+    extern __shared__ __align__(128) unsigned char s_dyn[];
+    const int part = blockIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int W = (int)(blockDim.x >> 5) - 1;
+    double* s_y0 = reinterpret_cast<double*>(s_dyn + (size_t)REC_STAGES * stage_bytes);       // [REC_STAGES][5 y0_rows]
+    unsigned char* s_lb = reinterpret_cast<unsigned char*>(s_y0 + (size_t)REC_STAGES * 5 * y0_rows);   // [2 lb_rows + 1]
+    const unsigned full0 = (unsigned)__cvta_generic_to_shared(&s_bar[0]), empty0 = full0 + 8 * REC_STAGES;
+    const unsigned fdone = empty0 + 8 * REC_STAGES;
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < REC_STAGES; ++k) {
+            mbar_init(full0 + 8 * k, 33);          // the record's expect_tx, and each producer lane's y0 copies
+            mbar_init(empty0 + 8 * k, W);
+        }
+        mbar_init(fdone, W);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    auto off = [&](int l) { return staged ? s_off[l - l0] : P.lvl_off[l]; };
-    unsigned par = 0;          // compute warps: bit k, parity of stage k's next completion
-    unsigned ipar = 0;         // producer: bit k, parity of the next copy issued into stage k
-    unsigned lastp = 0;        // producer: bit k, parity of the last copy issued into stage k
-    unsigned issued = 0;       // producer: bit k, stage k has taken a copy
+    const int gf0 = P.part_gf[part], ngf = P.part_gf[part + 1] - gf0;
+    const int gb0 = P.part_gb[part], ngb = P.part_gb[part + 1] - gb0;
 
-#pragma unroll 1
-    for (int sweep = 0; sweep < 2; ++sweep) {
-        const bool back = sweep == 1;
-        const int dir = back ? -1 : 1;
-        const unsigned char* rec = back ? P.rec_b : P.rec_f;
-        const double* ysrc = back ? x : b;
-        IluCursor cur{back ? l1 - 1 : l0, 0};
-        int tcount = 0;        // tasks of this sweep issued so far (producer)
-        auto in_range = [&](int l) { return back ? l >= l0 : l < l1; };
-        // producer: the next task into stage d (cursor, s_q, record copy,
-        // y0 copies of the compute lanes: thread 32k + lane, row 6k + lane/5)
-        auto prepare = [&](int d) {
-            const bool v = in_range(cur.l);
-            int r0q = 0, nq = 0, aq = 0, bufq = 0, paq = 0, pwq = 0;
-            if (v) {
-                const int r0 = off(cur.l), r1 = off(cur.l + 1), n = r1 - r0;
-                r0q = r0 + cur.base;
-                nq = min(RPT, n - cur.base);
-                if (LB) {
-                    aq = r0;
-                    bufq = (cur.l & 1) * lb_rows * LR;
-                    const int lp = cur.l - dir;          // the level taken just before
-                    if (in_range(lp)) { paq = off(lp); pwq = off(lp + 1) - paq; }
-                }
-                cur.base += RPT;
-                if (cur.base >= n) { cur.l += dir; cur.base = 0; }
-                if (lane == 0) {
-                    const uint2 tk = tstaged ? s_task[(back ? ntf : 0) + tcount]
-                                             : (back ? P.task_b[tb0 + tcount] : P.task_f[tf0 + tcount]);
-                    mbar_expect_tx(bar0 + 8 * d, tk.y);
-                    bulk_g2s(stage0 + (unsigned)(d * stage_bytes), rec + (size_t)tk.x * 16, tk.y, bar0 + 8 * d);
-                }
-                ++tcount;
-                lastp = (lastp & ~(1u << d)) | (ipar & (1u << d));
-                ipar ^= 1u << d;
-                issued |= 1u << d;
-            }
+    if (warp == W) {
+        // ---------------- producer
+        const unsigned stage0 = (unsigned)__cvta_generic_to_shared(s_dyn), y0s = (unsigned)__cvta_generic_to_shared(s_y0);
+        int s = 0;
+        unsigned ph = 0;                           // parity of the next fill of stage s
+        unsigned used = 0, lastp = 0;              // stages that took a copy, parity of the last one
+        bool ok = true;
+        auto record = [&](const RecGroup& g, const unsigned char* rec) {
+            ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1u));
+            if (!ok) return;
             if (lane == 0) {
-                s_q[d][0] = v; s_q[d][1] = r0q; s_q[d][2] = nq; s_q[d][3] = aq;
-                s_q[d][4] = bufq; s_q[d][5] = paq; s_q[d][6] = pwq;
+                mbar_expect_tx(full0 + 8 * s, g.bytes);
+                bulk_g2s(stage0 + (unsigned)(s * stage_bytes), rec + (size_t)g.off16 * 16, g.bytes, full0 + 8 * s);
             }
-#pragma unroll
-            for (int k = 0; k < T / 32; ++k) {
-                const int row = 6 * k + rsub;
-                const bool ok = v && lane < 30 && row < nq;
-                cpa8(y0s + (unsigned)((d * T + 32 * k + lane) * 8), ysrc + (ok ? 5 * (size_t)(r0q + row) + comp : 0),
-                     ok);
-            }
-            cpa_commit();
+            used |= 1u << s;
+            lastp = (lastp & ~(1u << s)) | (ph << s);
         };
-        // compute warps: task d, after its stage has landed: y = y0 -
-        // sum_k (L_rk x_k) (backward x_r = inv(U_rr) y)
-        auto run = [&](int d) {
-            if (!mbar_wait(bar0 + 8 * d, (par >> d) & 1u)) {
-                atomicOr(flags, 4);
-                s_abort = 1;
-            }
-            par ^= 1u << d;
-            const int qr0 = s_q[d][1], qn = s_q[d][2], qa = s_q[d][3], qbuf = s_q[d][4];
-            const int qpa = s_q[d][5], qpw = s_q[d][6];
-            const bool act = lane_ok && i_row < qn && !s_abort;
-            const int r = qr0 + i_row;
-            const unsigned char* st0 = s_stage + (size_t)d * stage_bytes;
-            const unsigned hdr = act ? reinterpret_cast<const unsigned*>(st0)[i_row] : 0u;
-            const int cnt = (int)(hdr >> 24);
-            const int* cols = reinterpret_cast<const int*>(st0 + (hdr & 0xffffffu));
-            const MT* vals = reinterpret_cast<const MT*>(st0 + (hdr & 0xffffffu) + 16 * ((cnt + 3) >> 2));
-            CT y = to_ct(s_y0[d * T + tid], CT());
-            if (act) {
-                // the first four blocks side by side (their products are
-                // independent), then subtracted in column order; a block
-                // past the row's count loads nothing and contributes 0
-                const CT* pbuf = s_lvx + (lb_rows * LR - qbuf);   // the other level buffer
-                CT part4[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    CT t = CT(0);
-                    if (k < cnt) {
-                        const int ck = cols[k];
-                        const unsigned rel = (unsigned)(ck - qpa);
-                        CT xk[5];
-                        if (LB && rel < (unsigned)qpw) {
-                            lb_load(pbuf + LR * rel, xk);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 5; ++j) xk[j] = to_ct(x[5 * ck + j], CT());
-                        }
-                        t = to_ct(vals[25 * k + 5 * comp], CT()) * xk[0];
-#pragma unroll
-                        for (int j = 1; j < 5; ++j) t += to_ct(vals[25 * k + 5 * comp + j], CT()) * xk[j];
-                    }
-                    part4[k] = t;
-                }
-#pragma unroll
-                for (int k = 0; k < 4; ++k) y -= part4[k];
-                for (int k = 4; k < cnt; ++k) {
-                    const int ck = cols[k];
-                    const unsigned rel = (unsigned)(ck - qpa);
-                    CT xk[5];
-                    if (LB && rel < (unsigned)qpw) {
-                        lb_load(pbuf + LR * rel, xk);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 5; ++j) xk[j] = to_ct(x[5 * ck + j], CT());
-                    }
-                    CT t = to_ct(vals[25 * k + 5 * comp], CT()) * xk[0];
-#pragma unroll
-                    for (int j = 1; j < 5; ++j) t += to_ct(vals[25 * k + 5 * comp + j], CT()) * xk[j];
-                    y -= t;
-                }
-            }
-            if (back) {
-                CT a = CT(0);
-#pragma unroll
-                for (int j = 0; j < 5; ++j) {
-                    const CT yj = __shfl_sync(0xffffffffu, y, (lane_ok ? 5 * rsub : 0) + j);
-                    a += (act ? to_ct(vals[25 * cnt + 5 * comp + j], CT()) : CT(0)) * yj;
-                }
-                y = a;
-            }
-            if (act) {
-                x[5 * (size_t)r + comp] = (double)y;
-                if (LB) s_lvx[qbuf + LR * (r - qa) + comp] = y;
-            }
+        auto start = [&](const RecGroup& g, int st, const double* src) {
+            const double* p = src + 5 * (size_t)g.row0;
+            const unsigned d = y0s + (unsigned)(st * 5 * y0_rows) * 8;
+            for (int i = lane; i < 5 * g.nrows; i += 32) cpa8(d + 8 * i, p + i);
+            cpa_arrive(full0 + 8 * st);
         };
-        if (producer) {
-#pragma unroll
-            for (int d = 0; d < NS - 1; ++d) prepare(d);
-            cpa_wait<0>();
+        auto step = [&] { if (++s == REC_STAGES) { s = 0; ph ^= 1u; } };
+        // the descriptors are read one group ahead: their latency would be
+        // paid once per group otherwise
+        RecGroup nx = P.grp_f[gf0], nb = P.grp_b[gb0];
+        for (int g = 0; g < ngf && ok; ++g) {
+            const RecGroup cur = nx;
+            if (g + 1 < ngf) nx = P.grp_f[gf0 + g + 1];
+            record(cur, P.rec_f);
+            if (ok) { start(cur, s, b); step(); }
         }
-        __syncthreads();
-        bool go = s_q[0][0] != 0;
-        while (go) {
-            // stage slots rotate with compile-time indices (the body is
-            // unrolled NS times), so the queue stays in registers
-#pragma unroll
-            for (int u = 0; u < NS; ++u) {
-                if (go) {
-                    if (producer) {
-                        prepare((u + NS - 1) % NS);
-                        cpa_wait<0>();
-                    } else {
-                        run(u);
-                    }
-                    __syncthreads();
-                    go = s_q[(u + 1) % NS][0] != 0 && !s_abort;
-                }
+        // the backward records may run ahead of the forward sweep, their
+        // starting values not
+        const int nahead = min(REC_STAGES, ngb);
+        const int s_first = s;
+        for (int g = 0; g < nahead && ok; ++g) {
+            const RecGroup cur = nb;
+            if (g + 1 < ngb) nb = P.grp_b[gb0 + g + 1];
+            record(cur, P.rec_b);
+            if (ok) step();
+        }
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(fdone, 0));
+        if (ok) {
+            int st = s_first;
+            for (int g = 0; g < nahead; ++g) {
+                start(P.grp_b[gb0 + g], st, x);
+                if (++st == REC_STAGES) st = 0;
             }
         }
-        if (s_abort) {
-            // copies still in flight land before the CTA's shared memory goes
-            if (producer && lane == 0)
-                for (int d = 0; d < NS; ++d)
-                    if ((issued >> d) & 1u) mbar_wait(bar0 + 8 * d, (lastp >> d) & 1u);
-            return;
+        for (int g = nahead; g < ngb && ok; ++g) {
+            const RecGroup cur = nb;
+            if (g + 1 < ngb) nb = P.grp_b[gb0 + g + 1];
+            record(cur, P.rec_b);
+            if (ok) { start(cur, s, x); step(); }
         }
-        // the next sweep prepares its first tasks into stages 0..NS-2 again:
-        // the rotation restarts, parities carry on
-        __syncthreads();
+        // abandoned: copies still in flight land before the CTA's shared memory goes
+        if (!ok && lane == 0) {
+            atomicOr(flags, 4);
+            for (int d = 0; d < REC_STAGES; ++d)
+                if ((used >> d) & 1u) mbar_wait(full0 + 8 * d, (lastp >> d) & 1u);
+        }
+        return;
     }
+
+    // ---------------- compute warps
+    constexpr unsigned LRB = lb_row_bytes<CT>();
+    // ids of the level barriers: more than the W levels a warp can be ahead of
+    // the slowest.  An SM has 64 barriers and a kernel that names one in a
+    // register reserves all 16, which would leave four CTAs an SM.
+    constexpr int NBAR = TIGHT ? 4 : 15;
+    const int rsub = lane / 5, comp = lane - 5 * rsub;
+    const int pos0 = lane < 30 ? rsub : 0x7fffffff;       // position in the task
+    const int sbase = lane < 30 ? 5 * rsub : 0;
+    const unsigned dyn = (unsigned)__cvta_generic_to_shared(s_dyn), lb = (unsigned)__cvta_generic_to_shared(s_lb);
+    const unsigned y0a = (unsigned)__cvta_generic_to_shared(s_y0);
+    const int nlev = P.part_lvl0[part + 1] - P.part_lvl0[part];
+    // the row of zeros (every warp its own copy of the same zeros: no warp
+    // reads it before it has written it)
+    if (lane < (int)LRB / 4) sts(lb + 2 * lb_rows * LRB + 4 * lane, 0.0f);
+    __syncwarp();
+    int s = 0;                  // stage of the group the warp is in
+    unsigned ph = 0;
+    auto sweep = [&](auto back_tag) -> bool {
+        constexpr bool BACK = decltype(back_tag)::value;
+        const int ngrp = BACK ? ngb : ngf;
+        int grp = 0, arrived = 0, bid = 1;      // group in the sweep; level barriers arrived on, the next one's id
+        unsigned gn = 0;                        // the group's address
+        bool held = false;                      // the group is not returned yet
+        auto arrive = [&] {                     // end of a level on which nobody here waits
+            if (TIGHT) {
+                if (bid == 1) asm volatile("bar.arrive 1, %0;" ::"r"(W * 32) : "memory");
+                else if (bid == 2) asm volatile("bar.arrive 2, %0;" ::"r"(W * 32) : "memory");
+                else if (bid == 3) asm volatile("bar.arrive 3, %0;" ::"r"(W * 32) : "memory");
+                else asm volatile("bar.arrive 4, %0;" ::"r"(W * 32) : "memory");
+            } else {
+                asm volatile("bar.arrive %0, %1;" ::"r"(bid), "r"(W * 32) : "memory");
+            }
+            bid = bid == NBAR ? 1 : bid + 1;
+            ++arrived;
+        };
+        auto await = [&] {                      // end of the level before the next task's
+            if (TIGHT) {
+                if (bid == 1) asm volatile("bar.sync 1, %0;" ::"r"(W * 32) : "memory");
+                else if (bid == 2) asm volatile("bar.sync 2, %0;" ::"r"(W * 32) : "memory");
+                else if (bid == 3) asm volatile("bar.sync 3, %0;" ::"r"(W * 32) : "memory");
+                else asm volatile("bar.sync 4, %0;" ::"r"(W * 32) : "memory");
+            } else {
+                asm volatile("bar.sync %0, %1;" ::"r"(bid), "r"(W * 32) : "memory");
+            }
+            bid = bid == NBAR ? 1 : bid + 1;
+            ++arrived;
+        };
+        auto enter = [&] {                      // the group in stage s has landed
+            gn = dyn + (unsigned)(s * stage_bytes);
+            held = true;
+            if (__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, ph))) return true;
+            if (lane == 0) atomicOr(flags, 4);
+            while (arrived < nlev - 1) await();      // in step with the others, who may still run
+            return false;
+        };
+        auto release = [&] {
+            __syncwarp();
+            if (held && lane == 0) mbar_arrive(empty0 + 8 * s);
+            held = false;
+        };
+        auto next_group = [&] {
+            release();
+            if (++s == REC_STAGES) { s = 0; ph ^= 1u; }
+            ++grp;
+            return enter();
+        };
+        // the current task: what its rows need, in registers, and where its
+        // blocks lie
+        CT v[NB][5], di[5], y = CT(0);
+        int cq[NB], r = 0, S = 0, tot = 0, n = 0, pos = 0;
+        unsigned own = 0, fl = 0, cc = 0, cv = 0, nk4 = 0, way = 0;
+        bool act = false, kept = false;
+        auto load = [&](int t) {
+            const uint4 h = lds4(gn + 16 + 32 * t), g = lds4(gn + 32 + 32 * t);
+            n = (int)(h.y & 255u);
+            S = (int)((h.y >> 8) & 255u);
+            fl = h.y >> 16;
+            tot = (int)(h.w >> 16);
+            act = pos0 < n;
+            pos = act ? pos0 : 0;
+            cc = gn + 16 * (h.x & 0xffffu);
+            cv = gn + 16 * (h.x >> 16);
+            nk4 = g.x;
+            way = g.w;
+            const uint4 c4 = lds4(cc + 16 * pos);
+            const int rid = (int)((pos < 4 ? g.y >> (8 * pos) : g.z >> (8 * (pos - 4))) & 255u);
+            y = (CT)lds_double(y0a + 8u * (unsigned)(5 * (s * y0_rows + (int)(way >> 16) + rid) + comp));
+            if (BACK) rec_load(cv, tot, 5 * pos + comp, act, di, MT());
+            int blk = (BACK ? n : 0) + pos;
+#pragma unroll
+            for (int k = 0; k < NB; ++k) {
+                const int nk = (int)((nk4 >> (8 * k)) & 255u);
+                rec_load(cv, tot, 5 * blk + comp, pos0 < nk, v[k], MT());
+                blk += nk;
+            }
+            const unsigned ca[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+            for (int k = 0; k < NB; ++k) cq[k] = (int)ca[k];
+            r = (int)h.z + rid;
+            kept = act && (h.w & 0xffffu) != 0xffffu;
+            own = lb + ((h.w & 0xffffu) + rid) * LRB + (unsigned)sizeof(CT) * comp;
+            // a group whose last task of this warp is in registers goes back
+            if (((way >> 8) & 255u) && (!EXT || S <= NB)) release();
+            return (int)(g.z >> 16);
+        };
+        auto far_row = [&](int c, CT (&o)[5]) {
+            const double* xk = x + 5 * (size_t)(-1 - c);
+#pragma unroll
+            for (int j = 0; j < 5; ++j) o[j] = (CT)xk[j];
+        };
+        auto product = [&](const CT (&m)[5], const CT (&xk)[5]) {
+            CT t = m[0] * xk[0];
+#pragma unroll
+            for (int j = 1; j < 5; ++j) t += m[j] * xk[j];
+            return t;
+        };
+        // ---- the warp's first task
+        if (!enter()) return false;
+        int first = warp, ntask = (int)lds1(gn + 8);
+        if (first < ntask) {
+            for (int T = (int)lds1(gn); first >= T; T = (int)lds1(gn)) {
+                first -= T;
+                if (!next_group()) return false;
+            }
+            const int level = load(first);
+            while (arrived < level - 1) arrive();
+            if (arrived < level) await();
+            for (;;) {
+                // ---- the chain: x of the level before, products, hand on
+                CT part_k[NB];
+                auto blocks = [&](auto far_tag) {
+#pragma unroll
+                    for (int k = 0; k < NB; ++k) {
+                        CT xk[5];
+                        lb_load(lb + (decltype(far_tag)::value ? max(cq[k], 0) : cq[k]), xk);
+                        if (decltype(far_tag)::value && cq[k] < 0) far_row(cq[k], xk);
+                        part_k[k] = product(v[k], xk);
+                    }
+                };
+                if (fl & REC_FAR) blocks(std::true_type{});
+                else blocks(std::false_type{});
+#pragma unroll
+                for (int k = 0; k < NB; ++k) y -= part_k[k];
+                if (EXT && S > NB) {
+                    int blk = (BACK ? n : 0) + pos;
+#pragma unroll
+                    for (int k = 0; k < NB; ++k) blk += (int)((nk4 >> (8 * k)) & 255u);
+                    for (int k = NB; k < S; ++k) {
+                        const int nk = k < 4 ? (int)((nk4 >> (8 * k)) & 255u) : (int)lds_byte(cv - 16 + k);
+                        const int c = (int)lds1(cc + 16 * ((k >> 2) * n + pos) + 4 * (k & 3));
+                        CT xe[5], m[5];
+                        lb_load(lb + max(c, 0), xe);
+                        if (c < 0) far_row(c, xe);
+                        rec_load(cv, tot, 5 * blk + comp, pos0 < nk, m, MT());
+                        y -= product(m, xe);
+                        blk += nk;
+                    }
+                }
+                if (BACK) {
+                    // x_r = inv(U_rr) y, the row's five components by shuffle
+                    CT a = CT(0);
+#pragma unroll
+                    for (int j = 0; j < 5; ++j) a += di[j] * __shfl_sync(0xffffffffu, y, sbase + j);
+                    y = a;
+                }
+                if (kept) sts(own, y);
+                if (act) x[5 * (size_t)r + comp] = (double)y;
+                if (fl & REC_WARP_LAST) break;
+                // ---- on to the warp's next task
+                const int dl = (int)(fl >> 8) & 255;
+                for (int q = 1; q < dl; ++q) arrive();
+                const int t = (int)(way & 255u);
+                for (unsigned q = (way >> 8) & 255u; q > 0; --q)
+                    if (!next_group()) return false;
+                load(t);
+                if (dl > 0) await();
+            }
+        }
+        while (arrived < nlev - 1) arrive();
+        if (!BACK) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(fdone);
+        }
+        // the groups of the other warps' last tasks pass by
+        while (grp + 1 < ngrp)
+            if (!next_group()) return false;
+        release();
+        if (++s == REC_STAGES) { s = 0; ph ^= 1u; }
+        return true;
+    };
+    if (!sweep(std::false_type{})) return;
+    sweep(std::true_type{});
 }
 
 // ---------------------------------------------------------------- vectors

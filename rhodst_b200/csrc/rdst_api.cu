@@ -269,21 +269,19 @@ struct rdst_ctx {
     DBuf<int> part_lvl0, lvl_off, low_start, nlu, tr_start, tr_kj, tr_rj, lu_col, lu_src;
     int lu_slots = 0;
     int ilu_ml = 0, ilu_mu = 0, ilu_mu_use = 0;
-    // task records of the bulk ILU apply (empty: the register apply runs)
+    // factor records of the ILU apply (empty: the register apply runs)
     DBuf<unsigned char> rec_f, rec_b;
-    DBuf<uint2> task_f, task_b;
-    DBuf<int> part_tf, part_tb;
-    DBuf<unsigned> val_f, val_b;
+    DBuf<RecGroup> grp_f, grp_b;
+    DBuf<int> part_gf, part_gb;
+    DBuf<RecTask> rec_task_f, rec_task_b;
+    bool rec_tight = false;
+    int rec_warps = 0, rec_stage_bytes = 0, rec_y0_rows = 0, rec_lb_rows = 0;
+    size_t rec_smem_bytes = 0;
     // addressing of the factorisation that reads A directly (else gather +
     // factor), both followed by the record pack
     DBuf<int> fr_trk, fr_trt;
     DBuf<int4> fr_desc;
     bool ilu_direct = false;
-    int ilu_stage_bytes = 0;         // largest task record, rounded to 128 bytes
-    int ilu_stages = 0;              // stages of the bulk apply (2 or 3)
-    int ilu_lb_rows = 0;             // rows of each level buffer (0: none)
-    int ilu_off_slots = 0;           // level offsets staged in shared memory (max levels + 1, even)
-    int ilu_task_slots = 0;          // task table entries staged (max forward + backward tasks, even)
     // Krylov
     DBuf<double> dx, r, t, Vb, s2, sh, ph, pv, xbar, Ax, pA;
     DBuf<double> gs_r, gs_z;        // residual and correction of Gauss-Seidel sweeps after the first
@@ -409,8 +407,8 @@ struct rdst_ctx {
         P.n_parts = n_parts; P.part_lvl0 = part_lvl0.p; P.lvl_off = lvl_off.p;
         P.nlu = nlu.p; P.low_start = low_start.p; P.ml = ilu_ml; P.mu = ilu_mu; P.mu_use = ilu_mu_use; P.lu_col = lu_col.p; P.lu_src = lu_src.p;
         P.tr_start = tr_start.p; P.tr_kj = tr_kj.p; P.tr_rj = tr_rj.p;
-        P.rec_f = rec_f.p; P.rec_b = rec_b.p; P.task_f = task_f.p; P.task_b = task_b.p;
-        P.part_tf = part_tf.p; P.part_tb = part_tb.p; P.val_f = val_f.p; P.val_b = val_b.p;
+        P.rec_f = rec_f.p; P.rec_b = rec_b.p; P.grp_f = grp_f.p; P.grp_b = grp_b.p;
+        P.part_gf = part_gf.p; P.part_gb = part_gb.p; P.task_f = rec_task_f.p; P.task_b = rec_task_b.p;
         P.fr_trk = fr_trk.p; P.fr_trt = fr_trt.p; P.fr_desc = fr_desc.p;
         return P;
     }
@@ -464,8 +462,8 @@ int lim_code(Limiter l) { return (int)l; }
 // holds at once the count is rounded to a whole number of such waves (a
 // partial last wave costs a whole extra chain: measured on the 1.2 M-cell
 // wing with the register apply, 784 parts took 23% longer than 592 or
-// 1184).  The bulk apply holds eight CTAs an SM (64 registers a thread, its
-// shared memory sized for that), the register apply four.
+// 1184).  A wave is counted as eight CTAs an SM with the record apply (it
+// holds six, the rest follow as those end), four with the register apply.
 int auto_ilu_parts(int N, Precision prec, bool bulk) {
     int dev = 0, sms = 0, per_sm = 0;
     CK(cudaGetDevice(&dev));
@@ -553,114 +551,34 @@ void load_geometry(rdst_ctx& c, const rdst_mesh* mh, bool in_place) {
     CK(cudaStreamSynchronize(s));
 }
 
-// The bulk apply's task records (IluDev::rec_f / rec_b): the tasks of each
-// part in the order the apply's cursor takes them (forward: levels
-// ascending; backward: levels descending; 24-row chunks of a level in
-// ascending rows), their headers and columns written here, the blocks by
-// k_ilu_pack after each factorisation.  Three stages when the CTAs every
-// subdomain needs at once (up to eight an SM) still fit with them, else
-// two; a task too large for one CTA's shared memory leaves the register
-// apply in place.
-void build_task_records(rdst_ctx& c, const Options& o, int nparts, const std::vector<int>& part_lvl0,
-                        const std::vector<int>& lvl_off, const std::vector<int>& lu_col,
-                        const std::vector<int>& lu_src, const std::vector<int>& nlu,
-                        const std::vector<int>& low_start, const std::vector<int>& tr_start,
-                        const std::vector<int>& tr_kj, const std::vector<int>& tr_rj, const std::vector<int>& nl,
-                        const std::vector<int>& nu, int ML, int MS) {
+// The apply's factor records (rdst_records.h) and the addressing of the
+// factorisation that reads A directly.  A plan that does not fit the shared
+// memory leaves the register apply in place.
+void build_records(rdst_ctx& c, const Options& o, int nparts, const std::vector<int>& part_lvl0,
+                   const std::vector<int>& lvl_off, const std::vector<int>& lu_col, const std::vector<int>& lu_src,
+                   const std::vector<int>& nlu, const std::vector<int>& low_start, const std::vector<int>& tr_start,
+                   const std::vector<int>& tr_kj, const std::vector<int>& tr_rj, const std::vector<int>& nl,
+                   const std::vector<int>& nu, int ML, int MS) {
     const int N = c.N;
-    const size_t S = o.precision == PREC_FP64 ? 8 : (o.precision == PREC_FP32 ? 4 : 2);
+    const int S = o.precision == PREC_FP64 ? 8 : (o.precision == PREC_FP32 ? 4 : 2);
     auto lfid = [&](int r, int sl) { return ((r >> 5) * MS + sl) * 32 + (r & 31); };
-    auto r16 = [](size_t v) { return (v + 15) / 16 * 16; };
-    auto cnt_of = [&](int r, bool back) { return back ? (c.ilu_mu_use ? nu[r] : 0) : nl[r]; };
-    auto rec_bytes = [&](int r, bool back) {
-        const int n = cnt_of(r, back);
-        return r16(16 * (size_t)((n + 3) / 4) + (size_t)(n + (back ? 1 : 0)) * 25 * S);
-    };
-    struct Tk { int r0, n; };
-    std::vector<Tk> tf, tb;
-    std::vector<int> ptf(nparts + 1, 0), ptb(nparts + 1, 0);
-    int maxw = 0, maxlv = 0, maxtasks = 0;
-    for (int p = 0; p < nparts; ++p) {
-        ptf[p] = (int)tf.size();
-        ptb[p] = (int)tb.size();
-        const int a = part_lvl0[p], e = part_lvl0[p + 1];
-        maxlv = std::max(maxlv, e - a);
-        for (int li = a; li < e; ++li) {
-            const int r0 = lvl_off[li], n = lvl_off[li + 1] - r0;
-            maxw = std::max(maxw, n);
-            for (int b = 0; b < n; b += ILU_BULK_RPT) tf.push_back({r0 + b, std::min(ILU_BULK_RPT, n - b)});
-        }
-        for (int li = e - 1; li >= a; --li) {
-            const int r0 = lvl_off[li], n = lvl_off[li + 1] - r0;
-            for (int b = 0; b < n; b += ILU_BULK_RPT) tb.push_back({r0 + b, std::min(ILU_BULK_RPT, n - b)});
-        }
-        maxtasks = std::max(maxtasks, (int)(tf.size() - ptf[p] + tb.size() - ptb[p]));
-    }
-    ptf[nparts] = (int)tf.size();
-    ptb[nparts] = (int)tb.size();
-    size_t max_task = 0;
-    auto layout = [&](const std::vector<Tk>& tasks, bool back, std::vector<uint2>& tab) {
-        tab.resize(tasks.size());
-        size_t pos = 0;
-        for (size_t t = 0; t < tasks.size(); ++t) {
-            size_t bytes = ILU_BULK_HDR;
-            for (int i = 0; i < tasks[t].n; ++i) bytes += rec_bytes(tasks[t].r0 + i, back);
-            tab[t] = make_uint2((unsigned)(pos / 16), (unsigned)bytes);
-            pos += bytes;
-            max_task = std::max(max_task, bytes);
-        }
-        return pos;
-    };
-    std::vector<uint2> tabf, tabb;
-    const size_t totf = layout(tf, false, tabf), totb = layout(tb, true, tabb);
-    // shared memory: stages, y0 slots, level buffers, task table, level offsets
-    const int stage = (int)((max_task + 127) / 128 * 128);
-    const int lb = maxw <= ILU_LB_MAX ? maxw : 0;
-    const int task_slots = (maxtasks + 1) / 2 * 2;
-    const int off_slots = (maxlv + 2) / 2 * 2;
-    auto smem = [&](int ns) {
-        return (size_t)ns * stage + (size_t)ns * ILU_BULK_TPB * 8 + (size_t)lb * (S == 8 ? 96 : 64) +
-               (size_t)task_slots * 8 + (size_t)off_slots * 4 + 64;
-    };
-    int dev = 0, per_sm = 0, per_block = 0, reserved = 0;
+    int dev = 0, per_sm = 0, per_block = 0, reserved = 0, sms = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     CK(cudaDeviceGetAttribute(&per_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     CK(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
-    // CTAs an SM must hold for all subdomains to run at once (up to 8)
-    int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const size_t want = (size_t)std::min(8, std::max(1, (nparts + sms - 1) / std::max(sms, 1)));
-    int ns = 3;
-    if ((smem(3) + reserved) * want > (size_t)per_sm) ns = 2;
-    if (smem(ns) > (size_t)per_block) return;
-    if ((size_t)(std::max(ML, MS - ML) + 1) * 25 * 33 * S > (size_t)per_block) return;   // the pack's tiles
-    std::vector<unsigned char> bf(totf, 0), bb(totb, 0);
-    std::vector<unsigned> vf(N, 0), vb(N, 0);
-    auto fill = [&](const std::vector<Tk>& tasks, const std::vector<uint2>& tab, bool back,
-                    std::vector<unsigned char>& buf, std::vector<unsigned>& val) {
-        for (size_t t = 0; t < tasks.size(); ++t) {
-            const size_t start = (size_t)tab[t].x * 16;
-            unsigned* hdr = reinterpret_cast<unsigned*>(buf.data() + start);
-            size_t pos = start + ILU_BULK_HDR;
-            for (int i = 0; i < tasks[t].n; ++i) {
-                const int r = tasks[t].r0 + i, n = cnt_of(r, back);
-                hdr[i] = (unsigned)(pos - start) | ((unsigned)n << 24);
-                int* cols = reinterpret_cast<int*>(buf.data() + pos);
-                const int ncol = 4 * ((n + 3) / 4);
-                for (int q = 0; q < ncol; ++q) cols[q] = q < n ? lu_col[lfid(r, back ? ML + q : q)] : -1;
-                val[r] = (unsigned)((pos + 16 * (size_t)((n + 3) / 4)) / 16);
-                pos += rec_bytes(r, back);
-            }
-        }
-    };
-    fill(tf, tabf, false, bf, vf);
-    fill(tb, tabb, true, bb, vb);
+    const std::vector<int> none(c.ilu_mu_use ? 0 : N, 0);
+    RecPlan P = rec_plan(N, nparts, part_lvl0, lvl_off, lu_col, nl, c.ilu_mu_use ? nu : none, ML, MS, S, sms,
+                         (size_t)per_sm, (size_t)per_block, (size_t)reserved);
+    if (!P.ok) return;
     cudaStream_t s = c.s;
-    c.rec_f.upload(bf, s); c.rec_b.upload(bb, s);
-    c.task_f.upload(tabf, s); c.task_b.upload(tabb, s);
-    c.part_tf.upload(ptf, s); c.part_tb.upload(ptb, s);
-    c.val_f.upload(vf, s); c.val_b.upload(vb, s);
+    c.rec_f.upload(P.f.rec, s); c.rec_b.upload(P.b.rec, s);
+    c.grp_f.upload(P.f.groups, s); c.grp_b.upload(P.b.groups, s);
+    c.part_gf.upload(P.f.part_g, s); c.part_gb.upload(P.b.part_g, s);
+    c.rec_task_f.upload(P.f.tasks, s); c.rec_task_b.upload(P.b.tasks, s);
+    c.rec_warps = P.warps; c.rec_tight = P.tight; c.rec_stage_bytes = P.stage_bytes;
+    c.rec_y0_rows = P.y0_rows; c.rec_lb_rows = P.lb_rows; c.rec_smem_bytes = rec_smem(P, S);
     // the factorisation reading A directly: where each update triple reads
     // U_kj and which slot of row r takes it, and one descriptor per L slot
     {
@@ -689,16 +607,11 @@ void build_task_records(rdst_ctx& c, const Options& o, int nparts, const std::ve
             c.ilu_direct = true;
         }
     }
-    c.ilu_stage_bytes = stage;
-    c.ilu_stages = ns;
-    c.ilu_lb_rows = lb;
-    c.ilu_task_slots = task_slots;
-    c.ilu_off_slots = off_slots;
     CK(cudaStreamSynchronize(s));
 }
 
 template <typename MT>
-static void ilu_bulk_attr(rdst_ctx& c);
+static void ilu_rec_attr();
 
 void build(rdst_ctx& c, const rdst_mesh* mh) {
     cudaStream_t s = c.s;
@@ -996,8 +909,8 @@ void build(rdst_ctx& c, const rdst_mesh* mh) {
         c.lu_col.upload(lu_col, s); c.lu_src.upload(lu_src, s);
         c.lu_slots = MS;
         if (o.ilu_bulk)
-            build_task_records(c, o, nparts, part_lvl0, lvl_off, lu_col, lu_src, nlu, low_start, tr_start, tr_kj, tr_rj,
-                               nl, nu, ML, MS);
+            build_records(c, o, nparts, part_lvl0, lvl_off, lu_col, lu_src, nlu, low_start, tr_start, tr_kj, tr_rj,
+                          nl, nu, ML, MS);
     }
     // ---- AMG hierarchy: plan on the cell graph (original numbering), level
     // 0 in the internal row order; the Galerkin gather lists sum the finer
@@ -1140,9 +1053,9 @@ void build(rdst_ctx& c, const rdst_mesh* mh) {
     }
     if (o.precon != PRECON_NONE) CK(cudaMalloc(&c.dinv, (size_t)c.n_slices * 32 * 25 * c.mt_size));
     if (c.rec_f.p) {
-        if (o.precision == PREC_FP64) ilu_bulk_attr<double>(c);
-        else if (o.precision == PREC_FP32) ilu_bulk_attr<float>(c);
-        else ilu_bulk_attr<__nv_bfloat16>(c);
+        if (o.precision == PREC_FP64) ilu_rec_attr<double>();
+        else if (o.precision == PREC_FP32) ilu_rec_attr<float>();
+        else ilu_rec_attr<__nv_bfloat16>();
     }
     if (o.precon == PRECON_GAUSS_SEIDEL && o.n_sweeps > 1) { c.gs_r.alloc(5L * N); c.gs_z.alloc(5L * N); }
     // ---- Krylov
@@ -1160,20 +1073,6 @@ void build(rdst_ctx& c, const rdst_mesh* mh) {
 }
 
 // ---------------------------------------------------------------- step pieces
-// The bulk-copy apply (factor rows as records, one TMA copy per task):
-// its dynamic shared memory is the stages, the lanes' y0 slots and the x
-// ring when the context has one.
-// the pack's shared memory: the widest side's slots (L, or U + pivot inverse)
-template <typename MT>
-static size_t ilu_pack_smem(const rdst_ctx& c) {
-    return (size_t)(std::max(c.ilu_ml, c.ilu_mu) + 1) * ilu_pack_tile<MT>() * sizeof(MT);
-}
-template <typename MT>
-static size_t ilu_bulk_smem(const rdst_ctx& c) {
-    return (size_t)c.ilu_stages * c.ilu_stage_bytes + (size_t)c.ilu_stages * ILU_BULK_TPB * 8 +
-           (size_t)c.ilu_lb_rows * (sizeof(MT) == 8 ? 96 : 64) + (size_t)c.ilu_task_slots * 8 +
-           (size_t)c.ilu_off_slots * 4;
-}
 // A kernel's dynamic shared memory limit is a property of the function on
 // the device, shared by every context of the process: it is raised to the
 // device's per-block maximum less the kernel's static shared memory (never
@@ -1188,47 +1087,41 @@ static void set_max_dyn_smem(K* kernel) {
     CK(cudaFuncGetAttributes(&fa, kernel));
     CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, per_block - (int)fa.sharedSizeBytes));
 }
-template <typename MT, int NS, bool LB>
-static void ilu_bulk_launch(rdst_ctx& c, bool attr_only, const IluDev& P, const double* in, double* out,
-                            const int* active) {
-    const size_t sm = ilu_bulk_smem<MT>(c);
-    if (attr_only) {
-        set_max_dyn_smem(k_ilu_apply_bulk<MT, NS, LB>);
-        return;
-    }
-    k_ilu_apply_bulk<MT, NS, LB><<<c.n_parts, ILU_BULK_THREADS, sm, c.s>>>(P, in, out, active, c.ilu_lb_rows,
-                                                                        c.ilu_stage_bytes, c.ilu_off_slots,
-                                                                        c.ilu_task_slots, &c.sc.p->flags);
-}
-template <typename MT>
-static void ilu_bulk_dispatch(rdst_ctx& c, bool attr_only, const IluDev& P, const double* in, double* out,
-                              const int* active) {
-    const bool lb = c.ilu_lb_rows > 0;
-    if (c.ilu_stages == 3) {
-        if (lb) ilu_bulk_launch<MT, 3, true>(c, attr_only, P, in, out, active);
-        else ilu_bulk_launch<MT, 3, false>(c, attr_only, P, in, out, active);
+// The record apply's instance: rows with up to two blocks a side (2D quads),
+// or three in registers and the rest from the stage; the tight one for five
+// or six CTAs an SM.
+template <typename MT, typename F>
+static void ilu_rec_instance(int width, bool tight, F&& f) {
+    if (width <= 2) {
+        if (tight) f(k_ilu_apply_rec<MT, 2, false, true>);
+        else f(k_ilu_apply_rec<MT, 2, false, false>);
     } else {
-        if (lb) ilu_bulk_launch<MT, 2, true>(c, attr_only, P, in, out, active);
-        else ilu_bulk_launch<MT, 2, false>(c, attr_only, P, in, out, active);
+        if (tight) f(k_ilu_apply_rec<MT, 3, true, true>);
+        else f(k_ilu_apply_rec<MT, 3, true, false>);
     }
 }
 // dynamic shared memory above the default 48 KB: set when a context is
 // built (not while a step is being captured)
 template <typename MT>
-static void ilu_bulk_attr(rdst_ctx& c) {
-    ilu_bulk_dispatch<MT>(c, true, c.ilu(), nullptr, nullptr, nullptr);
-    set_max_dyn_smem(k_ilu_pack<MT>);
+static void ilu_rec_attr() {
+    for (int width : {2, 3})
+        for (bool tight : {false, true}) ilu_rec_instance<MT>(width, tight, [](auto* k) { set_max_dyn_smem(k); });
 }
 template <typename MT>
-static void ilu_apply_bulk(rdst_ctx& c, const IluDev& P, const double* in, double* out, const int* active) {
-    ilu_bulk_dispatch<MT>(c, false, P, in, out, active);
+static void ilu_apply_rec(rdst_ctx& c, const IluDev& P, const double* in, double* out, const int* active) {
+    const int threads = 32 * (c.rec_warps + 1);
+    ilu_rec_instance<MT>(std::max(c.ilu_ml, c.ilu_mu), c.rec_tight, [&](auto* k) {
+        k<<<c.n_parts, threads, c.rec_smem_bytes, c.s>>>(P, in, out, active, c.rec_stage_bytes, c.rec_y0_rows,
+                                                         c.rec_lb_rows, &c.sc.p->flags);
+    });
 }
-// blocks of the fresh factors -> the task records
+// blocks of the fresh factors -> the records
 template <typename MT>
 static void ilu_pack(rdst_ctx& c, void* val) {
     if (!c.rec_f.p) return;
-    k_ilu_pack<MT><<<c.n_slices, 256, ilu_pack_smem<MT>(c), c.s>>>(c.N, c.mat<MT>(val), (const MT*)c.LUval,
-                                                                   (const MT*)c.dinv, c.ilu());
+    const int nf = (int)c.rec_task_f.n, nb = (int)c.rec_task_b.n;
+    k_ilu_pack<MT><<<nblk(32L * (nf + nb), 256), 256, 0, c.s>>>(nf, nb, c.mat<MT>(val), (const MT*)c.LUval,
+                                                               (const MT*)c.dinv, c.ilu());
     CKL();
 }
 
@@ -1403,7 +1296,7 @@ struct Ops {
         const MT* di = (const MT*)c.dinv;
         const int N = c.N;
         if (c.rec_f.p) {
-            ilu_apply_bulk<MT>(c, P, in, out, active);
+            ilu_apply_rec<MT>(c, P, in, out, active);
         } else {
             if (nb <= 2) k_ilu_apply<MT, 2><<<c.n_parts, ILU_APPLY_TPB, 0, c.s>>>(N, LU, di, P, in, out, active);
             else if (nb <= 3) k_ilu_apply<MT, 3><<<c.n_parts, ILU_APPLY_TPB, 0, c.s>>>(N, LU, di, P, in, out, active);

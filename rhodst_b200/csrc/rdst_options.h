@@ -107,7 +107,7 @@ struct Options {
     bool ilu_graph = false;           // subdomains by graph bisection (true) or coordinate bisection
     int ilu_order = -1;               // rows of a subdomain: 0 mesh order, 1 breadth-first (rdst_order.h),
                                       // -1 breadth-first with more than one subdomain, else mesh order
-    bool ilu_bulk = true;             // ILU apply: task records, one bulk copy per task (same results)
+    bool ilu_bulk = true;             // ILU apply from factor records brought in by bulk copies (same results)
     int ilu_factor_threads = 32;      // threads of the factorisation's CTA (one CTA per subdomain): 32, 64 or 128
     bool graphs = true;               // capture steps in CUDA graphs
     int device = -1;                  // GPU ordinal of the context (-1: the calling thread's current one)

@@ -1,0 +1,289 @@
+// rdst_records.h -- the factor records of the subdomain ILU apply (host code,
+// no CUDA: the plan is checked on the CPU by tests/test_ilu_records.py).
+//
+// A sweep of one subdomain is a list of tasks, each up to six rows of one
+// wavefront level (a warp, five lanes a row).  Task t belongs to compute warp
+// t mod W; consecutive tasks form groups, and a group is one contiguous byte
+// range that one bulk copy brings into a shared-memory stage:
+//
+//   16 B    group header: tasks of the group, first row, tasks of the sweep,
+//           levels of the sweep
+//   32 B    per task:
+//     w0    columns/16 | values/16 << 16      offsets from the group start
+//     w1    n | S << 8 | flags << 16 | dl << 24    rows; slots of the longest
+//           row; levels from here to the warp's next task (or to the last)
+//     w2    first row
+//     w3    level-buffer row of the first row (0xffff: level not kept)
+//           | blocks << 16
+//     w4    rows that have more than k slots, k = 0..3 (a byte each)
+//     w5-6  row of the task at each position (six bytes) | level << 16
+//     w7    index of the warp's next task in its group | groups to get there
+//           << 8 | first row less the group's << 16
+//   then per task
+//     columns  max(1, ceil(S/4)) x [n] int4: >= 0 byte offset of the row in
+//              the level buffers (a row of zeros past them where the row has
+//              no such slot), < 0 row -v - 1 of the global vector; with more
+//              than four slots, 16 bytes: rows that have more than k slots
+//     values   the blocks' rows of five entries, in vector pieces so that
+//              lane (position, component) of a slot reads whole 16-byte (8
+//              for BF16) words, neighbouring lanes neighbouring words:
+//              FP64  [5 blocks] double2 (entries 0, 1), [5 blocks] double2
+//                    (2, 3), [5 blocks] double (4)
+//              FP32  [5 blocks] float4 (0..3), [5 blocks] float (4)
+//              BF16  [5 blocks] four bf16 (0..3), [5 blocks] bf16 (4)
+//
+// The rows of a task are held in descending order of their slot counts, so
+// the blocks of slot k are those of the first n_k positions: block number
+// n_0 + ... + n_{k-1} + position.  Backward the pivot inverses come first
+// (n blocks).  Only stored blocks take space.
+#pragma once
+
+#include <algorithm>
+#include <cstdint>
+#include <cstring>
+#include <vector>
+
+namespace rdst {
+
+constexpr int REC_ROWS = 6;             // rows of a task
+constexpr int REC_MAXW = 8;             // compute warps at most
+constexpr int REC_MAXS = 16;            // slots of a row at most
+// Stages, and the bytes of one at most.  A group's end costs every warp a
+// wait and the producer a round trip, so two large stages beat more and
+// smaller ones (1.2 M-cell wing FP32: two 196 -> 187 us against three, 256
+// against six; 442 k-cell wing FP64 with 16 / 24 / 32 KB: 140 / 111 / 110 us).
+// The first two groups of a sweep are smaller: nothing runs before the first.
+constexpr int REC_STAGES = 2;
+constexpr size_t REC_STAGE_CAP = 65536, REC_RAMP0 = 8192, REC_RAMP1 = 20480;
+constexpr int REC_WARP_LAST = 1;        // the warp's last task of the sweep
+constexpr int REC_FAR = 2;              // some column lies in the global vector
+
+struct RecGroup { uint32_t off16; uint32_t bytes; int32_t row0; int32_t nrows; };
+struct RecTask { uint32_t head16; uint32_t group16; };   // a task's header and its group, from the records' start / 16
+
+struct RecSide {
+    std::vector<unsigned char> rec;
+    std::vector<RecGroup> groups;
+    std::vector<int> part_g;            // first group of each part
+    std::vector<RecTask> tasks;
+};
+
+struct RecPlan {
+    bool ok = false;
+    int warps = 0;                      // compute warps W
+    bool tight = false;                 // the instance for five or six CTAs an SM
+    int stage_bytes = 0;                // largest group, multiple of 128
+    int y0_rows = 0;                    // rows of a stage's starting values (even)
+    int lb_rows = 0;                    // rows of each of the two level buffers
+    RecSide f, b;
+};
+
+// bytes of one level-buffer row: five values in the compute type, padded to
+// 16-byte words
+inline int rec_lb_row_bytes(int elem) { return elem == 8 ? 48 : 32; }
+
+inline size_t rec_smem(const RecPlan& P, int elem) {
+    return (size_t)REC_STAGES * (P.stage_bytes + 40 * (size_t)P.y0_rows) +
+           (2 * (size_t)P.lb_rows + 1) * rec_lb_row_bytes(elem);
+}
+
+// Plan for factors of `elem` bytes.  Rows of part p are the levels
+// part_lvl0[p] .. part_lvl0[p+1]-1, level l the rows lvl_off[l] ..
+// lvl_off[l+1]-1; factor slot s of row r has id ((r/32) MS + s) 32 + r % 32
+// and column lu_col[id]; nl lower slots from s = 0, nu upper ones from ML
+// (nu 0: the backward sweep applies the pivot inverses alone).
+inline RecPlan rec_plan(int N, int nparts, const std::vector<int>& part_lvl0, const std::vector<int>& lvl_off,
+                        const std::vector<int>& lu_col, const std::vector<int>& nl, const std::vector<int>& nu, int ML,
+                        int MS, int elem, int sms, size_t smem_sm, size_t smem_block, size_t reserved) {
+    RecPlan P;
+    const int nlev = (int)lvl_off.size() - 1;
+    std::vector<int> lev(N);
+    int maxw = 0;
+    for (int l = 0; l < nlev; ++l) {
+        maxw = std::max(maxw, lvl_off[l + 1] - lvl_off[l]);
+        for (int r = lvl_off[l]; r < lvl_off[l + 1]; ++r) lev[r] = l;
+    }
+    auto fid = [&](int r, int s) { return ((r >> 5) * MS + s) * 32 + (r & 31); };
+    auto r16 = [](size_t v) { return (v + 15) / 16 * 16; };
+    // CTAs an SM has to hold for all subdomains to run at once, six at most
+    // (a larger number runs in turns)
+    const int k = std::min(6, std::max(1, (nparts + sms - 1) / std::max(sms, 1)));
+    // Compute warps.  A warp spends longer on bringing a task's data into
+    // registers than on the part of it that waits for the level before, so
+    // even levels of one task want several warps taking turns (four: airfoil
+    // 34.4 us, eight 35.9), and wider levels as many as there are (110 k-cell
+    // wing FP64, 3.5 tasks a level: four 54.8, six 50.7, eight 48.6 us).  The
+    // registers of k CTAs bound the number: 96 a thread up to four CTAs; with
+    // five or six three warps of 80, two of 112 with FP64.
+    P.tight = k >= 5;
+    const int wmax = P.tight ? (elem == 8 ? 2 : 3) : std::min(REC_MAXW, 21 / k - 1);
+    const int want = N > REC_ROWS * nlev ? REC_MAXW : 4;
+    const size_t budget = std::min(smem_block, smem_sm / k - reserved) - 1024;    // static shared memory, alignment
+
+    struct Task { int r0, n, l; };
+    for (int W = std::min(wmax, want); W > 0; W /= 2) {
+        P.warps = W;
+        const int lbr = rec_lb_row_bytes(elem);
+        P.lb_rows = (int)std::min<size_t>(maxw, budget / 2 / (2 * (size_t)lbr));
+        P.lb_rows = std::min(P.lb_rows, 16383);
+        auto cnt = [&](int r, bool back) { return back ? nu[r] : nl[r]; };
+        // tasks of a sweep; the backward chunks of a level descend, so that
+        // consecutive tasks always cover one contiguous row range
+        auto tasks_of = [&](int p, bool back) {
+            std::vector<Task> t;
+            const int a = part_lvl0[p], e = part_lvl0[p + 1];
+            for (int i = 0; i < e - a; ++i) {
+                const int l = back ? e - 1 - i : a + i;
+                const int r0 = lvl_off[l], n = lvl_off[l + 1] - r0, nc = (n + REC_ROWS - 1) / REC_ROWS;
+                for (int c = 0; c < nc; ++c) {
+                    const int cc = back ? nc - 1 - c : c;
+                    t.push_back({r0 + cc * REC_ROWS, std::min(REC_ROWS, n - cc * REC_ROWS), l});
+                }
+            }
+            return t;
+        };
+        auto widest = [&](const Task& t, bool back) {
+            int S = 0;
+            for (int i = 0; i < t.n; ++i) S = std::max(S, cnt(t.r0 + i, back));
+            return S;
+        };
+        auto data_bytes = [&](const Task& t, bool back) {
+            const int S = widest(t, back);
+            size_t tot = back ? t.n : 0;
+            for (int i = 0; i < t.n; ++i) tot += cnt(t.r0 + i, back);
+            return (size_t)16 * t.n * std::max(1, (S + 3) / 4) + (S > 4 ? 16 : 0) + r16(tot * 25 * elem);
+        };
+        size_t max_one = 0, total[2] = {0, 0}, ntasks[2] = {0, 0};
+        for (int p = 0; p < nparts; ++p)
+            for (int back = 0; back < 2; ++back)
+                for (const Task& t : tasks_of(p, back)) {
+                    const size_t b = 32 + data_bytes(t, back);
+                    max_one = std::max(max_one, b);
+                    total[back] += b;
+                    ++ntasks[back];
+                }
+        // a warp may hold a stage until its task is computed while another
+        // waits W - 1 tasks further on: that window must fit the stages
+        const size_t room = budget - (2 * (size_t)P.lb_rows + 1) * lbr;
+        const size_t qmin = std::max(1, W - 1), least = 16 + qmin * max_one;
+        size_t cap = room / REC_STAGES;           // a stage: its group and the rows' starting values
+        if (cap < least + 40 * qmin * REC_ROWS + 256) continue;      // 256: rounding of both parts
+        cap = std::max(least + 40 * qmin * REC_ROWS, std::min(cap - 256, REC_STAGE_CAP));
+        // rows of a group of the mean size, never fewer than qmin tasks'
+        const size_t mean = std::max(total[0], total[1]) / N + 40;
+        const size_t cap_rows = std::max<size_t>(qmin * REC_ROWS, std::min((cap - least) / 40, cap / mean));
+        const size_t cap_bytes = cap - 40 * cap_rows;
+        // ---- groups
+        size_t max_group = 0;
+        int max_rows = 0;
+        for (int back = 0; back < 2; ++back) {
+            RecSide& S = back ? P.b : P.f;
+            S.rec.clear();
+            S.rec.reserve(total[back] + 16 * ntasks[back]);
+            S.groups.clear();
+            S.tasks.clear();
+            S.part_g.assign(nparts + 1, 0);
+            for (int p = 0; p < nparts; ++p) {
+                S.part_g[p] = (int)S.groups.size();
+                const std::vector<Task> ts = tasks_of(p, back);
+                // group bounds and, per task, its group and place there
+                std::vector<size_t> gstart(1, 0);
+                std::vector<int> grp(ts.size()), place(ts.size());
+                {
+                    size_t bytes = 16, rows = 0;
+                    for (size_t t = 0; t < ts.size(); ++t) {
+                        const size_t b = 32 + data_bytes(ts[t], back), in = t - gstart.back();
+                        const size_t most = gstart.size() == 1 ? REC_RAMP0 : gstart.size() == 2 ? REC_RAMP1 : cap_bytes;
+                        if (in >= qmin && (bytes + b > std::min(most, cap_bytes) || rows + ts[t].n > cap_rows || in >= 255)) {
+                            gstart.push_back(t);
+                            bytes = 16;
+                            rows = 0;
+                        }
+                        bytes += b;
+                        rows += ts[t].n;
+                        grp[t] = (int)gstart.size() - 1;
+                        place[t] = (int)(t - gstart.back());
+                    }
+                    gstart.push_back(ts.size());
+                }
+                const int nlv = part_lvl0[p + 1] - part_lvl0[p];
+                for (size_t gi = 0; gi + 1 < gstart.size(); ++gi) {
+                    const size_t i = gstart[gi], j = gstart[gi + 1];
+                    int lo = ts[i].r0, hi = lo;
+                    size_t bytes = 16 + 32 * (j - i);
+                    for (size_t t = i; t < j; ++t) {
+                        lo = std::min(lo, ts[t].r0);
+                        hi = std::max(hi, ts[t].r0 + ts[t].n);
+                        bytes += data_bytes(ts[t], back);
+                    }
+                    const size_t g0 = S.rec.size();
+                    S.rec.resize(g0 + bytes, 0);
+                    unsigned char* g = S.rec.data() + g0;
+                    const int32_t gh[4] = {(int32_t)(j - i), lo, (int32_t)ts.size(), nlv};
+                    std::memcpy(g, gh, 16);
+                    size_t pos = 16 + 32 * (j - i);
+                    for (size_t t = i; t < j; ++t) {
+                        const Task& T = ts[t];
+                        int ord[REC_ROWS];
+                        for (int q = 0; q < T.n; ++q) ord[q] = q;
+                        std::stable_sort(ord, ord + T.n, [&](int a, int b2) {
+                            return cnt(T.r0 + a, back) > cnt(T.r0 + b2, back);
+                        });
+                        const int Sx = widest(T, back), nq = std::max(1, (Sx + 3) / 4);
+                        unsigned char nk[REC_MAXS] = {0};
+                        int tot = back ? T.n : 0;
+                        for (int q = 0; q < T.n; ++q)
+                            for (int s = 0; s < cnt(T.r0 + q, back); ++s) { ++nk[s]; ++tot; }
+                        const size_t coff = pos, voff = coff + (size_t)16 * T.n * nq + (Sx > 4 ? 16 : 0);
+                        if (Sx > 4) std::memcpy(g + voff - 16, nk, REC_MAXS);
+                        // levels as wide as the buffers are kept there
+                        auto kept = [&](int l) { return lvl_off[l + 1] - lvl_off[l] <= P.lb_rows; };
+                        const int own = kept(T.l) ? (T.l & 1) * P.lb_rows + T.r0 - lvl_off[T.l] : 0xffff;
+                        int32_t* cols = reinterpret_cast<int32_t*>(g + coff);
+                        for (int q = 0; q < T.n * 4 * nq; ++q) cols[q] = 2 * P.lb_rows * lbr;
+                        bool far = false;
+                        for (int s = 0; s < Sx; ++s)
+                            for (int q = 0; q < nk[s]; ++q) {
+                                const int c = lu_col[fid(T.r0 + ord[q], back ? ML + s : s)];
+                                const int lp = back ? T.l + 1 : T.l - 1;      // the level taken just before
+                                const bool near = lev[c] == lp && kept(lp);
+                                cols[((size_t)(s / 4) * T.n + q) * 4 + s % 4] =
+                                    near ? ((lp & 1) * P.lb_rows + c - lvl_off[lp]) * lbr : -1 - c;
+                                far |= !near;
+                            }
+                        // sweep-relative level, and the way to the warp's next task
+                        auto level_of = [&](size_t tt) {
+                            return back ? part_lvl0[p + 1] - 1 - ts[tt].l : ts[tt].l - part_lvl0[p];
+                        };
+                        const bool last = t + W >= ts.size();
+                        const int dl = last ? 0 : level_of(t + W) - level_of(t);
+                        const uint32_t fl = (last ? REC_WARP_LAST : 0) | (far ? REC_FAR : 0);
+                        uint32_t h[8] = {(uint32_t)(coff / 16) | (uint32_t)(voff / 16) << 16,
+                                         (uint32_t)T.n | (uint32_t)Sx << 8 | fl << 16 | (uint32_t)dl << 24,
+                                         (uint32_t)T.r0, (uint32_t)own | (uint32_t)tot << 16, 0u, 0u,
+                                         (uint32_t)level_of(t) << 16,
+                                         (last ? 0u : (uint32_t)place[t + W] | (uint32_t)(grp[t + W] - grp[t]) << 8) |
+                                             (uint32_t)(T.r0 - lo) << 16};
+                        for (int q = 0; q < 4; ++q) h[4] |= (uint32_t)nk[q] << (8 * q);
+                        for (int q = 0; q < T.n; ++q) h[5 + q / 4] |= (uint32_t)ord[q] << (8 * (q % 4));
+                        std::memcpy(g + 16 + 32 * (t - i), h, 32);
+                        S.tasks.push_back({(uint32_t)((g0 + 16 + 32 * (t - i)) / 16), (uint32_t)(g0 / 16)});
+                        pos += data_bytes(T, back);
+                    }
+                    S.groups.push_back({(uint32_t)(g0 / 16), (uint32_t)bytes, lo, hi - lo});
+                    max_group = std::max(max_group, bytes);
+                    max_rows = std::max(max_rows, hi - lo);
+                }
+            }
+            S.part_g[nparts] = (int)S.groups.size();
+        }
+        P.stage_bytes = (int)((max_group + 127) / 128 * 128);
+        P.y0_rows = (max_rows + 1) / 2 * 2;
+        if (rec_smem(P, elem) > budget) continue;
+        P.ok = true;
+        return P;
+    }
+    return P;
+}
+
+}  // namespace rdst
