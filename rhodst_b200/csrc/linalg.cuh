@@ -1130,149 +1130,16 @@ __global__ void __launch_bounds__(RED_TPB) k_multidot(long n, int nv, const doub
     }
 }
 
-// Deterministic block reduction of NV per-thread values: warp shuffles,
-// then one fixed-order sum over the warps; result -> partial[blk*pstride+j].
-template <int NV>
-__device__ __forceinline__ void block_multi_sum(double (&acc)[NV], int nv, double* __restrict__ partial, int pstride) {
-    __shared__ double sh[RED_TPB / 32][NV];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        if (j < nv) {
-            double v = warp_sum(acc[j]);
-            if (lane == 0) sh[wid][j] = v;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < nv) {
-        double v = 0;
-        for (int w2 = 0; w2 < (int)(blockDim.x >> 5); ++w2) v += sh[w2][threadIdx.x];
-        partial[(long)blockIdx.x * pstride + threadIdx.x] = v;
-    }
-}
-
-// partial[blk][j] = sum_i V_j[i] w[i] for j < nv <= NV (one pass over w)
-// Four consecutive entries of a vector as doubles (16-byte loads; the
-// caller guarantees 4-entry alignment of p), or fewer at the vector's end.
-__device__ __forceinline__ void load4(const double* __restrict__ p, double (&o)[4]) {
+// Four consecutive entries of a vector as doubles (16-byte loads, p aligned
+// to 16 bytes).
+__device__ __forceinline__ void load4(const double* p, double (&o)[4]) {
     const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
     o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
 }
-__device__ __forceinline__ void load4(const float* __restrict__ p, double (&o)[4]) {
+__device__ __forceinline__ void load4(const float* p, double (&o)[4]) {
     const float4 a = *reinterpret_cast<const float4*>(p);
     o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
 }
-template <typename T>
-__device__ __forceinline__ void load4_tail(const T* __restrict__ p, long rem, double (&o)[4]) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[e] = e < rem ? tod(p[e]) : 0.0;
-}
-template <typename T>
-__device__ __forceinline__ void load4_any(const T* __restrict__ p, long i0, long n, double (&o)[4]) {
-    if (i0 + 4 <= n) load4(p + i0, o);
-    else load4_tail(p + i0, n - i0, o);
-}
-
-// partial[blk * pstride + j] = sum_i V_j[i] w[i], j < nv: four entries per
-// thread and 16-byte loads; V (fp64 or fp32) has a row stride ldv that is
-// a multiple of 4 entries.  Full chunks take a branch-free path so that
-// the loads of all nv vectors are in flight together.
-template <int NV, typename VT = double>
-__global__ void __launch_bounds__(RED_TPB, 2) k_vmultidot(long n, int nv, const VT* __restrict__ V, long ldv,
-                                                       const double* __restrict__ w, double* __restrict__ partial,
-                                                       int pstride, const int* __restrict__ active) {
-    if (active && !*active) return;
-    double acc[NV];
-#pragma unroll
-    for (int j = 0; j < NV; ++j) acc[j] = 0.0;
-    const long nc = (n + 3) / 4, nfull = n / 4;
-    for (long c = (long)blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += (long)gridDim.x * blockDim.x) {
-        const long i0 = 4 * c;
-        double wv[4];
-        if (c < nfull) {
-            load4(w + i0, wv);
-#pragma unroll
-            for (int j = 0; j < NV; ++j)
-                if (j < nv) {
-                    double v[4];
-                    load4(V + j * ldv + i0, v);
-                    acc[j] += v[0] * wv[0] + v[1] * wv[1] + v[2] * wv[2] + v[3] * wv[3];
-                }
-        } else {
-            load4_tail(w + i0, n - i0, wv);
-            for (int j = 0; j < nv && j < NV; ++j) {
-                double v[4];
-                load4_tail(V + j * ldv + i0, n - i0, v);
-                acc[j] += v[0] * wv[0] + v[1] * wv[1] + v[2] * wv[2] + v[3] * wv[3];
-            }
-        }
-    }
-    block_multi_sum<NV>(acc, nv, partial, pstride);
-}
-
-// w -= sum_j coef[j] V_j (j < nv), then in the same pass either the dots
-// V_j . w_new (mode 0: the second CGS2 pass) or w_new . w_new (mode 1);
-// four entries per thread as in k_vmultidot
-template <int NV, typename VT = double>
-__global__ void __launch_bounds__(RED_TPB, 2) k_maxpy_dot(long n, int nv, const VT* __restrict__ V, long ldv,
-                                                       const double* __restrict__ coef, double* __restrict__ w,
-                                                       double* __restrict__ partial, int pstride, int mode,
-                                                       const int* __restrict__ active) {
-    if (active && !*active) return;
-    __shared__ double cs[NV];
-    if (threadIdx.x < NV) cs[threadIdx.x] = threadIdx.x < nv ? coef[threadIdx.x] : 0.0;
-    __syncthreads();
-    double acc[NV];
-#pragma unroll
-    for (int j = 0; j < NV; ++j) acc[j] = 0.0;
-    const long nc = (n + 3) / 4, nfull = n / 4;
-    for (long c = (long)blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += (long)gridDim.x * blockDim.x) {
-        const long i0 = 4 * c;
-        double a[4];
-        if (c < nfull) {
-            load4(w + i0, a);
-#pragma unroll
-            for (int j = 0; j < NV; ++j)
-                if (j < nv) {
-                    double v[4];
-                    load4(V + j * ldv + i0, v);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) a[e] -= cs[j] * v[e];
-                }
-            reinterpret_cast<double2*>(w + i0)[0] = make_double2(a[0], a[1]);
-            reinterpret_cast<double2*>(w + i0)[1] = make_double2(a[2], a[3]);
-            if (mode == 0) {
-                // second read of V_j: the lines were just fetched (L1 hit)
-#pragma unroll
-                for (int j = 0; j < NV; ++j)
-                    if (j < nv) {
-                        double v[4];
-                        load4(V + j * ldv + i0, v);
-                        acc[j] += v[0] * a[0] + v[1] * a[1] + v[2] * a[2] + v[3] * a[3];
-                    }
-            }
-        } else {
-            load4_tail(w + i0, n - i0, a);
-            for (int j = 0; j < nv && j < NV; ++j) {
-                double v[4];
-                load4_tail(V + j * ldv + i0, n - i0, v);
-                for (int e = 0; e < 4; ++e) a[e] -= cs[j] * v[e];
-            }
-            for (int e = 0; e < 4; ++e)
-                if (i0 + e < n) w[i0 + e] = a[e];
-            if (mode == 0) {
-                for (int j = 0; j < nv && j < NV; ++j) {
-                    double v[4];
-                    load4_tail(V + j * ldv + i0, n - i0, v);
-                    acc[j] += v[0] * a[0] + v[1] * a[1] + v[2] * a[2] + v[3] * a[3];
-                }
-            }
-        }
-        if (mode != 0) acc[0] += a[0] * a[0] + a[1] * a[1] + a[2] * a[2] + a[3] * a[3];
-    }
-    block_multi_sum<NV>(acc, mode == 0 ? nv : 1, partial, pstride);
-}
-
 // out[j] = sum_b partial[b * pstride + j] (fixed order); optional sqrt
 __global__ void k_finalize(const double* __restrict__ partial, int nb, int nv, int pstride, double* __restrict__ out,
                            int take_sqrt, const int* __restrict__ active) {
@@ -1283,34 +1150,6 @@ __global__ void k_finalize(const double* __restrict__ partial, int nb, int nv, i
     for (int b = threadIdx.x; b < nb; b += blockDim.x) s += partial[(long)b * pstride + j];
     s = block_sum(s);
     if (threadIdx.x == 0) out[j] = take_sqrt ? sqrt(s) : s;
-}
-
-// w -= sum_j coef[j] V_j (j < nv); coef on the device
-template <typename VT = double>
-__global__ void k_maxpy(long n, int nv, const VT* __restrict__ V, long ldv, const double* __restrict__ coef,
-                        double* __restrict__ w, double sign, const int* __restrict__ active) {
-    if (active && !*active) return;
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double a = w[i];
-    for (int j = 0; j < nv; ++j) a -= sign * coef[j] * tod(V[j * ldv + i]);
-    w[i] = a;
-}
-
-// x /= *s
-__global__ void k_scale_inv(long n, double* __restrict__ x, const double* __restrict__ s, const int* __restrict__ active) {
-    if (active && !*active) return;
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) x[i] = x[i] / *s;
-}
-
-// v = w / *s stored as a (FP32) basis vector
-template <typename VT>
-__global__ void k_scale_store(long n, const double* __restrict__ w, VT* __restrict__ v, const double* __restrict__ s,
-                              const int* __restrict__ active) {
-    if (active && !*active) return;
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) v[i] = (VT)(w[i] / *s);
 }
 
 // per-component sum |r_c| and the foam normFactor pieces
@@ -1409,49 +1248,609 @@ __global__ void k_check(Scalars* sc, double tol, double relTol, int minIter, int
 }
 
 // ---------------------------------------------------------------- GMRES
-__global__ void k_gm_start(Scalars* sc) {
-    if (threadIdx.x != 0) return;
-    for (int i = 0; i < 65; ++i) sc->bh[i] = 0.0;
-    for (int i = 0; i < 64 * 65; ++i) sc->H[i] = 0.0;
-    sc->bh[0] = sc->beta;
-    sc->gm_active = (sc->beta != 0.0);
-    sc->gm_used = 0;
+// One Arnoldi vector's orthogonalisation in one cooperative launch (FP64
+// basis; k_orth_cgs2 for FP32).
+//
+// The basis is what this path reads (V: nv vectors, 4 or 8 bytes an entry),
+// so it is read twice, not three times as two classical Gram-Schmidt passes
+// with their own dot products would: the first pass takes h = V^T w and, in
+// the same read, e = V^T v of the newest basis vector v, the new column of
+// the Gram matrix G = V^T V.  The coefficients that a second pass would add,
+// V^T (w - V h), are then h - G h without touching V, which takes out what
+// the basis itself lacks in orthogonality; the second read subtracts c = 2 h - G h.  Rounding of w - V c
+// is amplified by |w| / |w - V c|, so where that ratio exceeds 100 a true
+// second pass follows (a branch that all blocks take together).
+//
+// A launch per pass and one per sum costs more than the passes themselves up
+// to about 1e5 unknowns; the passes are therefore separated by a grid-wide
+// barrier (all blocks resident: cooperative launch), each block adding up
+// the blocks' partial sums by itself in the same order.  The second read
+// runs through the vectors backwards: what the first read last is still in
+// L2 (126 MB).  In the dot pass a thread takes four consecutive entries of
+// eight vectors, two groups of warps sharing the sixteen of a round (that
+// leaves registers for loads in flight); in the others two entries of all
+// vectors.  Vectors are padded to 64 entries of
+// zeros, so no load needs a test for the end.
+//
+// Per direction, mean of 20 (before: dots, update and dots, update and norm,
+// each with its own sum, then the Givens rotation and the scaling, ten
+// launches): 4 k cells 45 -> 13 us, 442 k 170 -> 88.
+constexpr int ORTH_TPB = 512;
+constexpr int ORTH_PIECES = ORTH_TPB / 2;       // four-entry pieces a block takes at a time
+constexpr int ORTH_NV = 8;                      // basis vectors whose dots a thread holds at once
+constexpr int ORTH_MAXV = 64;                   // GMRES directions at most
+constexpr int ORTH_COLS = 3 * ORTH_MAXV + 3;    // partial sums per block: h, e, |w|^2, |w|^2 after each pass, h of the second
+constexpr double ORTH_AGAIN = 1.0e-4;           // |w - V c|^2 below this part of |w|^2: a second pass
+
+// the warp's sums of 16 values: lane l gets that of a[l / 2]
+__device__ __forceinline__ double warp_sum16(double (&a)[16]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16; o > 1; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o / 2; ++i) {
+            const double send = up ? a[i] : a[i + o / 2], keep = up ? a[i + o / 2] : a[i];
+            a[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
 }
 
-// H[:,i] = h1 + h2 (CGS2), Givens rotations (foam givensRotation), bh
-__global__ void k_gm_givens(Scalars* sc, int i, int m) {
-    if (threadIdx.x != 0 || !sc->gm_active) return;
-    double* H = sc->H;
-    for (int j = 0; j <= i; ++j) H[j * m + i] = sc->hcol[0][j] + sc->hcol[1][j];
-    double beta = sc->beta;
-    for (int j = 0; j < i; ++j) {
-        double Hji = H[j * m + i];
-        H[j * m + i] = sc->cs[j] * Hji - sc->sn[j] * H[(j + 1) * m + i];
-        H[(j + 1) * m + i] = sc->sn[j] * Hji + sc->cs[j] * H[(j + 1) * m + i];
+// all blocks of a cooperative launch; false after 2 s (bit 2 of *flags)
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, int* flags) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        unsigned v;
+        unsigned long long t0 = 0;
+        int ok = 0;
+        for (unsigned it = 0;; ++it) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            if (v >= target) { ok = 1; break; }
+            if ((it & 255u) == 255u) {
+                const unsigned long long now = globaltimer_ns();
+                if (t0 == 0) t0 = now;
+                else if (now - t0 > 2000000000ull) { atomicOr(flags, 4); break; }
+            }
+        }
+        s_ok = ok;
     }
-    double hh = H[i * m + i], c, s;
+    __syncthreads();
+    return s_ok != 0;
+}
+
+// out[c] = sum over the blocks of part[c * nb + block], c < ncol, by all
+// threads of the block (a warp per column, eight columns in flight)
+__device__ __forceinline__ void sum_columns(const double* part, int ncol, int nb, double* out) {
+    constexpr int NW = ORTH_TPB / 32;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int c0 = 0; c0 < ncol; c0 += 8 * NW) {
+        double s[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s[q] = 0.0;
+        for (int b = lane; b < nb; b += 32)
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (c0 + wid + NW * q < ncol) s[q] += __ldcg(part + (size_t)(c0 + wid + NW * q) * nb + b);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (c0 + wid + NW * q < ncol) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+                if (lane == 0) out[c0 + wid + NW * q] = s[q];
+            }
+    }
+    __syncthreads();
+}
+
+// two consecutive entries as doubles
+__device__ __forceinline__ void load2(const double* p, double (&o)[2]) {
+    const double2 a = *reinterpret_cast<const double2*>(p);
+    o[0] = a.x; o[1] = a.y;
+}
+__device__ __forceinline__ void load2(const float* p, double (&o)[2]) {
+    const float2 a = *reinterpret_cast<const float2*>(p);
+    o[0] = a.x; o[1] = a.y;
+}
+// two entries stored, the padding past n left as it is
+__device__ __forceinline__ void store2(double* p, long i0, long n, const double (&a)[2]) {
+    if (i0 + 2 <= n) *reinterpret_cast<double2*>(p + i0) = make_double2(a[0], a[1]);
+    else if (i0 < n) p[i0] = a[0];
+}
+__device__ __forceinline__ void store2(float* p, long i0, long n, const double (&a)[2]) {
+    if (i0 + 2 <= n) *reinterpret_cast<float2*>(p + i0) = make_float2((float)a[0], (float)a[1]);
+    else if (i0 < n) p[i0] = (float)a[0];
+}
+// a -= sum_j c_j V_j at entries i0, i0 + 1
+template <typename VT>
+__device__ __forceinline__ void orth_subtract(const VT* V, long ldv, int nv, const double* c, long i0, double (&a)[2]) {
+    int j = 0;
+    for (; j + 8 <= nv; j += 8) {
+        double v[8][2];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) load2(V + (j + q) * ldv + i0, v[q]);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) { a[0] -= c[j + q] * v[q][0]; a[1] -= c[j + q] * v[q][1]; }
+    }
+    if (j < nv) {
+        double v[7][2];
+#pragma unroll
+        for (int q = 0; q < 7; ++q)
+            if (j + q < nv) load2(V + (j + q) * ldv + i0, v[q]);
+#pragma unroll
+        for (int q = 0; q < 7; ++q)
+            if (j + q < nv) { a[0] -= c[j + q] * v[q][0]; a[1] -= c[j + q] * v[q][1]; }
+    }
+}
+
+// the cycle's start (one block): bh = beta e_0
+__device__ __forceinline__ void gm_start(Scalars* sc, double beta) {
+    for (int q = threadIdx.x; q < 65; q += blockDim.x) sc->bh[q] = q == 0 ? beta : 0.0;
+    if (threadIdx.x == 0) {
+        sc->beta = beta;
+        sc->gm_active = beta != 0.0;
+        sc->gm_used = 0;
+    }
+}
+// H(:, i) = h with the earlier rotations, its own (foam givensRotation) and
+// bh (one block; the rotations come through shared memory)
+__device__ __forceinline__ void gm_rotate(Scalars* sc, const double* h, double* s_cs, double* s_sn, int i, int m,
+                                          double beta) {
+    __syncthreads();
+    if ((int)threadIdx.x < i) { s_cs[threadIdx.x] = sc->cs[threadIdx.x]; s_sn[threadIdx.x] = sc->sn[threadIdx.x]; }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    double hh = h[0];
+    for (int j = 0; j < i; ++j) {
+        const double Hji = hh, Hn = h[j + 1];
+        sc->H[j * m + i] = s_cs[j] * Hji - s_sn[j] * Hn;
+        hh = s_sn[j] * Hji + s_cs[j] * Hn;
+    }
+    double c, s;
     if (beta == 0.0) { c = 1; s = 0; }
     else if (fabs(beta) > fabs(hh)) { double tau = -hh / beta; s = 1.0 / sqrt(1.0 + tau * tau); c = s * tau; }
     else { double tau = -beta / hh; c = 1.0 / sqrt(1.0 + tau * tau); s = c * tau; }
     sc->cs[i] = c;
     sc->sn[i] = s;
-    double bhi = sc->bh[i];
-    sc->bh[i] = c * bhi - s * sc->bh[i + 1];
-    sc->bh[i + 1] = s * bhi + c * sc->bh[i + 1];
-    H[i * m + i] = c * H[i * m + i] - s * beta;
+    const double bhi = sc->bh[i], bhn = sc->bh[i + 1];
+    sc->bh[i] = c * bhi - s * bhn;
+    sc->bh[i + 1] = s * bhi + c * bhn;
+    sc->H[i * m + i] = c * hh - s * beta;
+    sc->beta = beta;
     sc->gm_used = i + 1;
     if (beta == 0.0) sc->gm_active = 0;
 }
+// the last block out leaves the barrier as the next launch needs it
+__device__ __forceinline__ void grid_leave(Scalars* sc) {
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&sc->orth_out, 1u) == gridDim.x - 1) { sc->orth_bar = 0; sc->orth_out = 0; }
+}
 
-__global__ void k_gm_backsub(Scalars* sc, int m) {
-    if (threadIdx.x != 0) return;
-    int used = sc->gm_used;
-    for (int i = used - 1; i >= 0; --i) {
-        double sum = sc->bh[i];
-        for (int j = i + 1; j < used; ++j) sum -= sc->H[i * m + j] * sc->yh[j];
-        sc->yh[i] = sum / sc->H[i * m + i];
+// Orthogonalise w against V_0 .. V_{nv-1}, beta = |w|, and (vout) V_nv =
+// w / beta; H(:, nv-1), its Givens rotation and bh by the first block.  nv 0
+// starts a cycle: beta = |w|, V_0 = w / beta, bh = beta e_0.  w may be vout
+// (FP64 basis).  partial: ORTH_COLS columns of gridDim.x doubles.
+template <typename VT>
+__global__ void __launch_bounds__(ORTH_TPB, 1)
+    k_orth(long n, int nv, const VT* V, long ldv, double* w, VT* vout, double* partial, Scalars* sc, int m) {
+    if (nv > 0 && !sc->gm_active) return;
+    constexpr int NW = ORTH_TPB / 32;
+    __shared__ double s_red[NW][17];
+    __shared__ double s_col[2 * ORTH_MAXV + 1], s_c[ORTH_MAXV], s_b[2];
+    extern __shared__ double s_G[];                 // [nv][nv]
+    const int nb = gridDim.x, blk = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int group = tid / ORTH_PIECES;            // which eight vectors of sixteen, which half of a piece
+    const long nc = (n + 3) / 4, stride = (long)nb * ORTH_PIECES, c0 = (long)blk * ORTH_PIECES + tid % ORTH_PIECES;
+    const bool single = nc <= stride;               // one piece a thread pair: w stays in registers
+    const int i = nv - 1;
+    for (int q = tid; q < i * i; q += ORTH_TPB) s_G[(q / i) * nv + q % i] = sc->G[(q / i) * ORTH_MAXV + q % i];
+    unsigned round = 0;
+    auto barrier = [&] { return grid_barrier(&sc->orth_bar, ++round * (unsigned)nb, &sc->flags); };
+    // sum of x over the block into column col
+    auto block_col = [&](double x, int col) {
+        x = warp_sum(x);
+        if (lane == 0) s_red[wid][16] = x;
+        __syncthreads();
+        if (tid == 0) {
+            double s = 0;
+            for (int q = 0; q < NW; ++q) s += s_red[q][16];
+            partial[(size_t)col * nb + blk] = s;
+        }
+        __syncthreads();
+    };
+    double keep[2] = {0, 0};                        // single: this thread's half of w
+    // V^T w into columns col.., V^T V_i into columns ecol.. (if >= 0)
+    auto dots = [&](int col, int ecol) {
+        for (int jb = 0; jb < nv; jb += 2 * ORTH_NV) {
+            const int j0 = jb + ORTH_NV * group, cnt = min(ORTH_NV, nv - j0);
+            double acc[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) acc[q] = 0.0;
+            auto piece = [&](long i0, auto full) {
+                double wv[4], vi[4];
+                load4(w + i0, wv);
+                load4(V + i * ldv + i0, vi);
+#pragma unroll
+                for (int j = 0; j < ORTH_NV; ++j)
+                    if (decltype(full)::value || j < cnt) {
+                        double v[4];
+                        load4(V + (j0 + j) * ldv + i0, v);
+                        acc[j] += v[0] * wv[0] + v[1] * wv[1] + v[2] * wv[2] + v[3] * wv[3];
+                        acc[8 + j] += v[0] * vi[0] + v[1] * vi[1] + v[2] * vi[2] + v[3] * vi[3];
+                    }
+            };
+            if (cnt >= ORTH_NV) for (long c = c0; c < nc; c += stride) piece(4 * c, std::true_type{});
+            else if (cnt > 0) for (long c = c0; c < nc; c += stride) piece(4 * c, std::false_type{});
+            const double s = warp_sum16(acc);
+            if ((lane & 1) == 0) s_red[wid][lane >> 1] = s;
+            __syncthreads();
+            if (tid < 32) {
+                const int g = tid >> 4, q = tid & 15, j = jb + ORTH_NV * g + (q & 7);
+                if (j < nv && (q < 8 || ecol >= 0)) {
+                    double t = 0;
+                    for (int k = 0; k < NW / 2; ++k) t += s_red[g * (NW / 2) + k][q];
+                    partial[(size_t)((q < 8 ? col : ecol) + j) * nb + blk] = t;
+                }
+            }
+            __syncthreads();
+        }
+    };
+    // w -= V c, pieces in descending order; |w|^2 into column col
+    auto subtract = [&](const double* c, int col) {
+        double nrm = 0.0;
+        for (long p = c0 < nc ? c0 + (nc - 1 - c0) / stride * stride : -1; p >= 0; p -= stride) {
+            const long i0 = 4 * p + 2 * group;
+            double a[2];
+            if (single) { a[0] = keep[0]; a[1] = keep[1]; }
+            else load2(w + i0, a);
+            orth_subtract(V, ldv, nv, c, i0, a);
+            nrm += a[0] * a[0] + a[1] * a[1];
+            if (single) { keep[0] = a[0]; keep[1] = a[1]; }
+            store2(w, i0, n, a);
+        }
+        block_col(nrm, col);
+    };
+    // ---- dots: h, e and |w|^2
+    {
+        double ww = 0.0;
+        for (long c = c0; c < nc; c += stride) {
+            double a[2];
+            load2(w + 4 * c + 2 * group, a);
+            ww += a[0] * a[0] + a[1] * a[1];
+            if (single) { keep[0] = a[0]; keep[1] = a[1]; }
+        }
+        block_col(ww, 2 * nv);
+        dots(0, nv);
     }
-    for (int i = used; i < m; ++i) sc->yh[i] = 0.0;
+    if (!barrier()) return;
+    sum_columns(partial, 2 * nv + 1, nb, s_col);
+    double beta2 = s_col[2 * nv];
+    const double ww = beta2;
+    if (nv > 0) {
+        if (tid < nv) {
+            const double e = s_col[nv + tid];
+            s_G[tid * nv + i] = e;
+            s_G[i * nv + tid] = e;
+            if (blk == 0) { sc->G[tid * ORTH_MAXV + i] = e; sc->G[i * ORTH_MAXV + tid] = e; }
+        }
+        __syncthreads();
+        if (tid < nv) {
+            double s = 2.0 * s_col[tid];
+            for (int k = 0; k < nv; ++k) s -= s_G[tid * nv + k] * s_col[k];
+            s_c[tid] = s;
+        }
+        __syncthreads();
+        subtract(s_c, 2 * nv + 1);
+        if (!barrier()) return;
+        sum_columns(partial + (size_t)(2 * nv + 1) * nb, 1, nb, s_b);
+        beta2 = s_b[0];
+        if (beta2 < ORTH_AGAIN * ww) {
+            // w lay almost in the basis: a second pass with dots of its own
+            dots(2 * nv + 2, -1);
+            if (!barrier()) return;
+            sum_columns(partial + (size_t)(2 * nv + 2) * nb, nv, nb, s_col);
+            subtract(s_col, 3 * nv + 2);
+            if (tid < nv) s_c[tid] += s_col[tid];
+            if (!barrier()) return;
+            sum_columns(partial + (size_t)(3 * nv + 2) * nb, 1, nb, s_b + 1);
+            beta2 = s_b[1];
+        }
+    }
+    const double beta = sqrt(beta2);
+    if (vout && beta != 0.0) {
+        for (long c = c0; c < nc; c += stride) {
+            const long i0 = 4 * c + 2 * group;
+            double a[2];
+            if (single) { a[0] = keep[0]; a[1] = keep[1]; }
+            else load2(w + i0, a);
+            a[0] /= beta;
+            a[1] /= beta;
+            store2(vout, i0, n, a);
+        }
+    }
+    if (blk == 0) {
+        if (nv == 0) gm_start(sc, beta);
+        else gm_rotate(sc, s_c, s_col, s_col + ORTH_MAXV, i, m, beta);
+    }
+    grid_leave(sc);
+}
+
+// The same for a basis stored in FP32 (FP32 and BF16 Jacobians), by two
+// classical passes with dots of their own: there the Arnoldi vector is rounded
+// to FP32 after every direction and in every preconditioner application, so a
+// last-bit difference in a coefficient is a difference of 1e-7 in the solve.
+// This kernel therefore keeps the sums of the launches it replaces to the
+// order of every addition: red_blocks(n) "blocks" of 256 threads (a CTA takes
+// two at a time, all of one SM's in turn), four entries a thread per piece,
+// the pieces in ascending order, the warps' tree, the eight warps one after
+// the other, then the blocks' sums as one block of 256 threads adds them up.
+constexpr int CGS_TPB = 512;
+constexpr int CGS_NV = 16;                      // basis vectors whose dots a thread holds at once
+
+// sum of part[0..nb) as one block of RED_TPB threads takes it: thread t the
+// entries t, t + RED_TPB, .., a tree over each warp, a tree over the warps;
+// by one warp, all lanes the result
+__device__ __forceinline__ double sum_as_block(const double* part, int nb) {
+    constexpr int NW = RED_TPB / 32;            // 8
+    const int lane = threadIdx.x & 31;
+    double s[NW];
+#pragma unroll
+    for (int q = 0; q < NW; ++q) s[q] = 0.0;
+    for (int b0 = 0; b0 < nb; b0 += RED_TPB)
+#pragma unroll
+        for (int q = 0; q < NW; ++q) {
+            const int b = b0 + 32 * q + lane;
+            if (b < nb) s[q] += __ldcg(part + b);
+        }
+    // the eight trees at once: after three halvings lane l holds warp l / 4's
+    // partial sum over its four lanes' residues, two more steps complete it
+#pragma unroll
+    for (int o = 16, h = NW / 2; h > 0; o >>= 1, h >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int q = 0; q < h; ++q) {
+            const double send = up ? s[q] : s[q + h], keep = up ? s[q + h] : s[q];
+            s[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    double v = s[0];
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    // tree over the warps (lane 4 w): partners 4, 2, 1 warps apart
+    v += __shfl_xor_sync(0xffffffffu, v, 16);
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    return v;
+}
+
+template <typename VT>
+__global__ void __launch_bounds__(CGS_TPB, 1)
+    k_orth_cgs2(long n, int nv, const VT* V, long ldv, double* w, VT* vout, double* partial, Scalars* sc, int m, int nbv) {
+    if (nv > 0 && !sc->gm_active) return;
+    constexpr int NWB = RED_TPB / 32;               // warps of a virtual block
+    __shared__ double s_red[CGS_TPB / 32][CGS_NV];
+    __shared__ double s_h[2][ORTH_MAXV], s_rot[2][ORTH_MAXV], s_b;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = tid / RED_TPB, t = tid % RED_TPB;
+    const int i = nv - 1;
+    const long nc = (n + 3) / 4, stride = (long)nbv * RED_TPB;
+    unsigned round = 0;
+    auto barrier = [&] { return grid_barrier(&sc->orth_bar, ++round * gridDim.x, &sc->flags); };
+    // every virtual block of this CTA, two at a time (f is called by all
+    // threads, with a block past the end for a CTA's odd last one)
+    auto blocks = [&](auto f) {
+        for (int b0 = 2 * blockIdx.x; b0 < nbv; b0 += 2 * gridDim.x) f(b0 + g);
+    };
+    // the block's sums of cnt values into columns col.. : a tree over each
+    // warp, the warps one after the other
+    auto block_sums = [&](double (&acc)[CGS_NV], int cnt, int col, int vb) {
+        const double s = warp_sum16(acc);
+        if ((lane & 1) == 0) s_red[wid][lane >> 1] = s;
+        __syncthreads();
+        if (t < cnt && vb < nbv) {
+            double v = 0;
+            for (int q = 0; q < NWB; ++q) v += s_red[g * NWB + q][t];
+            partial[(size_t)(col + t) * nbv + vb] = v;
+        }
+        __syncthreads();
+    };
+    auto dot4 = [&](double& acc, const double (&v)[4], const double (&a)[4]) {
+        acc += v[0] * a[0] + v[1] * a[1] + v[2] * a[2] + v[3] * a[3];
+    };
+    auto store4 = [&](long i0, const double (&a)[4]) {
+        if (i0 + 4 <= n) {
+            reinterpret_cast<double2*>(w + i0)[0] = make_double2(a[0], a[1]);
+            reinterpret_cast<double2*>(w + i0)[1] = make_double2(a[2], a[3]);
+        } else {
+            for (int e = 0; e < 4 && i0 + e < n; ++e) w[i0 + e] = a[e];
+        }
+    };
+    // dots with vectors jb.. < nv into columns col + jb..; with `coef` the
+    // vector is first reduced by coef_j V_j over all j (once, jb 0)
+    auto dots = [&](int col, const double* coef) {
+        for (int jb = 0; jb < nv; jb += CGS_NV) {
+            const int cnt = min(CGS_NV, nv - jb);
+            blocks([&](int vb) {
+                double acc[CGS_NV];
+#pragma unroll
+                for (int q = 0; q < CGS_NV; ++q) acc[q] = 0.0;
+                if (vb < nbv)
+                    for (long c = (long)vb * RED_TPB + t; c < nc; c += stride) {
+                        double a[4];
+                        load4(w + 4 * c, a);
+                        if (coef && jb == 0) {
+                            int j = 0;
+                            for (; j + 8 <= nv; j += 8) {
+                                double v[8][4];
+#pragma unroll
+                                for (int q = 0; q < 8; ++q) load4(V + (j + q) * ldv + 4 * c, v[q]);
+#pragma unroll
+                                for (int q = 0; q < 8; ++q)
+#pragma unroll
+                                    for (int e = 0; e < 4; ++e) a[e] -= coef[j + q] * v[q][e];
+                            }
+                            for (; j < nv; ++j) {
+                                double v[4];
+                                load4(V + j * ldv + 4 * c, v);
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) a[e] -= coef[j] * v[e];
+                            }
+                            store4(4 * c, a);
+                        }
+                        if (cnt == CGS_NV) {
+#pragma unroll
+                            for (int q = 0; q < CGS_NV; ++q) {
+                                double v[4];
+                                load4(V + (jb + q) * ldv + 4 * c, v);
+                                dot4(acc[q], v, a);
+                            }
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < CGS_NV; ++q)
+                                if (q < cnt) {
+                                    double v[4];
+                                    load4(V + (jb + q) * ldv + 4 * c, v);
+                                    dot4(acc[q], v, a);
+                                }
+                        }
+                    }
+                block_sums(acc, cnt, col + jb, vb);
+            });
+        }
+    };
+    double beta;
+    if (nv == 0) {
+        // |w|^2 entry by entry, the warps' sums by a tree
+        blocks([&](int vb) {
+            double acc = 0.0;
+            if (vb < nbv)
+                for (long k = (long)vb * RED_TPB + t; k < n; k += stride) {
+                    const double a = w[k];
+                    acc += a * a;
+                }
+            acc = warp_sum(acc);
+            if (lane == 0) s_red[wid][0] = acc;
+            __syncthreads();
+            if (t < 32) {
+                double v = t < NWB ? s_red[g * NWB + t][0] : 0.0;
+                v = warp_sum(v);
+                if (t == 0 && vb < nbv) partial[vb] = v;
+            }
+            __syncthreads();
+        });
+        if (!barrier()) return;
+        if (wid == 0) {
+            const double s = sum_as_block(partial, nbv);
+            if (lane == 0) s_b = sqrt(s);
+        }
+    } else {
+        double* part1 = partial + (size_t)nv * nbv;
+        double* part2 = partial + 2 * (size_t)nv * nbv;
+        auto sums = [&](const double* part, double* out) {
+            for (int j = wid; j < nv; j += CGS_TPB / 32) {
+                const double s = sum_as_block(part + (size_t)j * nbv, nbv);
+                if (lane == 0) out[j] = s;
+            }
+            __syncthreads();
+        };
+        dots(0, nullptr);
+        if (!barrier()) return;
+        sums(partial, s_h[0]);
+        dots(nv, s_h[0]);
+        if (!barrier()) return;
+        sums(part1, s_h[1]);
+        blocks([&](int vb) {
+            double acc[CGS_NV];
+#pragma unroll
+            for (int q = 0; q < CGS_NV; ++q) acc[q] = 0.0;
+            if (vb < nbv)
+                for (long c = (long)vb * RED_TPB + t; c < nc; c += stride) {
+                    double a[4];
+                    load4(w + 4 * c, a);
+                    int j = 0;
+                    for (; j + 8 <= nv; j += 8) {
+                        double v[8][4];
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) load4(V + (j + q) * ldv + 4 * c, v[q]);
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) a[e] -= s_h[1][j + q] * v[q][e];
+                    }
+                    for (; j < nv; ++j) {
+                        double v[4];
+                        load4(V + j * ldv + 4 * c, v);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) a[e] -= s_h[1][j] * v[e];
+                    }
+                    store4(4 * c, a);
+                    acc[0] += a[0] * a[0] + a[1] * a[1] + a[2] * a[2] + a[3] * a[3];
+                }
+            block_sums(acc, 1, 2 * nv, vb);
+        });
+        if (!barrier()) return;
+        if (wid == 0) {
+            const double s = sum_as_block(part2, nbv);
+            if (lane == 0) s_b = sqrt(s);
+        }
+    }
+    __syncthreads();
+    beta = s_b;
+    if (vout && beta != 0.0)
+        blocks([&](int vb) {
+            if (vb < nbv)
+                for (long c = (long)vb * RED_TPB + t; c < nc; c += stride)
+                    for (int hf = 0; hf < 2; ++hf) {
+                        const long i0 = 4 * c + 2 * hf;
+                        double a[2];
+                        load2(w + i0, a);
+                        a[0] /= beta;
+                        a[1] /= beta;
+                        store2(vout, i0, n, a);
+                    }
+        });
+    if (blockIdx.x == 0) {
+        if (nv == 0) gm_start(sc, beta);
+        else {
+            __syncthreads();
+            if (tid < nv) s_h[0][tid] += s_h[1][tid];
+            gm_rotate(sc, s_h[0], s_rot[0], s_rot[1], i, m, beta);
+        }
+    }
+    grid_leave(sc);
+}
+
+// dx += V y with H y = bh (each block solves for y itself, H through shared
+// memory: 20 rows in ~3 us, where a launch of one thread reading H from
+// global memory took 25)
+template <typename VT>
+__global__ void __launch_bounds__(ORTH_TPB, 2) k_gm_update(long n, int m, const VT* __restrict__ V, long ldv,
+                                                           double* __restrict__ dx, const Scalars* __restrict__ sc) {
+    __shared__ double s_y[ORTH_MAXV];
+    extern __shared__ double s_H[];                 // [used][used]
+    const int tid = threadIdx.x, used = sc->gm_used;
+    for (int q = tid; q < used * used; q += ORTH_TPB) s_H[q] = sc->H[(q / used) * m + q % used];
+    if (tid < used) s_y[tid] = sc->bh[tid];
+    __syncthreads();
+    if (tid == 0) {
+        for (int i = used - 1; i >= 0; --i) {
+            double sum = s_y[i];
+#pragma unroll 4
+            for (int j = i + 1; j < used; ++j) sum -= s_H[i * used + j] * s_y[j];
+            s_y[i] = sum / s_H[i * used + i];
+        }
+    }
+    __syncthreads();
+    if (tid < used) s_y[tid] = -s_y[tid];
+    __syncthreads();
+    const long nh = (n + 1) / 2;
+    for (long c = (long)blockIdx.x * ORTH_TPB + tid; c < nh; c += (long)gridDim.x * ORTH_TPB) {
+        double a[2];
+        load2(dx + 2 * c, a);
+        orth_subtract(V, ldv, used, s_y, 2 * c, a);
+        store2(dx, 2 * c, n, a);
+    }
 }
 
 // ---------------------------------------------------------------- BiCGStab
@@ -1464,12 +1863,12 @@ __global__ void k_bi_p(long n, const double* __restrict__ r, const double* __res
 __global__ void k_bi_scal_rho(Scalars* sc) {       // rho, beta from rw.r
     if (threadIdx.x != 0) return;
     sc->bi_rhoOld = sc->bi_rho;
-    sc->bi_rho = sc->hcol[0][0];
+    sc->bi_rho = sc->dots[0];
     sc->bi_beta = sc->bi_rho / sc->bi_rhoOld * (sc->bi_alpha / sc->bi_omega);
 }
 __global__ void k_bi_scal_alpha(Scalars* sc) {
     if (threadIdx.x != 0) return;
-    sc->bi_alpha = sc->bi_rho / sc->hcol[0][0];
+    sc->bi_alpha = sc->bi_rho / sc->dots[0];
 }
 __global__ void k_bi_s(long n, const double* __restrict__ r, const double* __restrict__ v, double* __restrict__ s,
                        const Scalars* sc) {
@@ -1478,7 +1877,7 @@ __global__ void k_bi_s(long n, const double* __restrict__ r, const double* __res
 }
 __global__ void k_bi_scal_omega(Scalars* sc) {     // omega = (t.s)/(t.t)
     if (threadIdx.x != 0) return;
-    double tt = sc->hcol[0][0], ts = sc->hcol[0][1];
+    double tt = sc->dots[0], ts = sc->dots[1];
     sc->bi_omega = tt > 0 ? ts / tt : 0.0;
 }
 __global__ void k_bi_update(long n, double* __restrict__ x, double* __restrict__ r, const double* __restrict__ ph,

@@ -300,6 +300,8 @@ struct rdst_ctx {
     DBuf<unsigned char> rmask;      // held cells (internal order): zero residual, identity rows; empty: none
     DBuf<float> Vf;                 // GMRES basis when it is kept in FP32
     long ldv = 0;                   // stride between basis vectors (entries)
+    DBuf<double> orth_part;         // partial sums of k_orth's blocks
+    int orth_blocks = 0, sms = 0;   // blocks of k_orth that are resident together
     DBuf<double> wv;                // FP64 Arnoldi vector that is orthogonalised before it is stored in Vf
     // discrete adjoint (allocated on first use)
     DBuf<double> a_fbar, a_qbbar, a_qbar, a_gbar, a_vval, a_hval, a_wbar, a_wbarb, a_ubarb, a_pbar;
@@ -1060,12 +1062,27 @@ void build(rdst_ctx& c, const rdst_mesh* mh) {
     if (o.precon == PRECON_GAUSS_SEIDEL && o.n_sweeps > 1) { c.gs_r.alloc(5L * N); c.gs_z.alloc(5L * N); }
     // ---- Krylov
     const long n5 = 5L * N;
-    c.dx.alloc(n5); c.r.alloc(n5); c.t.alloc(n5); c.Ax.alloc(n5); c.pA.alloc(n5); c.xbar.alloc(8);
+    c.r.alloc(n5); c.t.alloc(n5); c.Ax.alloc(n5); c.pA.alloc(n5); c.xbar.alloc(8);
     // basis vectors 64-entry aligned (the orthogonalisation reads 4 entries per 16-byte load)
     c.ldv = (n5 + 63) / 64 * 64;
-    if (o.solver == SOLVER_GMRES && o.basis32) { c.Vf.alloc((size_t)(o.n_directions + 1) * c.ldv); c.wv.alloc(n5); }
-    else if (o.solver == SOLVER_GMRES) c.Vb.alloc((size_t)(o.n_directions + 1) * c.ldv);
+    // (with zeros past the end, which the orthogonalisation reads along)
+    c.dx.alloc(c.ldv); c.dx.zero(s);
+    if (o.solver == SOLVER_GMRES && o.basis32) {
+        c.Vf.alloc((size_t)(o.n_directions + 1) * c.ldv); c.Vf.zero(s);
+        c.wv.alloc(c.ldv); c.wv.zero(s);
+    } else if (o.solver == SOLVER_GMRES) { c.Vb.alloc((size_t)(o.n_directions + 1) * c.ldv); c.Vb.zero(s); }
     else { c.s2.alloc(n5); c.sh.alloc(n5); c.ph.alloc(n5); c.pv.alloc(n5); c.Vb.alloc(2 * n5); }
+    {
+        int dev = 0, per = 0, per32 = 0;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev));
+        const size_t sm = sizeof(double) * ORTH_MAXV * ORTH_MAXV;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_orth<double>, ORTH_TPB, sm));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per32, k_orth_cgs2<float>, CGS_TPB, 0));
+        c.orth_blocks = c.sms * std::max(1, std::min({1, per, per32}));
+        // partial sums: of k_orth's blocks, or two dots a direction and a norm of red_blocks(n)
+        c.orth_part.alloc(std::max((size_t)ORTH_COLS * c.orth_blocks, (size_t)(2 * ORTH_MAXV + 1) * red_blocks(n5)));
+    }
     // limiter needs
     auto vk = [](Limiter l) { return l == LIM_VENKATAKRISHNAN; };
     c.venkat_mask = (vk(o.lim_rho) ? 1 : 0) | (vk(o.lim_U) ? 0xE : 0) | (vk(o.lim_T) ? 0x70 : 0);
@@ -1369,72 +1386,56 @@ struct Ops {
         k_multidot<<<nb, RED_TPB, 0, c.s>>>(n, 1, a, 0, b, c.partial.p, 8, active); CKL();
         k_finalize<<<1, RED_TPB, 0, c.s>>>(c.partial.p, nb, 1, 8, out, sq, active); CKL();
     }
-    // V^T w (one pass over w) into out[0..nv)
-    template <int NV, typename VT>
-    static void vmultidot(rdst_ctx& c, const VT* V, int nv, const double* w, double* out, const int* active) {
-        long n = c.nvec();
-        int nb = red_blocks(n);
-        k_vmultidot<NV, VT><<<nb, RED_TPB, 0, c.s>>>(n, nv, V, c.ldv, w, c.partial.p, 64, active); CKL();
-        k_finalize<<<nv, RED_TPB, 0, c.s>>>(c.partial.p, nb, nv, 64, out, 0, active); CKL();
+    // w orthogonalised against V_0..V_{nv-1} and (vout) stored normalised, or
+    // (nv 0) the cycle's start; all blocks resident (k_orth)
+    template <typename VT>
+    static void orth(rdst_ctx& c, Scalars* sc, const VT* V, int nv, double* w, VT* vout, int m) {
+        Timed tm(c, KS_ORTH);
+        long n = c.nvec(), ldv = c.ldv;
+        double* part = c.orth_part.p;
+        if constexpr (std::is_same<VT, double>::value) {
+            const int nb = (int)std::min<long>(c.orth_blocks, nblk((n + 3) / 4, ORTH_PIECES));
+            void* args[] = {&n, &nv, &V, &ldv, &w, &vout, &part, &sc, &m};
+            CK(cudaLaunchCooperativeKernel((const void*)k_orth<VT>, dim3(nb), dim3(ORTH_TPB), args,
+                                           sizeof(double) * nv * nv, c.s));
+        } else {
+            int nbv = red_blocks(n);
+            const int nb = std::min(c.orth_blocks, (nbv + 1) / 2);
+            void* args[] = {&n, &nv, &V, &ldv, &w, &vout, &part, &sc, &m, &nbv};
+            CK(cudaLaunchCooperativeKernel((const void*)k_orth_cgs2<VT>, dim3(nb), dim3(CGS_TPB), args, 0, c.s));
+        }
+        count_launch();
     }
-    // w -= V coef, fused with the next dots (mode 0) or the norm (mode 1)
-    template <int NV, typename VT>
-    static void maxpy_dot(rdst_ctx& c, const VT* V, int nv, const double* coef, double* w, double* out, int mode,
-                          const int* active) {
-        long n = c.nvec();
-        int nb = red_blocks(n);
-        k_maxpy_dot<NV, VT><<<nb, RED_TPB, 0, c.s>>>(n, nv, V, c.ldv, coef, w, c.partial.p, 64, mode, active); CKL();
-        if (mode == 0) { k_finalize<<<nv, RED_TPB, 0, c.s>>>(c.partial.p, nb, nv, 64, out, 0, active); CKL(); }
-        else { k_finalize<<<1, RED_TPB, 0, c.s>>>(c.partial.p, nb, 1, 64, out, 1, active); CKL(); }
+    // x += V y, H y = bh
+    template <typename VT>
+    static void gm_update(rdst_ctx& c, const Scalars* sc, const VT* V, double* x, int m) {
+        const long n = c.nvec();
+        k_gm_update<VT><<<std::min(4 * c.sms, nblk((n + 1) / 2, ORTH_TPB)), ORTH_TPB, sizeof(double) * m * m, c.s>>>(
+            n, m, V, c.ldv, x, sc);
+        CKL();
     }
-    // CGS2 orthogonalisation of w against V_0..V_i: H[:,i] pieces, beta = |w|
-    template <int NV, typename VT>
-    static void orth(rdst_ctx& c, const VT* V, int nv, double* w, const int* act) {
-        Scalars* sc = c.sc.p;
-        vmultidot<NV, VT>(c, V, nv, w, sc->hcol[0], act);
-        maxpy_dot<NV, VT>(c, V, nv, sc->hcol[0], w, sc->hcol[1], 0, act);
-        maxpy_dot<NV, VT>(c, V, nv, sc->hcol[1], w, &sc->beta, 1, act);
-    }
-    // One restart cycle of left-preconditioned GMRES(m) with CGS2.  With an
-    // FP64 basis each Arnoldi vector is built in place in its basis slot;
-    // with an FP32 basis it is built and orthogonalised in the FP64 vector
-    // wv (dots, Hessenberg and Givens stay FP64) and stored normalised.
+    // One restart cycle of left-preconditioned GMRES(m).  With an FP64 basis
+    // each Arnoldi vector is built in place in its basis slot; with an FP32
+    // basis it is built and orthogonalised in the FP64 vector wv (dots,
+    // Hessenberg and Givens stay FP64) and stored normalised.
     template <typename VT>
     static void gmres_cycle_t(rdst_ctx& c, VT* Vb) {
         constexpr bool in_place = std::is_same<VT, double>::value;
-        cudaStream_t s = c.s;
-        const long n = c.nvec();
         const int m = c.o.n_directions;
         Scalars* sc = c.sc.p;
         int* act = &sc->gm_active;
-        double* w0 = in_place ? (double*)Vb : c.wv.p;
+        auto slot = [&](int i) { return in_place ? (double*)(Vb + i * c.ldv) : c.wv.p; };
         spmv(c, c.dx.p, c.r.p, c.rhs.p, nullptr);            // r = rhs - A dx
-        precond(c, c.r.p, w0, nullptr);                      // w = M^-1 r
-        dot(c, w0, w0, &sc->beta, 1, nullptr);
-        k_gm_start<<<1, 1, 0, s>>>(sc); CKL();
-        if (in_place) { k_scale_inv<<<nblk(n, TPB), TPB, 0, s>>>(n, w0, &sc->beta, act); CKL(); }
-        else { k_scale_store<VT><<<nblk(n, TPB), TPB, 0, s>>>(n, w0, Vb, &sc->beta, act); CKL(); }
+        precond(c, c.r.p, slot(0), nullptr);                 // w = M^-1 r
+        orth<VT>(c, sc, Vb, 0, slot(0), Vb, m);
         for (int i = 0; i < m; ++i) {
             const VT* Vi = Vb + i * c.ldv;
-            double* w = in_place ? (double*)(Vb + (i + 1) * c.ldv) : c.wv.p;
+            double* w = slot(i + 1);
             spmv(c, Vi, c.t.p, nullptr, act);
             precond(c, c.t.p, w, act);
-            {
-                Timed tm(c, KS_ORTH);
-                const int nv = i + 1;
-                if (nv <= 8) orth<8, VT>(c, Vb, nv, w, act);
-                else if (nv <= 16) orth<16, VT>(c, Vb, nv, w, act);
-                else if (nv <= 32) orth<32, VT>(c, Vb, nv, w, act);
-                else orth<64, VT>(c, Vb, nv, w, act);
-            }
-            k_gm_givens<<<1, 1, 0, s>>>(sc, i, m); CKL();
-            if (i < m - 1) {
-                if (in_place) { k_scale_inv<<<nblk(n, TPB), TPB, 0, s>>>(n, w, &sc->beta, act); CKL(); }
-                else { k_scale_store<VT><<<nblk(n, TPB), TPB, 0, s>>>(n, w, Vb + (i + 1) * c.ldv, &sc->beta, act); CKL(); }
-            }
+            orth<VT>(c, sc, Vb, i + 1, w, i < m - 1 ? Vb + (i + 1) * c.ldv : nullptr, m);
         }
-        k_gm_backsub<<<1, 1, 0, s>>>(sc, m); CKL();
-        k_maxpy<VT><<<nblk(n, TPB), TPB, 0, s>>>(n, m, Vb, c.ldv, sc->yh, c.dx.p, -1.0, nullptr); CKL();
+        gm_update<VT>(c, sc, Vb, c.dx.p, m);
         finish_iteration(c);
     }
     static void gmres_cycle(rdst_ctx& c) {
@@ -1455,18 +1456,18 @@ struct Ops {
         Scalars* sc = c.sc.p;
         double* rw = c.Vb.p;
         double* t2 = c.Vb.p + n;
-        dot(c, rw, c.r.p, &sc->hcol[0][0], 0, nullptr);
+        dot(c, rw, c.r.p, &sc->dots[0], 0, nullptr);
         k_bi_scal_rho<<<1, 1, 0, s>>>(sc); CKL();
         k_bi_p<<<nblk(n, TPB), TPB, 0, s>>>(n, c.r.p, c.pv.p, c.t.p, sc); CKL();      // t holds p
         precond(c, c.t.p, c.ph.p, nullptr);
         spmv(c, c.ph.p, c.pv.p, nullptr, nullptr);                                  // v = A ph
-        dot(c, rw, c.pv.p, &sc->hcol[0][0], 0, nullptr);
+        dot(c, rw, c.pv.p, &sc->dots[0], 0, nullptr);
         k_bi_scal_alpha<<<1, 1, 0, s>>>(sc); CKL();
         k_bi_s<<<nblk(n, TPB), TPB, 0, s>>>(n, c.r.p, c.pv.p, c.s2.p, sc); CKL();
         precond(c, c.s2.p, c.sh.p, nullptr);
         spmv(c, c.sh.p, t2, nullptr, nullptr);
-        dot(c, t2, t2, &sc->hcol[0][0], 0, nullptr);
-        dot(c, t2, c.s2.p, &sc->hcol[0][1], 0, nullptr);
+        dot(c, t2, t2, &sc->dots[0], 0, nullptr);
+        dot(c, t2, c.s2.p, &sc->dots[1], 0, nullptr);
         k_bi_scal_omega<<<1, 1, 0, s>>>(sc); CKL();
         k_bi_update<<<nblk(n, TPB), TPB, 0, s>>>(n, c.dx.p, c.r.p, c.ph.p, c.sh.p, c.s2.p, t2, sc); CKL();
         int nb = red_blocks(c.N);
@@ -1615,6 +1616,7 @@ __global__ void k_init_scalars(Scalars* sc, double time, double dt, double co) {
     sc->residual = -1;
     sc->residualRatio = 1;
     sc->flags = 0;
+    sc->orth_bar = sc->orth_out = 0;     // left behind by a launch whose barrier expired
 }
 
 // timeDST::initialize (timeDST.C:67-208) on the freshly set state
@@ -2015,7 +2017,7 @@ void adj_alloc(rdst_ctx& c, int m) {
         c.a_wbar.alloc(n5);
         c.a_wbarb.alloc(5L * std::max(c.NB, 1)); c.a_ubarb.alloc(3L * std::max(c.NB, 1));
         c.a_pbar.alloc(std::max(c.NB, 1));
-        c.a_r.alloc(n5); c.a_z.alloc(n5); c.a_t.alloc(n5); c.a_psi.alloc(n5); c.a_rhs.alloc(n5);
+        c.a_r.alloc(n5); c.a_z.alloc(n5); c.a_t.alloc(n5); c.a_psi.alloc(c.ldv); c.a_psi.zero(c.s); c.a_rhs.alloc(n5);
         c.a_tmp.alloc(n5); c.a_u3.alloc(16);
         c.a_fbar.zero(c.s); c.a_qbbar.zero(c.s);
         if (c.tr.viscous) {
@@ -2025,8 +2027,8 @@ void adj_alloc(rdst_ctx& c, int m) {
         }
     }
     if (m > 0 && c.a_m != m) {
-        c.a_V.alloc((size_t)(m + 1) * c.ldv);
-        c.a_Z.alloc((size_t)(m + 1) * c.ldv);
+        c.a_V.alloc((size_t)(m + 1) * c.ldv); c.a_V.zero(c.s);      // zeros past the end of each vector
+        c.a_Z.alloc((size_t)(m + 1) * c.ldv); c.a_Z.zero(c.s);
         c.a_m = m;
     }
     if (!c.a_sc.p) { c.a_sc.alloc(1); c.a_sc.zero(c.s); }
@@ -2186,7 +2188,6 @@ int adj_solve(rdst_ctx& c, const double* rhs, double* psi, double rel_tol, int m
     cudaStream_t s = c.s;
     const long n = c.nvec();
     Scalars* sc = c.a_sc.p;
-    int* act = &sc->gm_active;
     double* Vb = c.a_V.p;
     double* Zb = c.a_Z.p;
     CK(cudaMemsetAsync(psi, 0, sizeof(double) * n, s));
@@ -2198,7 +2199,7 @@ int adj_solve(rdst_ctx& c, const double* rhs, double* psi, double rel_tol, int m
         // r = rhs - J^T psi (into V_0)
         adj_product(c, psi, c.a_t.p, nullptr);
         k_adj_sub<<<nblk(n, TPB), TPB, 0, s>>>(n, rhs, c.a_t.p, Vb); CKL();
-        Ops<MT>::dot(c, Vb, Vb, &sc->beta, 1, nullptr);
+        Ops<MT>::template orth<double>(c, sc, Vb, 0, Vb, Vb, m);
         double beta = 0.0;
         CK(cudaMemcpyAsync(&beta, &sc->beta, sizeof(double), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
@@ -2206,33 +2207,16 @@ int adj_solve(rdst_ctx& c, const double* rhs, double* psi, double rel_tol, int m
         if (cyc == 0) res0 = res;
         if (res <= rel_tol * res0 || res == 0.0) break;
         ++cycles;
-        k_gm_start<<<1, 1, 0, s>>>(sc); CKL();
-        k_scale_inv<<<nblk(n, TPB), TPB, 0, s>>>(n, Vb, &sc->beta, act); CKL();
         for (int i = 0; i < m; ++i) {
             const double* Vi = Vb + i * c.ldv;
             double* Zi = Zb + i * c.ldv;
             double* w = Vb + (i + 1) * c.ldv;
             adj_prec<MT>(c, Vi, Zi);
             adj_product(c, Zi, w, nullptr);
-            const int nv = i + 1;
-            // CGS2 against V_0..V_i into this solve's own Hessenberg column
-            auto orth = [&](auto nvtag) {
-                constexpr int NV = decltype(nvtag)::value;
-                Ops<MT>::template vmultidot<NV, double>(c, Vb, nv, w, sc->hcol[0], act);
-                Ops<MT>::template maxpy_dot<NV, double>(c, Vb, nv, sc->hcol[0], w, sc->hcol[1], 0, act);
-                Ops<MT>::template maxpy_dot<NV, double>(c, Vb, nv, sc->hcol[1], w, &sc->beta, 1, act);
-            };
-            if (nv <= 8) orth(std::integral_constant<int, 8>());
-            else if (nv <= 16) orth(std::integral_constant<int, 16>());
-            else if (nv <= 32) orth(std::integral_constant<int, 32>());
-            else orth(std::integral_constant<int, 64>());
-            k_gm_givens<<<1, 1, 0, s>>>(sc, i, m); CKL();
-            if (i < m - 1) { k_scale_inv<<<nblk(n, TPB), TPB, 0, s>>>(n, w, &sc->beta, act); CKL(); }
+            Ops<MT>::template orth<double>(c, sc, Vb, i + 1, w, i < m - 1 ? w : nullptr, m);
             ++iters;
         }
-        k_gm_backsub<<<1, 1, 0, s>>>(sc, m); CKL();
-        // psi += Z y
-        k_maxpy<double><<<nblk(n, TPB), TPB, 0, s>>>(n, m, Zb, c.ldv, sc->yh, psi, -1.0, nullptr); CKL();
+        Ops<MT>::template gm_update<double>(c, sc, Zb, psi, m);      // psi += Z y
     }
     return iters;
 }

@@ -84,7 +84,10 @@ struct Scalars {
     // GMRES
     double beta;
     int gm_active, gm_used;
-    double H[64 * 65], bh[65], cs[64], sn[64], yh[64], hcol[2][65];
+    double H[64 * 65], bh[65], cs[64], sn[64];
+    double G[64 * 64];                  // V^T V of the cycle's basis
+    unsigned orth_bar, orth_out;        // grid barrier of k_orth (zero between launches)
+    double dots[2];
     // BiCGStab
     double bi_rho, bi_rhoOld, bi_alpha, bi_omega, bi_beta, bi_tt, bi_ts, bi_rwv;
 };
