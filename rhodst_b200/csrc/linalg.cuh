@@ -73,31 +73,59 @@ __device__ __forceinline__ void inv5(const T A[25], T X[25]) {
         for (int j = 0; j < 5; ++j) X[5 * i + j] = a[i][j + 5];
 }
 
-// y = A x  (or y = b - A x when b != nullptr); one row per thread; x in
-// FP64 or (a Krylov basis vector) FP32, products and y in FP64
-template <typename MT, typename XT = double>
-__global__ void __launch_bounds__(256) k_spmv(SellMat<MT> A, const XT* __restrict__ x, double* __restrict__ y,
-                                              const double* __restrict__ b, const int* __restrict__ active) {
+// y = A x, or b - A x with b, or with JACOBI the block-Jacobi preconditioner
+// applied to that, Dinv (...), in the same pass; x in FP64 or (a Krylov basis
+// vector) FP32, products and y in FP64.  One row per thread: bound by the
+// bytes of the matrix, on few rows by the chain column -> x of each slot.  So
+// all 25 entries and the x of a slot are loaded before the first is used, and
+// the next slot's column with them; the register bound that allows it (48,
+// FP64 80) leaves warps enough (per launch, before with 32 registers and the
+// loads one by one -> now: 442 k-cell wing FP64 117 -> 109 us, 0.95 of the copy
+// bandwidth, 1.2 M FP32 174 -> 164, 371 k BF16 67 -> 49, 111 k FP64 45 -> 33).
+// Five warps a slice, one per component, were no faster on 4 k to 100 k rows.
+template <typename MT, typename XT, bool JACOBI>
+__global__ void __launch_bounds__(256, sizeof(MT) == 8 ? 3 : 5) k_spmv(SellMat<MT> A, const XT* __restrict__ x, double* __restrict__ y,
+                                              const double* __restrict__ b, const MT* __restrict__ dinv,
+                                              const int* __restrict__ active) {
     if (active && !*active) return;
     int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= A.N) return;
     const int s = r >> 5, lane = r & 31;
     const int base = A.slice_off[s], width = A.slice_w[s];
     double acc[5] = {0, 0, 0, 0, 0};
+    int cn = width > 0 ? A.col[(size_t)base * 32 + lane] : -1;      // the next slot's column
     for (int k = 0; k < width; ++k) {
-        size_t slot = (size_t)(base + k);
-        int c = A.col[slot * 32 + lane];
+        const size_t slot = (size_t)(base + k);
+        const int c = cn;
+        if (k + 1 < width) cn = A.col[(slot + 1) * 32 + lane];
         if (c < 0) continue;
-        const XT* xc = x + 5 * c;
-        double xv[5] = {tod(xc[0]), tod(xc[1]), tod(xc[2]), tod(xc[3]), tod(xc[4])};
+        const XT* xc = x + 5 * (size_t)c;
         const MT* v = A.val + slot * (32 * 25) + lane;
+        MT m[25];
+        XT xv[5];
+#pragma unroll
+        for (int e = 0; e < 25; ++e) m[e] = v[e * 32];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) xv[j] = xc[j];
 #pragma unroll
         for (int i = 0; i < 5; ++i)
 #pragma unroll
-            for (int j = 0; j < 5; ++j) acc[i] += ld(v + (5 * i + j) * 32) * xv[j];
+            for (int j = 0; j < 5; ++j) acc[i] += tod(m[5 * i + j]) * tod(xv[j]);
     }
     double* yr = y + 5 * r;
-    if (b) {
+    if (JACOBI) {
+        if (b) {
+#pragma unroll
+            for (int i = 0; i < 5; ++i) acc[i] = b[5 * r + i] - acc[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            double a = 0;
+#pragma unroll
+            for (int j = 0; j < 5; ++j) a += ld(&dinv[flat_e(r, 5 * i + j)]) * acc[j];
+            yr[i] = a;
+        }
+    } else if (b) {
 #pragma unroll
         for (int i = 0; i < 5; ++i) yr[i] = b[5 * r + i] - acc[i];
     } else {

@@ -1245,7 +1245,8 @@ struct Ops {
     // r = b - A x and the damped block-Jacobi update on level l
     static void amg_resid(rdst_ctx& c, int l, const double* x, const double* b, double* r, const int* act) {
         if (l == 0) {
-            k_spmv<MT, double><<<nblk(c.N, 256), 256, 0, c.s>>>(c.mat<MT>(c.Aval), x, r, b, act);
+            spmv_launch<double, false>(c, x, r, b, act);
+            return;
         } else {
             auto& L = *c.amg[l - 1];
             k_amg_resid<<<nblk(L.n, 128), 128, 0, c.s>>>(L.n, L.start.p, L.col.p, L.val.p, x, b, r, act);
@@ -1335,8 +1336,7 @@ struct Ops {
             lu_apply(c, in, out, active);
             // further Gauss-Seidel sweeps: out += (D + L)^-1 (in - A out)
             for (int sw = 1; c.o.precon == PRECON_GAUSS_SEIDEL && sw < c.o.n_sweeps; ++sw) {
-                k_spmv<MT, double><<<nblk(c.N, 256), 256, 0, c.s>>>(c.mat<MT>(c.Aval), out, c.gs_r.p, in, active);
-                CKL();
+                spmv_launch<double, false>(c, out, c.gs_r.p, in, active);
                 lu_apply(c, c.gs_r.p, c.gs_z.p, active);
                 k_vadd<<<nblk(c.nvec(), TPB), TPB, 0, c.s>>>(c.nvec(), c.gs_z.p, out, active);
                 CKL();
@@ -1346,11 +1346,30 @@ struct Ops {
             CKL();
         }
     }
+    template <typename XT, bool JACOBI>
+    static void spmv_launch(rdst_ctx& c, const XT* x, double* y, const double* b, const int* active) {
+        const SellMat<MT> M = c.mat<MT>(c.Aval);
+        const MT* dinv = (const MT*)c.dinv;
+        k_spmv<MT, XT, JACOBI><<<nblk(c.N, 256), 256, 0, c.s>>>(M, x, y, b, dinv, active);
+        CKL();
+    }
+    // y = A x, or b - A x with b
     template <typename XT>
     static void spmv(rdst_ctx& c, const XT* x, double* y, const double* b, const int* active) {
         Timed tm(c, KS_SPMV);
-        k_spmv<MT, XT><<<nblk(c.N, 256), 256, 0, c.s>>>(c.mat<MT>(c.Aval), x, y, b, active);
-        CKL();
+        spmv_launch<XT, false>(c, x, y, b, active);
+    }
+    // w = M^-1 A x, or M^-1 (b - A x) with b (t: the product on the way,
+    // where the preconditioner is not applied in the product's own pass)
+    template <typename XT>
+    static void spmv_precond(rdst_ctx& c, const XT* x, double* t, double* w, const double* b, const int* active) {
+        if (c.o.precon == PRECON_DIAGONAL) {
+            Timed tm(c, KS_SPMV);
+            spmv_launch<XT, true>(c, x, w, b, active);
+        } else {
+            spmv(c, x, t, b, active);
+            precond(c, t, w, active);
+        }
     }
     // normFactor + initial residual (dx = 0 -> r = rhs)
     static void solve_init(rdst_ctx& c) {
@@ -1425,14 +1444,12 @@ struct Ops {
         Scalars* sc = c.sc.p;
         int* act = &sc->gm_active;
         auto slot = [&](int i) { return in_place ? (double*)(Vb + i * c.ldv) : c.wv.p; };
-        spmv(c, c.dx.p, c.r.p, c.rhs.p, nullptr);            // r = rhs - A dx
-        precond(c, c.r.p, slot(0), nullptr);                 // w = M^-1 r
+        spmv_precond(c, c.dx.p, c.r.p, slot(0), c.rhs.p, nullptr);      // w = M^-1 (rhs - A dx)
         orth<VT>(c, sc, Vb, 0, slot(0), Vb, m);
         for (int i = 0; i < m; ++i) {
             const VT* Vi = Vb + i * c.ldv;
             double* w = slot(i + 1);
-            spmv(c, Vi, c.t.p, nullptr, act);
-            precond(c, c.t.p, w, act);
+            spmv_precond(c, Vi, c.t.p, w, nullptr, act);
             orth<VT>(c, sc, Vb, i + 1, w, i < m - 1 ? Vb + (i + 1) * c.ldv : nullptr, m);
         }
         gm_update<VT>(c, sc, Vb, c.dx.p, m);
