@@ -795,6 +795,15 @@ __device__ __forceinline__ void rec_store(unsigned char* v, int tot, int idx, co
     *reinterpret_cast<unsigned short*>(v + 40 * (size_t)tot + 2 * (size_t)idx) = __bfloat16_as_ushort(o[4]);
 }
 
+// the plan's headers and columns -> the start of each group of the records
+// (once, when the context is built: a CTA per group)
+__global__ void k_rec_meta(const RecGroup* __restrict__ grp, const RecMeta* __restrict__ gm,
+                           const uint4* __restrict__ meta, uint4* __restrict__ rec) {
+    const RecMeta m = gm[blockIdx.x];
+    for (unsigned q = threadIdx.x; q < m.n16; q += blockDim.x)
+        rec[(size_t)grp[blockIdx.x].off16 + q] = meta[(size_t)m.off16 + q];
+}
+
 // factor blocks -> records (after each factorisation): a warp per task, lane
 // (position, component) as the apply reads it, so that every store of a slot
 // fills whole sectors of the record; the reads of the sliced stores are 6-row
@@ -815,6 +824,7 @@ __global__ void __launch_bounds__(256) k_ilu_pack(int nf, int nb, SellMat<MT> A,
     const int pos = lane / 5, comp = lane - 5 * pos;
     if (lane >= 30 || pos >= n) return;
     unsigned char* v = rec + (size_t)t.group16 * 16 + 16 * (size_t)(h.x >> 16);
+    const unsigned char* nks = rec + (size_t)t.group16 * 16 + 16 * ((size_t)(h.x & 0xffffu) + n * ((S + 3) >> 2));
     const int r = (int)h.z + (int)((pos < 4 ? g.y >> (8 * pos) : g.z >> (8 * (pos - 4))) & 255u);
     const int ms = P.ml + P.mu;
     auto copy = [&](const MT* src, int blk) {       // src: entry 0 of the block, entries 32 apart
@@ -828,7 +838,7 @@ __global__ void __launch_bounds__(256) k_ilu_pack(int nf, int nb, SellMat<MT> A,
     int blk = (back ? n : 0) + pos;
 #pragma unroll 4
     for (int k = 0; k < S; ++k) {
-        const int nk = k < 4 ? (int)((g.x >> (8 * k)) & 255u) : (int)v[k - 16];
+        const int nk = k < 4 ? (int)((g.x >> (8 * k)) & 255u) : (int)nks[k];
         if (pos < nk) {
             const int f = lu_fid(r, back ? P.ml + k : k, ms);
             const MT* src = lu + flat_e(f, 0);
@@ -1084,7 +1094,7 @@ __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TI
 #pragma unroll
                     for (int k = 0; k < NB; ++k) blk += (int)((nk4 >> (8 * k)) & 255u);
                     for (int k = NB; k < S; ++k) {
-                        const int nk = k < 4 ? (int)((nk4 >> (8 * k)) & 255u) : (int)lds_byte(cv - 16 + k);
+                        const int nk = k < 4 ? (int)((nk4 >> (8 * k)) & 255u) : (int)lds_byte(cc + 16 * n * ((S + 3) >> 2) + k);
                         const int c = (int)lds1(cc + 16 * ((k >> 2) * n + pos) + 4 * (k & 3));
                         CT xe[5], m[5];
                         lb_load(lb + max(c, 0), xe);

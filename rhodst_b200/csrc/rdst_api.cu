@@ -575,8 +575,20 @@ void build_records(rdst_ctx& c, const Options& o, int nparts, const std::vector<
                          (size_t)per_sm, (size_t)per_block, (size_t)reserved);
     if (!P.ok) return;
     cudaStream_t s = c.s;
-    c.rec_f.upload(P.f.rec, s); c.rec_b.upload(P.b.rec, s);
     c.grp_f.upload(P.f.groups, s); c.grp_b.upload(P.b.groups, s);
+    for (int back = 0; back < 2; ++back) {
+        const RecSide& R = back ? P.b : P.f;
+        DBuf<unsigned char>& rec = back ? c.rec_b : c.rec_f;
+        DBuf<unsigned char> meta;
+        DBuf<RecMeta> gm;
+        rec.alloc(R.bytes);
+        meta.upload(R.meta, s);
+        gm.upload(R.group_meta, s);
+        k_rec_meta<<<(unsigned)R.groups.size(), 128, 0, s>>>((back ? c.grp_b : c.grp_f).p, gm.p,
+                                                             (const uint4*)meta.p, (uint4*)rec.p);
+        CKL();
+        CK(cudaStreamSynchronize(s));      // meta and gm go out of scope
+    }
     c.part_gf.upload(P.f.part_g, s); c.part_gb.upload(P.b.part_g, s);
     c.rec_task_f.upload(P.f.tasks, s); c.rec_task_b.upload(P.b.tasks, s);
     c.rec_warps = P.warps; c.rec_tight = P.tight; c.rec_stage_bytes = P.stage_bytes;

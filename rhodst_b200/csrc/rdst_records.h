@@ -24,6 +24,7 @@
 //              the level buffers (a row of zeros past them where the row has
 //              no such slot), < 0 row -v - 1 of the global vector; with more
 //              than four slots, 16 bytes: rows that have more than k slots
+//   then per task
 //     values   the blocks' rows of five entries, in vector pieces so that
 //              lane (position, component) of a slot reads whole 16-byte (8
 //              for BF16) words, neighbouring lanes neighbouring words:
@@ -41,6 +42,8 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 namespace rdst {
@@ -61,8 +64,14 @@ constexpr int REC_FAR = 2;              // some column lies in the global vector
 struct RecGroup { uint32_t off16; uint32_t bytes; int32_t row0; int32_t nrows; };
 struct RecTask { uint32_t head16; uint32_t group16; };   // a task's header and its group, from the records' start / 16
 
+// The plan holds what is known of the records before the factors are: each
+// group's headers and columns (its first meta bytes), one after the other.
+struct RecMeta { uint32_t off16; uint32_t n16; };        // a group's part of RecSide::meta, in 16-byte words
+
 struct RecSide {
-    std::vector<unsigned char> rec;
+    std::vector<unsigned char> meta;
+    std::vector<RecMeta> group_meta;
+    size_t bytes = 0;                   // of the records
     std::vector<RecGroup> groups;
     std::vector<int> part_g;            // first group of each part
     std::vector<RecTask> tasks;
@@ -120,48 +129,45 @@ inline RecPlan rec_plan(int N, int nparts, const std::vector<int>& part_lvl0, co
     const int want = N > REC_ROWS * nlev ? REC_MAXW : 4;
     const size_t budget = std::min(smem_block, smem_sm / k - reserved) - 1024;    // static shared memory, alignment
 
-    struct Task { int r0, n, l; };
-    for (int W = std::min(wmax, want); W > 0; W /= 2) {
-        P.warps = W;
-        const int lbr = rec_lb_row_bytes(elem);
-        P.lb_rows = (int)std::min<size_t>(maxw, budget / 2 / (2 * (size_t)lbr));
-        P.lb_rows = std::min(P.lb_rows, 16383);
-        auto cnt = [&](int r, bool back) { return back ? nu[r] : nl[r]; };
-        // tasks of a sweep; the backward chunks of a level descend, so that
-        // consecutive tasks always cover one contiguous row range
-        auto tasks_of = [&](int p, bool back) {
-            std::vector<Task> t;
+    struct Task { int r0, n, l, S, tot; };
+    auto cnt = [&](int r, bool back) { return back ? nu[r] : nl[r]; };
+    auto meta_bytes = [&](const Task& t) {
+        return 32 + (size_t)16 * t.n * std::max(1, (t.S + 3) / 4) + (t.S > 4 ? 16 : 0);
+    };
+    auto value_bytes = [&](const Task& t) { return r16((size_t)t.tot * 25 * elem); };
+    // tasks of both sweeps; the backward chunks of a level descend, so that
+    // consecutive tasks always cover one contiguous row range
+    std::vector<Task> tasks[2];
+    std::vector<size_t> task0[2];
+    size_t max_one = 0, total[2] = {0, 0};
+    for (int back = 0; back < 2; ++back) {
+        task0[back].assign(nparts + 1, 0);
+        for (int p = 0; p < nparts; ++p) {
             const int a = part_lvl0[p], e = part_lvl0[p + 1];
             for (int i = 0; i < e - a; ++i) {
                 const int l = back ? e - 1 - i : a + i;
                 const int r0 = lvl_off[l], n = lvl_off[l + 1] - r0, nc = (n + REC_ROWS - 1) / REC_ROWS;
                 for (int c = 0; c < nc; ++c) {
                     const int cc = back ? nc - 1 - c : c;
-                    t.push_back({r0 + cc * REC_ROWS, std::min(REC_ROWS, n - cc * REC_ROWS), l});
+                    Task t{r0 + cc * REC_ROWS, std::min(REC_ROWS, n - cc * REC_ROWS), l, 0, 0};
+                    t.tot = back ? t.n : 0;
+                    for (int q = 0; q < t.n; ++q) {
+                        t.S = std::max(t.S, cnt(t.r0 + q, back));
+                        t.tot += cnt(t.r0 + q, back);
+                    }
+                    max_one = std::max(max_one, meta_bytes(t) + value_bytes(t));
+                    total[back] += meta_bytes(t) + value_bytes(t);
+                    tasks[back].push_back(t);
                 }
             }
-            return t;
-        };
-        auto widest = [&](const Task& t, bool back) {
-            int S = 0;
-            for (int i = 0; i < t.n; ++i) S = std::max(S, cnt(t.r0 + i, back));
-            return S;
-        };
-        auto data_bytes = [&](const Task& t, bool back) {
-            const int S = widest(t, back);
-            size_t tot = back ? t.n : 0;
-            for (int i = 0; i < t.n; ++i) tot += cnt(t.r0 + i, back);
-            return (size_t)16 * t.n * std::max(1, (S + 3) / 4) + (S > 4 ? 16 : 0) + r16(tot * 25 * elem);
-        };
-        size_t max_one = 0, total[2] = {0, 0}, ntasks[2] = {0, 0};
-        for (int p = 0; p < nparts; ++p)
-            for (int back = 0; back < 2; ++back)
-                for (const Task& t : tasks_of(p, back)) {
-                    const size_t b = 32 + data_bytes(t, back);
-                    max_one = std::max(max_one, b);
-                    total[back] += b;
-                    ++ntasks[back];
-                }
+            task0[back][p + 1] = tasks[back].size();
+        }
+    }
+    for (int W = std::min(wmax, want); W > 0; W /= 2) {
+        P.warps = W;
+        const int lbr = rec_lb_row_bytes(elem);
+        P.lb_rows = (int)std::min<size_t>(maxw, budget / 2 / (2 * (size_t)lbr));
+        P.lb_rows = std::min(P.lb_rows, 16383);
         // a warp may hold a stage until its task is computed while another
         // waits W - 1 tasks further on: that window must fit the stages
         const size_t room = budget - (2 * (size_t)P.lb_rows + 1) * lbr;
@@ -173,109 +179,134 @@ inline RecPlan rec_plan(int N, int nparts, const std::vector<int>& part_lvl0, co
         const size_t mean = std::max(total[0], total[1]) / N + 40;
         const size_t cap_rows = std::max<size_t>(qmin * REC_ROWS, std::min((cap - least) / 40, cap / mean));
         const size_t cap_bytes = cap - 40 * cap_rows;
-        // ---- groups
         size_t max_group = 0;
         int max_rows = 0;
         for (int back = 0; back < 2; ++back) {
             RecSide& S = back ? P.b : P.f;
-            S.rec.clear();
-            S.rec.reserve(total[back] + 16 * ntasks[back]);
+            const std::vector<Task>& ts = tasks[back];
+            // ---- groups, and per task its group and place there
+            std::vector<int> grp(ts.size()), place(ts.size());
+            std::vector<size_t> gstart;
             S.groups.clear();
-            S.tasks.clear();
             S.part_g.assign(nparts + 1, 0);
             for (int p = 0; p < nparts; ++p) {
-                S.part_g[p] = (int)S.groups.size();
-                const std::vector<Task> ts = tasks_of(p, back);
-                // group bounds and, per task, its group and place there
-                std::vector<size_t> gstart(1, 0);
-                std::vector<int> grp(ts.size()), place(ts.size());
-                {
-                    size_t bytes = 16, rows = 0;
-                    for (size_t t = 0; t < ts.size(); ++t) {
-                        const size_t b = 32 + data_bytes(ts[t], back), in = t - gstart.back();
-                        const size_t most = gstart.size() == 1 ? REC_RAMP0 : gstart.size() == 2 ? REC_RAMP1 : cap_bytes;
-                        if (in >= qmin && (bytes + b > std::min(most, cap_bytes) || rows + ts[t].n > cap_rows || in >= 255)) {
-                            gstart.push_back(t);
-                            bytes = 16;
-                            rows = 0;
-                        }
-                        bytes += b;
-                        rows += ts[t].n;
-                        grp[t] = (int)gstart.size() - 1;
-                        place[t] = (int)(t - gstart.back());
+                S.part_g[p] = (int)gstart.size();
+                size_t bytes = 0, rows = 0;
+                for (size_t t = task0[back][p]; t < task0[back][p + 1]; ++t) {
+                    const size_t b = meta_bytes(ts[t]) + value_bytes(ts[t]);
+                    const size_t nth = gstart.size() - S.part_g[p];      // groups of the part so far
+                    const size_t most = nth <= 1 ? REC_RAMP0 : nth == 2 ? REC_RAMP1 : cap_bytes;
+                    const size_t in = nth ? t - gstart.back() : 0;
+                    if (nth == 0 || (in >= qmin && (bytes + b > std::min(most, cap_bytes) ||
+                                                    rows + ts[t].n > cap_rows || in >= 255))) {
+                        gstart.push_back(t);
+                        bytes = 16;
+                        rows = 0;
                     }
-                    gstart.push_back(ts.size());
-                }
-                const int nlv = part_lvl0[p + 1] - part_lvl0[p];
-                for (size_t gi = 0; gi + 1 < gstart.size(); ++gi) {
-                    const size_t i = gstart[gi], j = gstart[gi + 1];
-                    int lo = ts[i].r0, hi = lo;
-                    size_t bytes = 16 + 32 * (j - i);
-                    for (size_t t = i; t < j; ++t) {
-                        lo = std::min(lo, ts[t].r0);
-                        hi = std::max(hi, ts[t].r0 + ts[t].n);
-                        bytes += data_bytes(ts[t], back);
-                    }
-                    const size_t g0 = S.rec.size();
-                    S.rec.resize(g0 + bytes, 0);
-                    unsigned char* g = S.rec.data() + g0;
-                    const int32_t gh[4] = {(int32_t)(j - i), lo, (int32_t)ts.size(), nlv};
-                    std::memcpy(g, gh, 16);
-                    size_t pos = 16 + 32 * (j - i);
-                    for (size_t t = i; t < j; ++t) {
-                        const Task& T = ts[t];
-                        int ord[REC_ROWS];
-                        for (int q = 0; q < T.n; ++q) ord[q] = q;
-                        std::stable_sort(ord, ord + T.n, [&](int a, int b2) {
-                            return cnt(T.r0 + a, back) > cnt(T.r0 + b2, back);
-                        });
-                        const int Sx = widest(T, back), nq = std::max(1, (Sx + 3) / 4);
-                        unsigned char nk[REC_MAXS] = {0};
-                        int tot = back ? T.n : 0;
-                        for (int q = 0; q < T.n; ++q)
-                            for (int s = 0; s < cnt(T.r0 + q, back); ++s) { ++nk[s]; ++tot; }
-                        const size_t coff = pos, voff = coff + (size_t)16 * T.n * nq + (Sx > 4 ? 16 : 0);
-                        if (Sx > 4) std::memcpy(g + voff - 16, nk, REC_MAXS);
-                        // levels as wide as the buffers are kept there
-                        auto kept = [&](int l) { return lvl_off[l + 1] - lvl_off[l] <= P.lb_rows; };
-                        const int own = kept(T.l) ? (T.l & 1) * P.lb_rows + T.r0 - lvl_off[T.l] : 0xffff;
-                        int32_t* cols = reinterpret_cast<int32_t*>(g + coff);
-                        for (int q = 0; q < T.n * 4 * nq; ++q) cols[q] = 2 * P.lb_rows * lbr;
-                        bool far = false;
-                        for (int s = 0; s < Sx; ++s)
-                            for (int q = 0; q < nk[s]; ++q) {
-                                const int c = lu_col[fid(T.r0 + ord[q], back ? ML + s : s)];
-                                const int lp = back ? T.l + 1 : T.l - 1;      // the level taken just before
-                                const bool near = lev[c] == lp && kept(lp);
-                                cols[((size_t)(s / 4) * T.n + q) * 4 + s % 4] =
-                                    near ? ((lp & 1) * P.lb_rows + c - lvl_off[lp]) * lbr : -1 - c;
-                                far |= !near;
-                            }
-                        // sweep-relative level, and the way to the warp's next task
-                        auto level_of = [&](size_t tt) {
-                            return back ? part_lvl0[p + 1] - 1 - ts[tt].l : ts[tt].l - part_lvl0[p];
-                        };
-                        const bool last = t + W >= ts.size();
-                        const int dl = last ? 0 : level_of(t + W) - level_of(t);
-                        const uint32_t fl = (last ? REC_WARP_LAST : 0) | (far ? REC_FAR : 0);
-                        uint32_t h[8] = {(uint32_t)(coff / 16) | (uint32_t)(voff / 16) << 16,
-                                         (uint32_t)T.n | (uint32_t)Sx << 8 | fl << 16 | (uint32_t)dl << 24,
-                                         (uint32_t)T.r0, (uint32_t)own | (uint32_t)tot << 16, 0u, 0u,
-                                         (uint32_t)level_of(t) << 16,
-                                         (last ? 0u : (uint32_t)place[t + W] | (uint32_t)(grp[t + W] - grp[t]) << 8) |
-                                             (uint32_t)(T.r0 - lo) << 16};
-                        for (int q = 0; q < 4; ++q) h[4] |= (uint32_t)nk[q] << (8 * q);
-                        for (int q = 0; q < T.n; ++q) h[5 + q / 4] |= (uint32_t)ord[q] << (8 * (q % 4));
-                        std::memcpy(g + 16 + 32 * (t - i), h, 32);
-                        S.tasks.push_back({(uint32_t)((g0 + 16 + 32 * (t - i)) / 16), (uint32_t)(g0 / 16)});
-                        pos += data_bytes(T, back);
-                    }
-                    S.groups.push_back({(uint32_t)(g0 / 16), (uint32_t)bytes, lo, hi - lo});
-                    max_group = std::max(max_group, bytes);
-                    max_rows = std::max(max_rows, hi - lo);
+                    bytes += b;
+                    rows += ts[t].n;
+                    grp[t] = (int)gstart.size() - 1;
+                    place[t] = (int)(t - gstart.back());
                 }
             }
-            S.part_g[nparts] = (int)S.groups.size();
+            S.part_g[nparts] = (int)gstart.size();
+            gstart.push_back(ts.size());
+            const size_t ng = gstart.size() - 1;
+            S.group_meta.assign(ng, RecMeta{0, 0});
+            S.tasks.assign(ts.size(), RecTask{0, 0});
+            size_t rec = 0, meta = 0;
+            for (size_t g = 0; g < ng; ++g) {
+                int lo = ts[gstart[g]].r0, hi = lo;
+                size_t mb = 16, vb = 0;
+                for (size_t t = gstart[g]; t < gstart[g + 1]; ++t) {
+                    lo = std::min(lo, ts[t].r0);
+                    hi = std::max(hi, ts[t].r0 + ts[t].n);
+                    mb += meta_bytes(ts[t]);
+                    vb += value_bytes(ts[t]);
+                    S.tasks[t] = {(uint32_t)(rec / 16 + 1 + 2 * (t - gstart[g])), (uint32_t)(rec / 16)};
+                }
+                S.groups.push_back({(uint32_t)(rec / 16), (uint32_t)(mb + vb), lo, hi - lo});
+                S.group_meta[g] = {(uint32_t)(meta / 16), (uint32_t)(mb / 16)};
+                rec += mb + vb;
+                meta += mb;
+                max_group = std::max(max_group, mb + vb);
+                max_rows = std::max(max_rows, hi - lo);
+            }
+            S.bytes = rec;
+            S.meta.assign(meta, 0);
+            // ---- headers and columns, the parts shared out over threads
+            auto kept = [&](int l) { return lvl_off[l + 1] - lvl_off[l] <= P.lb_rows; };   // levels the buffers hold
+            auto fill = [&](int p0, int p1) {
+                for (int p = p0; p < p1; ++p) {
+                    const size_t tend = task0[back][p + 1];
+                    const int nlv = part_lvl0[p + 1] - part_lvl0[p];
+                    auto level_of = [&](size_t t) {       // in the order of the sweep
+                        return back ? part_lvl0[p + 1] - 1 - ts[t].l : ts[t].l - part_lvl0[p];
+                    };
+                    for (int gi = S.part_g[p]; gi < S.part_g[p + 1]; ++gi) {
+                        const size_t i = gstart[gi], j = gstart[gi + 1];
+                        const RecGroup& G = S.groups[gi];
+                        unsigned char* g = S.meta.data() + (size_t)S.group_meta[gi].off16 * 16;
+                        const int32_t gh[4] = {(int32_t)(j - i), G.row0, (int32_t)(tend - task0[back][p]), nlv};
+                        std::memcpy(g, gh, 16);
+                        size_t coff = 16 + 32 * (j - i), voff = (size_t)S.group_meta[gi].n16 * 16;
+                        for (size_t t = i; t < j; ++t) {
+                            const Task& T = ts[t];
+                            int ord[REC_ROWS];
+                            for (int q = 0; q < T.n; ++q) ord[q] = q;
+                            std::stable_sort(ord, ord + T.n, [&](int a, int b) {
+                                return cnt(T.r0 + a, back) > cnt(T.r0 + b, back);
+                            });
+                            const int nq = std::max(1, (T.S + 3) / 4);
+                            unsigned char nk[REC_MAXS] = {0};
+                            for (int q = 0; q < T.n; ++q)
+                                for (int s = 0; s < cnt(T.r0 + q, back); ++s) ++nk[s];
+                            if (T.S > 4) std::memcpy(g + coff + (size_t)16 * T.n * nq, nk, REC_MAXS);
+                            int32_t* cols = reinterpret_cast<int32_t*>(g + coff);
+                            for (int q = 0; q < T.n * 4 * nq; ++q) cols[q] = 2 * P.lb_rows * lbr;
+                            const int own = kept(T.l) ? (T.l & 1) * P.lb_rows + T.r0 - lvl_off[T.l] : 0xffff;
+                            const int lp = back ? T.l + 1 : T.l - 1;          // the level taken just before
+                            bool far = false;
+                            for (int s = 0; s < T.S; ++s)
+                                for (int q = 0; q < nk[s]; ++q) {
+                                    const int c = lu_col[fid(T.r0 + ord[q], back ? ML + s : s)];
+                                    const bool near = lev[c] == lp && kept(lp);
+                                    cols[((size_t)(s / 4) * T.n + q) * 4 + s % 4] =
+                                        near ? ((lp & 1) * P.lb_rows + c - lvl_off[lp]) * lbr : -1 - c;
+                                    far |= !near;
+                                }
+                            // the way to the warp's next task
+                            const bool last = t + W >= tend;
+                            const int dl = last ? 0 : level_of(t + W) - level_of(t);
+                            const uint32_t fl = (last ? REC_WARP_LAST : 0) | (far ? REC_FAR : 0);
+                            uint32_t h[8] = {(uint32_t)(coff / 16) | (uint32_t)(voff / 16) << 16,
+                                             (uint32_t)T.n | (uint32_t)T.S << 8 | fl << 16 | (uint32_t)dl << 24,
+                                             (uint32_t)T.r0, (uint32_t)own | (uint32_t)T.tot << 16, 0u, 0u,
+                                             (uint32_t)level_of(t) << 16,
+                                             (last ? 0u : (uint32_t)place[t + W] | (uint32_t)(grp[t + W] - grp[t]) << 8) |
+                                                 (uint32_t)(T.r0 - G.row0) << 16};
+                            for (int q = 0; q < 4; ++q) h[4] |= (uint32_t)nk[q] << (8 * q);
+                            for (int q = 0; q < T.n; ++q) h[5 + q / 4] |= (uint32_t)ord[q] << (8 * (q % 4));
+                            std::memcpy(g + 16 + 32 * (t - i), h, 32);
+                            coff += meta_bytes(T) - 32;
+                            voff += value_bytes(T);
+                        }
+                    }
+                }
+            };
+            const int nt = (int)std::min<size_t>({8, std::max(1u, std::thread::hardware_concurrency()), ts.size() / 2048 + 1,
+                                                  (size_t)nparts});
+            std::vector<std::thread> th;
+            for (int k2 = 1; k2 < nt; ++k2) {
+                const int p0 = (int)((long)nparts * k2 / nt), p1 = (int)((long)nparts * (k2 + 1) / nt);
+                try {
+                    th.emplace_back(fill, p0, p1);
+                } catch (const std::system_error&) {      // no thread to be had
+                    fill(p0, p1);
+                }
+            }
+            fill(0, (int)((long)nparts / nt));
+            for (auto& x : th) x.join();
         }
         P.stage_bytes = (int)((max_group + 127) / 128 * 128);
         P.y0_rows = (max_rows + 1) / 2 * 2;

@@ -108,21 +108,27 @@ extern "C" int check_records(int n, int nparts, int wide, int reach, int elem, i
         size_t task_no = 0;
         for (int p = 0; p < nparts; ++p) {
             // the tasks in sweep order, then each warp's walk over them
-            struct At { const RecGroup* G; const unsigned char* gp; int g, t; };
+            struct At { const RecGroup* G; const unsigned char* gp; int g, t, meta; };
+            int end_meta = 0;
             std::vector<At> tasks;
             int32_t sweep_tasks = 0, sweep_levels = 0;
             for (int g = S.part_g[p]; g < S.part_g[p + 1]; ++g) {
                 const RecGroup& G = S.groups[g];
                 if (G.bytes % 16 || (int)G.bytes > P.stage_bytes || G.nrows > P.y0_rows) return fail("group size", p, g);
-                if ((size_t)G.off16 * 16 + G.bytes > S.rec.size()) return fail("group outside the records");
-                const unsigned char* gp = S.rec.data() + (size_t)G.off16 * 16;
+                if ((size_t)G.off16 * 16 + G.bytes > S.bytes) return fail("group outside the records");
+                if (g > 0 && (size_t)G.off16 * 16 != (size_t)S.groups[g - 1].off16 * 16 + S.groups[g - 1].bytes)
+                    return fail("groups not one after the other", g);
+                const RecMeta& M = S.group_meta[g];
+                if (((size_t)M.off16 + M.n16) * 16 > S.meta.size() || (size_t)M.n16 * 16 > G.bytes) return fail("group meta", g);
+                const unsigned char* gp = S.meta.data() + (size_t)M.off16 * 16;
+                end_meta = 16 * M.n16;
                 int32_t gh[4];
                 std::memcpy(gh, gp, 16);
                 if (gh[1] != G.row0 || gh[0] < 1 || gh[0] > 256) return fail("group header");
                 sweep_tasks = gh[2];
                 sweep_levels = gh[3];
                 for (int t = 0; t < gh[0]; ++t) {
-                    tasks.push_back({&G, gp, g, t});
+                    tasks.push_back({&G, gp, g, t, end_meta});
                     const RecTask& T = S.tasks.at(task_no++);
                     if (T.group16 != G.off16 || T.head16 != G.off16 + 1 + 2 * (uint32_t)t) return fail("task list", g, t);
                 }
@@ -163,14 +169,15 @@ extern "C" int check_records(int n, int nparts, int wide, int reach, int elem, i
                 const unsigned fl = (h[1] >> 16) & 255;
                 const int r0 = (int)h[2], own = h[3] & 0xffff, tot = h[3] >> 16;
                 const int nq = std::max(1, (Sx + 3) / 4), lbr = rec_lb_row_bytes(elem), none = 2 * P.lb_rows * lbr;
-                if (Sx > 4) std::memcpy(nk, gp + voff - 16, REC_MAXS);
+                if (Sx > 4) std::memcpy(nk, gp + coff + 16 * m * nq, REC_MAXS);
                 if (m < 1 || m > REC_ROWS) return fail("task", g, t);
                 std::vector<char> filled(tot, 0);
                 for (int q = 0; back && q < m; ++q) ++filled[q];
                 if (r0 - G.row0 != (int)(h[7] >> 16) || r0 < G.row0 || r0 + m > G.row0 + G.nrows)
                     return fail("rows outside the group's range", g, t);
                 if ((size_t)voff + (size_t)tot * 25 * elem > G.bytes) return fail("values outside the group", g, t);
-                if (coff + 16 * m * nq + (Sx > 4 ? 16 : 0) > voff) return fail("columns over the values", g, t);
+                if (coff + 16 * m * nq + (Sx > 4 ? 16 : 0) > tasks[ti].meta || voff < tasks[ti].meta)
+                    return fail("columns and values", g, t);
                 char seen[REC_ROWS] = {0};
                 for (int q = 0; q < m; ++q) {
                     const int rid = (h[5 + q / 4] >> (8 * (q % 4))) & 255, r = r0 + rid;

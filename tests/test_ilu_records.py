@@ -14,7 +14,7 @@ HERE = Path(__file__).resolve().parent
 @pytest.fixture(scope="module")
 def lib(tmp_path_factory):
     so = tmp_path_factory.mktemp("rec") / "ilu_records_check.so"
-    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-o", str(so),
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-pthread", "-o", str(so),
                     str(HERE / "ilu_records_check.cpp")], check=True)
     return ctypes.CDLL(str(so))
 
