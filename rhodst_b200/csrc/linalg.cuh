@@ -243,6 +243,7 @@ struct IluDev {
     const int* part_gb;
     const RecTask* task_f;
     const RecTask* task_b;
+    const int* part_tf;     // first forward task of each part
     // the direct factorisation's addressing (null: gather + factor
     // instead).  Per update triple (tr_start ranges):
     // fr_trk: where U_kj is read, the flat SELL slot of A_kj (>= 0), factor
@@ -850,6 +851,253 @@ __global__ void __launch_bounds__(256) k_ilu_pack(int nf, int nb, SellMat<MT> A,
         }
         blk += nk;
     }
+}
+
+// ---- the factorisation on the apply's tasks
+//
+// Where no row updates blocks of its own (no three cells of a subdomain are
+// pairwise neighbours: quads, hexahedra, the Kuhn tetrahedra and prisms; and
+// Gauss-Seidel, which updates nothing) row r of the factorisation is
+//   L_rk = A_rk D_k,  D_r = (A_rr - sum_k L_rk A_kr)^-1   over its lower k,
+// a chain of levels like the apply's, and it takes the forward sweep's tasks
+// in the same way: six rows a warp, five lanes a row (lane i: block row i),
+// the W warps taking turns, a named barrier per level.  Before its level a
+// warp has the rows of A_rr and A_rk in registers and the blocks A_kr in
+// shared memory; what waits for the level before is D_k from the level
+// buffers (25 entries a row, by level parity; LBUF false: from global memory
+// where the buffers do not fit), the two products and the inverse.  The
+// inverse is the Gauss-Jordan elimination of inv5 with the rows on five
+// lanes: the pivot row travels by shuffle, row swaps are a change of labels.
+// L goes straight into the forward records, so only the backward ones are
+// packed afterwards.  Same operations and roundings as k_ilu_factor_direct
+// (a row in one thread, ~7,000 cycles a level), which stays for the patterns
+// with triangles or fill.  Factorisation and pack, us: 257x65 airfoil FP64 218
+// -> 100, RAE2822 334 -> 166, 442 k-cell wing FP64 968 -> 540, 371 k BF16 746 ->
+// 301; 1.2 M FP32 (three warps a CTA, six CTAs an SM) 1232 -> 1225.
+template <typename MT, int NBP, bool TIGHT, bool LBUF>
+__global__ void __launch_bounds__(TIGHT ? 96 : 256, TIGHT ? 6 : 2)
+    k_ilu_factor_rec(SellMat<MT> A, MT* dinv, IluDev P) {
+    using CT = typename IluCT<MT>::T;
+    constexpr int RS = sizeof(CT) == 8 ? 26 : 28;           // 25 entries padded to 16 bytes
+    constexpr int NBAR = TIGHT ? 4 : 15;                    // as in k_ilu_apply_rec
+    extern __shared__ __align__(16) unsigned char s_fac[];
+    CT* s_u = reinterpret_cast<CT*>(s_fac);                 // [W][6][NBP][RS]
+    const int part = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
+    CT* s_d = s_u + (size_t)W * REC_ROWS * NBP * RS;        // [2 lb_rows][RS]
+    const int rsub = lane / 5, comp = lane - 5 * rsub, sbase = lane < 30 ? 5 * rsub : 0;
+    const int pos0 = lane < 30 ? rsub : 0x7fffffff;
+    const int nlev = P.part_lvl0[part + 1] - P.part_lvl0[part];
+    const int t1 = P.part_tf[part + 1];
+    int arrived = 0, bid = 1;
+    auto arrive = [&] {
+        if (W > 1) {
+            if (!TIGHT) asm volatile("bar.arrive %0, %1;" ::"r"(bid), "r"(W * 32) : "memory");
+            else if (bid == 1) asm volatile("bar.arrive 1, %0;" ::"r"(W * 32) : "memory");
+            else if (bid == 2) asm volatile("bar.arrive 2, %0;" ::"r"(W * 32) : "memory");
+            else if (bid == 3) asm volatile("bar.arrive 3, %0;" ::"r"(W * 32) : "memory");
+            else asm volatile("bar.arrive 4, %0;" ::"r"(W * 32) : "memory");
+        }
+        bid = bid == NBAR ? 1 : bid + 1;
+        ++arrived;
+    };
+    auto await = [&] {
+        if (W > 1) {
+            if (!TIGHT) asm volatile("bar.sync %0, %1;" ::"r"(bid), "r"(W * 32) : "memory");
+            else if (bid == 1) asm volatile("bar.sync 1, %0;" ::"r"(W * 32) : "memory");
+            else if (bid == 2) asm volatile("bar.sync 2, %0;" ::"r"(W * 32) : "memory");
+            else if (bid == 3) asm volatile("bar.sync 3, %0;" ::"r"(W * 32) : "memory");
+            else asm volatile("bar.sync 4, %0;" ::"r"(W * 32) : "memory");
+        } else {
+            __syncwarp();
+        }
+        bid = bid == NBAR ? 1 : bid + 1;
+        ++arrived;
+    };
+    // the current task
+    CT D[5], Ar[NBP][5];
+    int cq[NBP], kq[NBP];
+    int n = 0, S = 0, tot = 0, r = 0, dl = 0, own = 0, q0 = 0;
+    unsigned nk4 = 0, last = 0;
+    bool act = false, kept = false;
+    unsigned char* vals = nullptr;
+    const unsigned char *cols = nullptr, *nks = nullptr;
+    bool upd[NBP];
+    auto load = [&](int t) {
+        const RecTask tk = P.task_f[t];
+        const unsigned char* hp = P.rec_f + (size_t)tk.head16 * 16;
+        const uint4 h = *reinterpret_cast<const uint4*>(hp), g = *reinterpret_cast<const uint4*>(hp + 16);
+        n = (int)(h.y & 255u);
+        S = (int)((h.y >> 8) & 255u);
+        last = (h.y >> 16) & REC_WARP_LAST;
+        dl = (int)(h.y >> 24);
+        tot = (int)(h.w >> 16);
+        nk4 = g.x;
+        act = pos0 < n;
+        const int pos = act ? pos0 : 0;
+        cols = P.rec_f + (size_t)tk.group16 * 16 + 16 * (size_t)(h.x & 0xffffu);
+        nks = cols + 16 * (size_t)(n * ((S + 3) >> 2));
+        vals = P.rec_f + (size_t)tk.group16 * 16 + 16 * (size_t)(h.x >> 16);
+        const int rid = (int)((pos < 4 ? g.y >> (8 * pos) : g.z >> (8 * (pos - 4))) & 255u);
+        r = (int)h.z + rid;
+        kept = (h.w & 0xffffu) != 0xffffu;
+        own = (int)(h.w & 0xffffu) + rid;
+        q0 = P.low_start[r];
+        const int4 c4 = *reinterpret_cast<const int4*>(cols + 16 * pos);
+        const int ca[4] = {c4.x, c4.y, c4.z, c4.w};
+        const MT* dv = A.val + (size_t)A.slice_off[r >> 5] * (32 * 25) + (r & 31);
+#pragma unroll
+        for (int j = 0; j < 5; ++j) D[j] = ct_ld(dv + (5 * comp + j) * 32);
+        CT* u = s_u + ((size_t)(warp * REC_ROWS + pos) * NBP) * RS + 5 * comp;
+#pragma unroll
+        for (int q = 0; q < NBP; ++q) {
+            cq[q] = ca[q];
+            upd[q] = false;
+            kq[q] = -1;
+            if (act && pos0 < (int)((nk4 >> (8 * q)) & 255u)) {
+                const int4 d = P.fr_desc[q0 + q];
+                kq[q] = d.x;
+                upd[q] = (d.w & 0xfffff) != 0;
+                const MT* a = A.val + flat_e(d.y, 5 * comp);
+#pragma unroll
+                for (int j = 0; j < 5; ++j) Ar[q][j] = ct_ld(a + j * 32);
+                if (upd[q]) {
+                    const MT* b = A.val + flat_e(d.z, 5 * comp);
+#pragma unroll
+                    for (int j = 0; j < 5; ++j) u[q * RS + j] = ct_ld(b + j * 32);
+                }
+            }
+        }
+        __syncwarp();
+        return (int)(g.z >> 16);
+    };
+    // D_k of one lower neighbour: from the level buffer row of byte offset c
+    // of the apply's buffers, or (far, or no buffers) from global memory
+    auto pivot_of = [&](int c, int k, CT (&o)[25]) {
+        if (LBUF && c >= 0) {
+            const CT* p = s_d + (size_t)(c / (sizeof(CT) == 8 ? 48 : 32)) * RS;
+            constexpr int V = 16 / (int)sizeof(CT);
+            alignas(16) CT tmp[RS];
+#pragma unroll
+            for (int e = 0; e < RS; e += V)
+                *reinterpret_cast<uint4*>(tmp + e) = *reinterpret_cast<const uint4*>(p + e);
+#pragma unroll
+            for (int e = 0; e < 25; ++e) o[e] = tmp[e];
+        } else {
+            const MT* p = dinv + flat_e(k, 0);
+#pragma unroll
+            for (int e = 0; e < 25; ++e) o[e] = ct_ld(p + e * 32);
+        }
+    };
+    // L_rk = A_rk D_k (this lane's row), into the records too; then D -= L_rk U
+    auto lower = [&](const CT (&a5)[5], const CT (&Dk)[25], int blk, CT (&L5)[5]) {
+        MT o[5];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            CT a = 0;
+#pragma unroll
+            for (int t = 0; t < 5; ++t) a += a5[t] * Dk[5 * t + j];
+            L5[j] = a;
+            ct_st(&o[j], a);
+        }
+        rec_store(vals, tot, 5 * blk + comp, o);
+    };
+    auto update = [&](const CT (&L5)[5], auto u) {
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            CT a = 0;
+#pragma unroll
+            for (int t = 0; t < 5; ++t) a += L5[t] * u(5 * t + j);
+            D[j] -= a;
+        }
+    };
+    int t = P.part_tf[part] + warp;
+    if (t < t1) {
+        const int level = load(t);
+        while (arrived < level - 1) arrive();
+        if (arrived < level) await();
+        for (;;) {
+            if (act) {
+                int blk = pos0;
+#pragma unroll
+                for (int q = 0; q < NBP; ++q) {
+                    const int nk = (int)((nk4 >> (8 * q)) & 255u);
+                    if (pos0 < nk) {
+                        CT Dk[25];
+                        pivot_of(cq[q], kq[q], Dk);
+                        CT L5[5];
+                        lower(Ar[q], Dk, blk, L5);
+                        const CT* u = s_u + ((size_t)(warp * REC_ROWS + pos0) * NBP + q) * RS;
+                        if (upd[q]) update(L5, [&](int e) { return u[e]; });
+                    }
+                    blk += nk;
+                }
+                for (int q = NBP; q < S; ++q) {
+                    const int nk = q < 4 ? (int)((nk4 >> (8 * q)) & 255u) : (int)nks[q];
+                    if (pos0 < nk) {
+                        const int4 d = P.fr_desc[q0 + q];
+                        const int c = reinterpret_cast<const int*>(cols)[4 * ((q >> 2) * n + pos0) + (q & 3)];
+                        CT Dk[25], a5[5], L5[5];
+                        pivot_of(c, d.x, Dk);
+#pragma unroll
+                        for (int j = 0; j < 5; ++j) a5[j] = ct_ld(A.val + flat_e(d.y, 5 * comp + j));
+                        lower(a5, Dk, blk, L5);
+                        if (d.w & 0xfffff) update(L5, [&](int e) { return ct_ld(A.val + flat_e(d.z, e)); });
+                    }
+                    blk += nk;
+                }
+            }
+            // X = D^-1: lane `comp` of a row holds row `row` of [D | I]; lane_of
+            // packs the lane that holds each row, three bits each
+            CT a[10];
+#pragma unroll
+            for (int j = 0; j < 5; ++j) { a[j] = D[j]; a[5 + j] = comp == j ? CT(1) : CT(0); }
+            int row = comp;
+            unsigned lane_of = 0u | 1u << 3 | 2u << 6 | 3u << 9 | 4u << 12;
+#pragma unroll
+            for (int c = 0; c < 5; ++c) {
+                int p = c;
+                CT best = CT(0);
+#pragma unroll
+                for (int q = c; q < 5; ++q) {
+                    const CT v = fabs(__shfl_sync(0xffffffffu, a[c], sbase + (int)((lane_of >> (3 * q)) & 7u)));
+                    if (q == c) best = v;
+                    else if (v > best) { best = v; p = q; }
+                }
+                if (p != c) {
+                    const unsigned lc = (lane_of >> (3 * c)) & 7u, lp = (lane_of >> (3 * p)) & 7u;
+                    lane_of ^= (lc ^ lp) << (3 * c) | (lc ^ lp) << (3 * p);
+                    row = row == c ? p : (row == p ? c : row);
+                }
+                const CT piv = CT(1) / a[c];
+                const bool mine = row == c;
+                const CT f = a[c];
+                const int src = sbase + (int)((lane_of >> (3 * c)) & 7u);
+#pragma unroll
+                for (int j = c + 1; j < 10; ++j) {
+                    if (mine) a[j] *= piv;
+                    const CT pr = __shfl_sync(0xffffffffu, a[j], src);
+                    if (!mine && f != CT(0)) a[j] -= f * pr;
+                }
+            }
+            if (act) {
+#pragma unroll
+                for (int j = 0; j < 5; ++j) {
+                    MT o;
+                    ct_st(&o, a[5 + j]);
+                    dinv[flat_e(r, 5 * row + j)] = o;
+                    if (LBUF && kept) s_d[(size_t)own * RS + 5 * row + j] = ct_ld(&o);
+                }
+            }
+            if (last) break;
+            for (int q = 1; q < dl; ++q) arrive();
+            const bool wait = dl > 0;
+            t += W;
+            __syncwarp();
+            load(t);
+            if (wait) await();
+        }
+    }
+    while (arrived < nlev - 1) arrive();
 }
 
 template <typename MT, int NB, bool EXT, bool TIGHT>

@@ -274,6 +274,9 @@ struct rdst_ctx {
     DBuf<RecGroup> grp_f, grp_b;
     DBuf<int> part_gf, part_gb;
     DBuf<RecTask> rec_task_f, rec_task_b;
+    DBuf<int> rec_part_tf;
+    bool fac_rec = false, fac_lbuf = false;     // factorisation on the records' tasks; its level buffers fit
+    size_t fac_smem = 0;
     bool rec_tight = false;
     int rec_warps = 0, rec_stage_bytes = 0, rec_y0_rows = 0, rec_lb_rows = 0;
     size_t rec_smem_bytes = 0;
@@ -411,6 +414,7 @@ struct rdst_ctx {
         P.tr_start = tr_start.p; P.tr_kj = tr_kj.p; P.tr_rj = tr_rj.p;
         P.rec_f = rec_f.p; P.rec_b = rec_b.p; P.grp_f = grp_f.p; P.grp_b = grp_b.p;
         P.part_gf = part_gf.p; P.part_gb = part_gb.p; P.task_f = rec_task_f.p; P.task_b = rec_task_b.p;
+        P.part_tf = rec_part_tf.p;
         P.fr_trk = fr_trk.p; P.fr_trt = fr_trt.p; P.fr_desc = fr_desc.p;
         return P;
     }
@@ -591,6 +595,7 @@ void build_records(rdst_ctx& c, const Options& o, int nparts, const std::vector<
     }
     c.part_gf.upload(P.f.part_g, s); c.part_gb.upload(P.b.part_g, s);
     c.rec_task_f.upload(P.f.tasks, s); c.rec_task_b.upload(P.b.tasks, s);
+    c.rec_part_tf.upload(P.f.part_t, s);
     c.rec_warps = P.warps; c.rec_tight = P.tight; c.rec_stage_bytes = P.stage_bytes;
     c.rec_y0_rows = P.y0_rows; c.rec_lb_rows = P.lb_rows; c.rec_smem_bytes = rec_smem(P, S);
     // the factorisation reading A directly: where each update triple reads
@@ -619,6 +624,17 @@ void build_records(rdst_ctx& c, const Options& o, int nparts, const std::vector<
             c.fr_trt.upload(trt, s);
             c.fr_desc.upload(desc, s);
             c.ilu_direct = true;
+            // every lower block in the matrix, and it updates the diagonal
+            // alone (from a block of A) or nothing
+            c.fac_rec = true;
+            for (const int4& d : desc) c.fac_rec = c.fac_rec && d.y >= 0 && (d.w == 0 || (d.w == 1 && d.z >= 0));
+            const int k = std::min(6, std::max(1, (nparts + sms - 1) / std::max(sms, 1)));
+            const size_t ct = S == 8 ? 8 : 4, row = (S == 8 ? 26 : 28) * ct;
+            const size_t room = std::min((size_t)per_block, (size_t)per_sm / k - reserved) - 256;
+            c.fac_smem = (size_t)c.rec_warps * REC_ROWS * (std::max(ML, 1) <= 2 ? 2 : 3) * row;
+            c.fac_lbuf = c.fac_smem + 2 * (size_t)c.rec_lb_rows * row <= room;
+            if (c.fac_lbuf) c.fac_smem += 2 * (size_t)c.rec_lb_rows * row;
+            c.fac_rec = c.fac_rec && c.fac_smem <= (size_t)per_block - 256;
         }
     }
     CK(cudaStreamSynchronize(s));
@@ -1131,8 +1147,22 @@ static void ilu_rec_instance(int width, bool tight, F&& f) {
 }
 // dynamic shared memory above the default 48 KB: set when a context is
 // built (not while a step is being captured)
+template <typename MT, typename F>
+static void ilu_fac_instance(int width, bool tight, bool lbuf, F&& f) {
+    auto pick = [&](auto nb) {
+        constexpr int NB = decltype(nb)::value;
+        if (tight) { if (lbuf) f(k_ilu_factor_rec<MT, NB, true, true>); else f(k_ilu_factor_rec<MT, NB, true, false>); }
+        else { if (lbuf) f(k_ilu_factor_rec<MT, NB, false, true>); else f(k_ilu_factor_rec<MT, NB, false, false>); }
+    };
+    if (width <= 2) pick(std::integral_constant<int, 2>());
+    else pick(std::integral_constant<int, 3>());
+}
 template <typename MT>
 static void ilu_rec_attr() {
+    for (int width : {2, 3})
+        for (bool tight : {false, true})
+            for (bool lbuf : {false, true})
+                ilu_fac_instance<MT>(width, tight, lbuf, [](auto* k) { set_max_dyn_smem(k); });
     for (int width : {2, 3})
         for (bool tight : {false, true}) ilu_rec_instance<MT>(width, tight, [](auto* k) { set_max_dyn_smem(k); });
 }
@@ -1144,11 +1174,12 @@ static void ilu_apply_rec(rdst_ctx& c, const IluDev& P, const double* in, double
                                                          c.rec_lb_rows, &c.sc.p->flags);
     });
 }
-// blocks of the fresh factors -> the records
+// blocks of the fresh factors -> the records (the backward ones alone after
+// k_ilu_factor_rec)
 template <typename MT>
 static void ilu_pack(rdst_ctx& c, void* val) {
     if (!c.rec_f.p) return;
-    const int nf = (int)c.rec_task_f.n, nb = (int)c.rec_task_b.n;
+    const int nf = c.fac_rec ? 0 : (int)c.rec_task_f.n, nb = (int)c.rec_task_b.n;
     k_ilu_pack<MT><<<nblk(32L * (nf + nb), 256), 256, 0, c.s>>>(nf, nb, c.mat<MT>(val), (const MT*)c.LUval,
                                                                (const MT*)c.dinv, c.ilu());
     CKL();
@@ -1159,7 +1190,12 @@ static void ilu_pack(rdst_ctx& c, void* val) {
 // then packed into the bulk apply's records when there are records
 template <typename MT>
 static void ilu_factorise(rdst_ctx& c, void* val) {
-    if (c.ilu_direct) {
+    if (c.fac_rec) {
+        ilu_fac_instance<MT>(c.ilu_ml, c.rec_tight, c.fac_lbuf, [&](auto* k) {
+            k<<<c.n_parts, 32 * c.rec_warps, c.fac_smem, c.s>>>(c.mat<MT>(val), (MT*)c.dinv, c.ilu());
+        });
+        CKL();
+    } else if (c.ilu_direct) {
         k_ilu_factor_direct<MT><<<c.n_parts, 32, 0, c.s>>>(c.mat<MT>(val), (MT*)c.LUval, (MT*)c.dinv, c.ilu());
         CKL();
     } else {

@@ -75,6 +75,7 @@ struct RecSide {
     std::vector<RecGroup> groups;
     std::vector<int> part_g;            // first group of each part
     std::vector<RecTask> tasks;
+    std::vector<int> part_t;            // first task of each part
 };
 
 struct RecPlan {
@@ -214,6 +215,7 @@ inline RecPlan rec_plan(int N, int nparts, const std::vector<int>& part_lvl0, co
             const size_t ng = gstart.size() - 1;
             S.group_meta.assign(ng, RecMeta{0, 0});
             S.tasks.assign(ts.size(), RecTask{0, 0});
+            S.part_t.assign(task0[back].begin(), task0[back].end());
             size_t rec = 0, meta = 0;
             for (size_t g = 0; g < ng; ++g) {
                 int lo = ts[gstart[g]].r0, hi = lo;
