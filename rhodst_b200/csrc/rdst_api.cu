@@ -349,6 +349,8 @@ struct rdst_ctx {
     long ks_launches[KS_N] = {0, 0, 0, 0, 0, 0, 0};
     double ks_ms[KS_N] = {0, 0, 0, 0, 0, 0, 0};
     cudaEvent_t step_ev[2] = {nullptr, nullptr};
+    int* conv_host = nullptr;           // convergence flags on their way to the host (pinned)
+    cudaEvent_t conv_ev[2] = {nullptr, nullptr};
     double last_step_ms = 0.0;
     cudaEvent_t get_event() {
         if (!ev_pool.empty()) { cudaEvent_t e = ev_pool.back(); ev_pool.pop_back(); return e; }
@@ -388,6 +390,8 @@ struct rdst_ctx {
     ~rdst_ctx() {
         for (auto e : ev_pool) cudaEventDestroy(e);
         for (auto e : step_ev) if (e) cudaEventDestroy(e);
+        for (auto e : conv_ev) if (e) cudaEventDestroy(e);
+        if (conv_host) cudaFreeHost(conv_host);
         for (auto& r : ev_pending) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
         for (Graph* g : {&g_step, &g_pre, &g_cycle, &g_post}) {
             if (g->exec) cudaGraphExecDestroy(g->exec);
@@ -1436,22 +1440,16 @@ struct Ops {
         k_linres_finalize<<<1, RED_TPB, 0, s>>>(c.partial.p, nb, c.sc.p, 1); CKL();
         CK(cudaMemsetAsync(c.dx.p, 0, sizeof(double) * c.nvec(), s));
         CK(cudaMemsetAsync(&c.sc.p->lin_iterations, 0, sizeof(int), s));
-        k_check<<<1, 1, 0, s>>>(c.sc.p, c.o.tolerance, c.o.rel_tol, c.o.min_iter, c.o.max_iter, 0); CKL();
+        k_check<<<1, 1, 0, s>>>(c.sc.p, criteria(c), 0); CKL();
         if (c.o.solver == SOLVER_BICGSTAB) {
-            CK(cudaMemcpyAsync(c.r.p, c.rhs.p, sizeof(double) * c.nvec(), cudaMemcpyDeviceToDevice, s));
-            CK(cudaMemcpyAsync(c.Vb.p, c.rhs.p, sizeof(double) * c.nvec(), cudaMemcpyDeviceToDevice, s));  // rw
-            c.pv.zero(s);
-            CK(cudaMemsetAsync(c.ph.p, 0, sizeof(double) * c.nvec(), s));
-            k_bi_init<<<1, 1, 0, s>>>(c.sc.p); CKL();
+            Scalars* sc = c.sc.p;
+            double *rw = c.Vb.p, *part = c.orth_part.p;
+            int n = N;
+            void* args[] = {&n, &c.rhs.p, &c.r.p, &rw, &c.t.p, &c.pv.p, &part, &sc};
+            coop(c, (const void*)k_bi_start, args);
         } else if (c.o.solver != SOLVER_GMRES) {
             CK(cudaMemcpyAsync(c.r.p, c.rhs.p, sizeof(double) * c.nvec(), cudaMemcpyDeviceToDevice, s));
         }
-    }
-    static void dot(rdst_ctx& c, const double* a, const double* b, double* out, int sq, const int* active) {
-        long n = c.nvec();
-        int nb = red_blocks(n);
-        k_multidot<<<nb, RED_TPB, 0, c.s>>>(n, 1, a, 0, b, c.partial.p, 8, active); CKL();
-        k_finalize<<<1, RED_TPB, 0, c.s>>>(c.partial.p, nb, 1, 8, out, sq, active); CKL();
     }
     // w orthogonalised against V_0..V_{nv-1} and (vout) stored normalised, or
     // (nv 0) the cycle's start; all blocks resident (k_orth)
@@ -1512,33 +1510,31 @@ struct Ops {
         int nb = red_blocks(c.N);
         k_abs5<<<nb, RED_TPB, 0, c.s>>>(c.N, c.r.p, c.partial.p); CKL();
         k_linres_finalize<<<1, RED_TPB, 0, c.s>>>(c.partial.p, nb, c.sc.p, 0); CKL();
-        k_check<<<1, 1, 0, c.s>>>(c.sc.p, c.o.tolerance, c.o.rel_tol, c.o.min_iter, c.o.max_iter, 1); CKL();
+        k_check<<<1, 1, 0, c.s>>>(c.sc.p, criteria(c), 1); CKL();
     }
     // one BiCGStab iteration (van der Vorst, right preconditioned)
     static void bicgstab_iter(rdst_ctx& c) {
-        cudaStream_t s = c.s;
-        const long n = c.nvec();
         Scalars* sc = c.sc.p;
-        double* rw = c.Vb.p;
-        double* t2 = c.Vb.p + n;
-        dot(c, rw, c.r.p, &sc->dots[0], 0, nullptr);
-        k_bi_scal_rho<<<1, 1, 0, s>>>(sc); CKL();
-        k_bi_p<<<nblk(n, TPB), TPB, 0, s>>>(n, c.r.p, c.pv.p, c.t.p, sc); CKL();      // t holds p
-        precond(c, c.t.p, c.ph.p, nullptr);
-        spmv(c, c.ph.p, c.pv.p, nullptr, nullptr);                                  // v = A ph
-        dot(c, rw, c.pv.p, &sc->dots[0], 0, nullptr);
-        k_bi_scal_alpha<<<1, 1, 0, s>>>(sc); CKL();
-        k_bi_s<<<nblk(n, TPB), TPB, 0, s>>>(n, c.r.p, c.pv.p, c.s2.p, sc); CKL();
-        precond(c, c.s2.p, c.sh.p, nullptr);
-        spmv(c, c.sh.p, t2, nullptr, nullptr);
-        dot(c, t2, t2, &sc->dots[0], 0, nullptr);
-        dot(c, t2, c.s2.p, &sc->dots[1], 0, nullptr);
-        k_bi_scal_omega<<<1, 1, 0, s>>>(sc); CKL();
-        k_bi_update<<<nblk(n, TPB), TPB, 0, s>>>(n, c.dx.p, c.r.p, c.ph.p, c.sh.p, c.s2.p, t2, sc); CKL();
-        int nb = red_blocks(c.N);
-        k_abs5<<<nb, RED_TPB, 0, s>>>(c.N, c.r.p, c.partial.p); CKL();
-        k_linres_finalize<<<1, RED_TPB, 0, s>>>(c.partial.p, nb, sc, 0); CKL();
-        k_check<<<1, 1, 0, s>>>(sc, c.o.tolerance, c.o.rel_tol, c.o.min_iter, c.o.max_iter, 1); CKL();
+        const int* act = &sc->bi_active;
+        double *rw = c.Vb.p, *t2 = c.Vb.p + c.nvec(), *part = c.orth_part.p;
+        int N = c.N;
+        Criteria k = criteria(c);
+        precond(c, c.t.p, c.ph.p, act);                       // t holds p
+        spmv(c, c.ph.p, c.pv.p, nullptr, act);                // v = A ph
+        void* a1[] = {&N, &rw, &c.r.p, &c.pv.p, &c.s2.p, &part, &sc};
+        coop(c, (const void*)k_bi_alpha, a1);
+        precond(c, c.s2.p, c.sh.p, act);
+        spmv(c, c.sh.p, t2, nullptr, act);
+        void* a2[] = {&N, &c.dx.p, &c.r.p, &c.ph.p, &c.sh.p, &c.s2.p, &t2, &rw, &c.pv.p, &c.t.p, &part, &sc, &k};
+        coop(c, (const void*)k_bi_omega, a2);
+    }
+    static Criteria criteria(const rdst_ctx& c) {
+        return Criteria{c.o.tolerance, c.o.rel_tol, c.o.min_iter, c.o.max_iter};
+    }
+    // a BiCGStab vector kernel, all blocks resident
+    static void coop(rdst_ctx& c, const void* f, void** args) {
+        CK(cudaLaunchCooperativeKernel(f, dim3(std::min(c.orth_blocks, nblk(c.N, BI_TPB))), dim3(BI_TPB), args, 0, c.s));
+        count_launch();
     }
     // one stationary iteration dx += M^-1 (rhs - A dx) (Gauss-Seidel sweeps
     // or the Cholesky-type factorisation), then the residual check
@@ -1813,11 +1809,26 @@ void run_steps(rdst_ctx& c, int n, rdst_step_report* host_reps) {
                     CK(cudaMemcpyAsync(&conv, &c.sc.p->converged, sizeof(int), cudaMemcpyDeviceToHost, s));
                     CK(cudaStreamSynchronize(s));
                 }
+                // BiCGStab: an iteration after the converged one does nothing
+                // (bi_active), so each iteration is launched before the flag
+                // of the one before it is waited for
+                const bool ahead = o.solver == SOLVER_BICGSTAB && !o.profile;
+                if (ahead && !c.conv_host) {
+                    CK(cudaMallocHost((void**)&c.conv_host, 2 * sizeof(int)));
+                    for (auto& e : c.conv_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+                }
                 for (int it = 1; !conv && it <= o.max_iter; ++it) {
                     launch_graph(c, c.g_cycle);
                     if (o.profile) { CK(cudaStreamSynchronize(s)); c.collect_graph_events(c.g_cycle); }
                     if (it >= o.max_iter) break;
-                    if (it >= o.min_iter) {
+                    if (ahead) {
+                        CK(cudaMemcpyAsync(&c.conv_host[it & 1], &c.sc.p->converged, sizeof(int), cudaMemcpyDeviceToHost, s));
+                        CK(cudaEventRecord(c.conv_ev[it & 1], s));
+                        if (it > 1 && it - 1 >= o.min_iter) {
+                            CK(cudaEventSynchronize(c.conv_ev[(it - 1) & 1]));
+                            conv = c.conv_host[(it - 1) & 1];
+                        }
+                    } else if (it >= o.min_iter) {
                         CK(cudaMemcpyAsync(&conv, &c.sc.p->converged, sizeof(int), cudaMemcpyDeviceToHost, s));
                         CK(cudaStreamSynchronize(s));
                     }

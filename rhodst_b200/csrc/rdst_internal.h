@@ -87,9 +87,9 @@ struct Scalars {
     double H[64 * 65], bh[65], cs[64], sn[64];
     double G[64 * 64];                  // V^T V of the cycle's basis
     unsigned orth_bar, orth_out;        // grid barrier of k_orth (zero between launches)
-    double dots[2];
     // BiCGStab
-    double bi_rho, bi_rhoOld, bi_alpha, bi_omega, bi_beta, bi_tt, bi_ts, bi_rwv;
+    double bi_rho, bi_alpha;
+    int bi_active;                      // 0 after the converged iteration
 };
 
 // SELL-32 block matrix
