@@ -155,6 +155,46 @@ __global__ void k_set_cells(int n, Thermo th, const int* __restrict__ rows, cons
     if (nut) nut[r] = v[5];
 }
 
+// primitive fields in the caller's cell order -> the primitive record
+// (h = Cp T) and, with a turbulence model, nuTilda in the internal order
+__global__ void k_set_primitive(int N, double Cp, const int* __restrict__ perm, const double* __restrict__ p,
+                                const double* __restrict__ U, const double* __restrict__ T,
+                                double* __restrict__ prim) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= N) return;
+    const int i = perm[r];
+    const double t = T[i];
+    double* P = prim + (size_t)PW * r;
+    P[0] = p[i]; P[1] = t; P[2] = __dmul_rn(Cp, t);
+    P[3] = U[3L * i]; P[4] = U[3L * i + 1]; P[5] = U[3L * i + 2];
+    P[6] = 0.0; P[7] = 0.0;
+}
+__global__ void k_get_primitive(int N, const int* __restrict__ perm, const double* __restrict__ prim,
+                                double* __restrict__ p, double* __restrict__ U, double* __restrict__ T) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= N) return;
+    const int i = perm[r];
+    const double* P = prim + (size_t)PW * r;
+    p[i] = P[0];
+    T[i] = P[1];
+    U[3L * i] = P[3]; U[3L * i + 1] = P[4]; U[3L * i + 2] = P[5];
+}
+// fields of w values a cell between the caller's order and the internal one
+__global__ void k_to_internal(int N, int w, const int* __restrict__ perm, const double* __restrict__ caller,
+                              double* __restrict__ internal) {
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long)N * w) return;
+    const int r = (int)(e / w), k = (int)(e - (long)r * w);
+    internal[e] = caller[(long)perm[r] * w + k];
+}
+__global__ void k_to_caller(int N, int w, const int* __restrict__ perm, const double* __restrict__ internal,
+                            double* __restrict__ caller) {
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long)N * w) return;
+    const int r = (int)(e / w), k = (int)(e - (long)r * w);
+    caller[(long)perm[r] * w + k] = internal[e];
+}
+
 // W (internal order) -> rho, rhoU, rhoE in the caller's cell order
 __global__ void k_get_conservative(int N, const int* __restrict__ perm, const double* __restrict__ W,
                                    double* __restrict__ rho, double* __restrict__ rhoU, double* __restrict__ rhoE) {

@@ -231,7 +231,7 @@ struct rdst_ctx {
     // numbering
     std::vector<int> perm, iperm;       // perm[internal] = original
     DBuf<int> perm_d;                   // perm on the device
-    DBuf<double> stage;                 // conservative fields in the caller's order (5N)
+    DBuf<double> stage;                 // fields in the caller's order on their way in or out (6N)
     std::vector<int> bface_orig;        // active bface -> foam face
     std::vector<double> hV, hC;         // original numbering, for forces
     std::vector<int> hown, hnei;        // foam owner/neighbour lists (topology check of a new geometry)
@@ -1043,7 +1043,7 @@ void build(rdst_ctx& c, const rdst_mesh* mh) {
     m.cf_start = c.cf_start.p; m.cf_list = c.cf_list.p; m.cc_start = c.cc_start.p; m.cc_list = c.cc_list.p;
     m.patches = c.patches.p;
     // ---- fields
-    c.perm_d.upload(c.perm, s); c.stage.alloc(5L * N);
+    c.perm_d.upload(c.perm, s); c.stage.alloc(6L * N);
     c.W.alloc(5L * N); c.prim.alloc((size_t)PW * N); c.bs.alloc((size_t)BW * std::max(NB, 1));
     c.bjac.alloc((size_t)25 * std::max(NB, 1));
     c.q.alloc((size_t)QW * N); c.qb.alloc((size_t)QW * std::max(NB, 1)); c.g.alloc((size_t)GW * N);
@@ -2371,19 +2371,16 @@ void tan_product(rdst_ctx& c, const double* u, double* Ju) {
 }
 
 // internal <-> caller order for N x 5 fields
-void adj_to_internal(rdst_ctx& c, const double* host, double* dev) {
-    std::vector<double> t(5L * c.N);
-    for (int r = 0; r < c.N; ++r)
-        for (int k = 0; k < 5; ++k) t[5L * r + k] = host[5L * c.perm[r] + k];
-    CK(cudaMemcpyAsync(dev, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice, c.s));
-    CK(cudaStreamSynchronize(c.s));
+void field_to_internal(rdst_ctx& c, const double* host, double* dev) {
+    CK(cudaMemcpyAsync(c.stage.p, host, 5L * c.N * sizeof(double), cudaMemcpyHostToDevice, c.s));
+    k_to_internal<<<nblk(5L * c.N, TPB), TPB, 0, c.s>>>(c.N, 5, c.perm_d.p, c.stage.p, dev);
+    CKL();
 }
-void adj_to_caller(rdst_ctx& c, const double* dev, double* host) {
-    std::vector<double> t(5L * c.N);
-    CK(cudaMemcpyAsync(t.data(), dev, t.size() * sizeof(double), cudaMemcpyDeviceToHost, c.s));
+void field_to_caller(rdst_ctx& c, const double* dev, double* host) {
+    k_to_caller<<<nblk(5L * c.N, TPB), TPB, 0, c.s>>>(c.N, 5, c.perm_d.p, dev, c.stage.p);
+    CKL();
+    CK(cudaMemcpyAsync(host, c.stage.p, 5L * c.N * sizeof(double), cudaMemcpyDeviceToHost, c.s));
     CK(cudaStreamSynchronize(c.s));
-    for (int r = 0; r < c.N; ++r)
-        for (int k = 0; k < 5; ++k) host[5L * c.perm[r] + k] = t[5L * r + k];
 }
 
 }  // namespace
@@ -2450,17 +2447,16 @@ RDST_API rdst_status rdst_set_primitive(rdst_ctx* c, const double* p, const doub
     if (!c || !p || !U || !T) return RDST_ERR_ARG;
     if (c->turb && !nut) { c->err = "Spalart-Allmaras needs an initial nuTilda"; return RDST_ERR_ARG; }
     return guarded(c, [&] {
-        std::vector<double> prim((size_t)PW * c->N, 0.0);
-        for (int r = 0; r < c->N; ++r) {
-            int i = c->perm[r];
-            double* P = &prim[(size_t)PW * r];
-            P[0] = p[i]; P[1] = T[i]; P[2] = c->o.Cp * T[i];
-            P[3] = U[3 * i]; P[4] = U[3 * i + 1]; P[5] = U[3 * i + 2];
-        }
-        CK(cudaMemcpyAsync(c->prim.p, prim.data(), prim.size() * sizeof(double), cudaMemcpyHostToDevice, c->s));
+        const long N = c->N;
+        double *d_p = c->stage.p, *d_U = d_p + N, *d_T = d_U + 3 * N, *d_nut = d_T + N;
+        CK(cudaMemcpyAsync(d_p, p, sizeof(double) * N, cudaMemcpyHostToDevice, c->s));
+        CK(cudaMemcpyAsync(d_U, U, sizeof(double) * 3 * N, cudaMemcpyHostToDevice, c->s));
+        CK(cudaMemcpyAsync(d_T, T, sizeof(double) * N, cudaMemcpyHostToDevice, c->s));
+        if (c->turb) CK(cudaMemcpyAsync(d_nut, nut, sizeof(double) * N, cudaMemcpyHostToDevice, c->s));
+        k_set_primitive<<<nblk(N, TPB), TPB, 0, c->s>>>((int)N, c->o.Cp, c->perm_d.p, d_p, d_U, d_T, c->prim.p);
+        CKL();
         k_init_state<<<nblk(c->N, TPB), TPB, 0, c->s>>>(c->N, c->th, c->prim.p, c->W.p);
         CKL();
-        CK(cudaStreamSynchronize(c->s));
         after_state_set(*c);
         // a new state: SARC1's old-time strain rate and the dual-time levels
         // restart from the current one; deltaT0 of the first step is
@@ -2469,9 +2465,8 @@ RDST_API rdst_status rdst_set_primitive(rdst_ctx* c, const double* p, const doub
         c->dual_started = false;
         c->dt_save = c->o.delta_t;
         if (c->turb) {
-            std::vector<double> nv(c->N);
-            for (int r = 0; r < c->N; ++r) nv[r] = nut[c->perm[r]];
-            CK(cudaMemcpyAsync(c->nut.p, nv.data(), nv.size() * sizeof(double), cudaMemcpyHostToDevice, c->s));
+            k_to_internal<<<nblk(N, TPB), TPB, 0, c->s>>>((int)N, 1, c->perm_d.p, d_nut, c->nut.p);
+            CKL();
             const DevMesh& m = c->m;
             if (m.NB > 0) { k_sa_bc<<<nblk(m.NB, TPB), TPB, 0, c->s>>>(m, c->bs.p, c->sa); CKL(); }
             k_sa_init_mut<<<nblk(c->N, TPB), TPB, 0, c->s>>>(c->N, c->tr, c->W.p, c->prim.p, c->sa); CKL();
@@ -2675,18 +2670,20 @@ RDST_API rdst_status rdst_get_conservative(rdst_ctx* c, double* rho, double* rho
 RDST_API rdst_status rdst_get_primitive(rdst_ctx* c, double* p, double* U, double* T, double* nut) {
     if (!c) return RDST_ERR_ARG;
     return guarded(c, [&] {
-        std::vector<double> P((size_t)PW * c->N), nv(c->turb ? c->N : 0);
-        CK(cudaMemcpyAsync(P.data(), c->prim.p, P.size() * sizeof(double), cudaMemcpyDeviceToHost, c->s));
-        if (c->turb) CK(cudaMemcpyAsync(nv.data(), c->nut.p, nv.size() * sizeof(double), cudaMemcpyDeviceToHost, c->s));
-        CK(cudaStreamSynchronize(c->s));
-        for (int r = 0; r < c->N; ++r) {
-            int i = c->perm[r];
-            const double* q = &P[(size_t)PW * r];
-            if (p) p[i] = q[0];
-            if (T) T[i] = q[1];
-            if (U) for (int k = 0; k < 3; ++k) U[3 * i + k] = q[3 + k];
-            if (nut) nut[i] = c->turb ? nv[r] : 0.0;
+        const long N = c->N;
+        double *d_p = c->stage.p, *d_U = d_p + N, *d_T = d_U + 3 * N, *d_nut = d_T + N;
+        k_get_primitive<<<nblk(N, TPB), TPB, 0, c->s>>>((int)N, c->perm_d.p, c->prim.p, d_p, d_U, d_T);
+        CKL();
+        if (p) CK(cudaMemcpyAsync(p, d_p, sizeof(double) * N, cudaMemcpyDeviceToHost, c->s));
+        if (U) CK(cudaMemcpyAsync(U, d_U, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, c->s));
+        if (T) CK(cudaMemcpyAsync(T, d_T, sizeof(double) * N, cudaMemcpyDeviceToHost, c->s));
+        if (nut && c->turb) {
+            k_to_caller<<<nblk(N, TPB), TPB, 0, c->s>>>((int)N, 1, c->perm_d.p, c->nut.p, d_nut);
+            CKL();
+            CK(cudaMemcpyAsync(nut, d_nut, sizeof(double) * N, cudaMemcpyDeviceToHost, c->s));
         }
+        CK(cudaStreamSynchronize(c->s));
+        if (nut && !c->turb) std::fill(nut, nut + N, 0.0);
     });
 }
 
@@ -2711,11 +2708,7 @@ RDST_API rdst_status rdst_residual(rdst_ctx* c, double* out) {
             using MT = std::remove_pointer_t<decltype(tag)>;
             Ops<MT>::flux(*c);
         });
-        std::vector<double> R(5L * c->N);
-        CK(cudaMemcpyAsync(R.data(), c->R.p, R.size() * sizeof(double), cudaMemcpyDeviceToHost, c->s));
-        CK(cudaStreamSynchronize(c->s));
-        for (int r = 0; r < c->N; ++r)
-            for (int k = 0; k < 5; ++k) out[5 * c->perm[r] + k] = R[5 * r + k];
+        field_to_caller(*c, c->R.p, out);
     });
 }
 
@@ -2864,7 +2857,7 @@ RDST_API rdst_status rdst_objective_gradient(rdst_ctx* c, const rdst_objective* 
         if (J) *J = out[0];
         if (force) for (int k = 0; k < 3; ++k) force[k] = out[1 + k];
         if (dJdU) for (int k = 0; k < 3; ++k) dJdU[k] = out[4 + k];
-        if (dJdW) adj_to_caller(*c, c->a_rhs.p, dJdW);
+        if (dJdW) field_to_caller(*c, c->a_rhs.p, dJdW);
     });
 }
 
@@ -2894,9 +2887,9 @@ RDST_API rdst_status rdst_tangent_product(rdst_ctx* c, const double* u, double* 
             adj_forward<MT>(*c);
         });
         adj_alloc(*c, 0);
-        adj_to_internal(*c, u, c->a_z.p);
+        field_to_internal(*c, u, c->a_z.p);
         tan_product(*c, c->a_z.p, c->a_t.p);
-        adj_to_caller(*c, c->a_t.p, Ju);
+        field_to_caller(*c, c->a_t.p, Ju);
     });
 }
 
@@ -2908,9 +2901,9 @@ RDST_API rdst_status rdst_adjoint_product(rdst_ctx* c, const double* v, double* 
             adj_forward<MT>(*c);
         });
         adj_alloc(*c, 0);
-        adj_to_internal(*c, v, c->a_z.p);
+        field_to_internal(*c, v, c->a_z.p);
         adj_product(*c, c->a_z.p, c->a_t.p, c->a_u3.p + 8);
-        adj_to_caller(*c, c->a_t.p, u);
+        field_to_caller(*c, c->a_t.p, u);
         if (dU) {
             CK(cudaMemcpyAsync(dU, c->a_u3.p + 8, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->s));
             CK(cudaStreamSynchronize(c->s));
@@ -2945,7 +2938,7 @@ RDST_API rdst_status rdst_adjoint(rdst_ctx* c, const rdst_objective* ob, double 
         CK(cudaEventElapsedTime(&ms, e0, e1));
         c->ev_pool.push_back(e0);
         c->ev_pool.push_back(e1);
-        if (psi) adj_to_caller(*c, c->a_psi.p, psi);
+        if (psi) field_to_caller(*c, c->a_psi.p, psi);
         if (rep) {
             rep->J = out[0];
             for (int k = 0; k < 3; ++k) { rep->force[k] = out[1 + k]; rep->dJ_dU[k] = out[4 + k] - usum[k]; }
