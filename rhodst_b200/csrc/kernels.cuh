@@ -394,9 +394,25 @@ __global__ void k_recon(DevMesh m, Thermo th, Transport tr, int use_c, const dou
     }
 }
 
+// a recon record (QW doubles, 64 bytes) as four 16-byte loads
+__device__ __forceinline__ void load_q(const double* p, double (&o)[QW]) {
+    const double2* v = reinterpret_cast<const double2*>(p);
+#pragma unroll
+    for (int k = 0; k < QW / 2; ++k) { const double2 a = v[k]; o[2 * k] = a.x; o[2 * k + 1] = a.y; }
+}
+
 // Gauss linear gradient of the 7 recon fields (cell gather over the faces
 // in foam order), plus optionally the Venkatakrishnan limiter per field and
 // the HLLCP pressure-ratio sensor fCells (HLLCPDST.C:131-164).
+//
+// Bound by the gathers, so each is made once: the cell's own record stays in
+// registers, the record across a face comes in four 16-byte loads, and with
+// Venkatakrishnan (a kernel of its own, which has the registers for it) the
+// extrema of all fields are taken in that same walk over the faces and their
+// limiters in one more, where a walk per field read every neighbour fourteen
+// times.  us, before -> after: 1.2 M cells hexahedra 453 -> 342, 495 k cells
+// prisms and tetrahedra with Venkatakrishnan 407 -> 216.
+template <bool VENKAT>
 __global__ void __launch_bounds__(128) k_grad(DevMesh m, int venkat_mask, double venkat_K, const double* __restrict__ q,
                                               const double* __restrict__ qb, const double* __restrict__ prim,
                                               double* __restrict__ g, double* __restrict__ psi,
@@ -411,16 +427,23 @@ __global__ void __launch_bounds__(128) k_grad(DevMesh m, int venkat_mask, double
     double fmin_c = 1.0;
     const double pi = prim[PW * i];
     double aU[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};    // (grad U)_ij = dU_j/dx_i
+    double qi[QW];
+    load_q(q + (size_t)QW * i, qi);
+    double mx[7], mn[7];
+#pragma unroll
+    for (int j = 0; j < 7; ++j) { mx[j] = qi[j]; mn[j] = qi[j]; }
     for (int k = k0; k < k1; ++k) {
         int code = m.cf_list[k];
         if (code < m.Fi) {
             int f = code, o = m.own[f], n = m.nei[f];
+            const bool mine = o == i;
+            const int other = mine ? n : o;
             double wf = m.w[f];
             V3 S = ldv3(m.Sf, m.Fi, f);
-            const double* qo = q + QW * o;
-            const double* qn = q + QW * n;
+            double qx[QW];
+            load_q(q + (size_t)QW * other, qx);
             if (gU) {
-                const double sg = (o == i) ? 1.0 : -1.0;
+                const double sg = mine ? 1.0 : -1.0;
                 const double Sv[3] = {sg * S.x, sg * S.y, sg * S.z};
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
@@ -429,31 +452,40 @@ __global__ void __launch_bounds__(128) k_grad(DevMesh m, int venkat_mask, double
                     for (int d = 0; d < 3; ++d) aU[3 * d + j] += Sv[d] * xf;
                 }
             }
-            if (o == i) {
+            if (mine) {
 #pragma unroll
                 for (int j = 0; j < 7; ++j) {
-                    double xf = wf * qo[j] + (1 - wf) * qn[j];
+                    double xf = wf * qi[j] + (1 - wf) * qx[j];
                     acc[3 * j] += xf * S.x; acc[3 * j + 1] += xf * S.y; acc[3 * j + 2] += xf * S.z;
                 }
             } else {
 #pragma unroll
                 for (int j = 0; j < 7; ++j) {
-                    double xf = wf * qo[j] + (1 - wf) * qn[j];
+                    double xf = wf * qx[j] + (1 - wf) * qi[j];
                     acc[3 * j] -= xf * S.x; acc[3 * j + 1] -= xf * S.y; acc[3 * j + 2] -= xf * S.z;
                 }
             }
+            if (VENKAT) {
+#pragma unroll
+                for (int j = 0; j < 7; ++j) { mx[j] = fmax(mx[j], qx[j]); mn[j] = fmin(mn[j], qx[j]); }
+            }
             if (hllcp) {
-                double pk = prim[PW * (o == i ? n : o)];
+                double pk = prim[PW * other];
                 fmin_c = fmin(fmin_c, fmin(pi / pk, pk / pi));
             }
         } else {
             int b = code - m.Fi;
             V3 S = ldv3(m.bSf, m.NB, b);
-            const double* qq = qb + QW * b;
+            double qq[QW];
+            load_q(qb + (size_t)QW * b, qq);
 #pragma unroll
             for (int j = 0; j < 7; ++j) {
                 double xf = qq[j];
                 acc[3 * j] += xf * S.x; acc[3 * j + 1] += xf * S.y; acc[3 * j + 2] += xf * S.z;
+            }
+            if (VENKAT) {
+#pragma unroll
+                for (int j = 0; j < 7; ++j) { mx[j] = fmax(mx[j], qq[j]); mn[j] = fmin(mn[j], qq[j]); }
             }
             if (gU) {
                 const double Sv[3] = {S.x, S.y, S.z};
@@ -473,37 +505,31 @@ __global__ void __launch_bounds__(128) k_grad(DevMesh m, int venkat_mask, double
 #pragma unroll
     for (int k = 0; k < 21; ++k) { acc[k] /= Vi; go[k] = acc[k]; }
     if (hllcp) fcell[i] = fmin_c;
-    if (venkat_mask) {
+    if (VENKAT) {
         // Venkatakrishnan (1995): psi = min_f phi(dmax|dmin, d2), eps^2 = (K h)^3
-        const double* qi = q + QW * i;
-        double eps2 = pow(venkat_K * cbrt(Vi), 3.0);
-        V3 Ci = ldv3(m.C, m.N, i);
-        // unrolled: acc stays in registers (indexed by constants only)
+        const double eps2 = pow(venkat_K * cbrt(Vi), 3.0);
+        const V3 Ci = ldv3(m.C, m.N, i);
+        double p[7];
 #pragma unroll
-        for (int j = 0; j < 7; ++j) {
-            if (!((venkat_mask >> j) & 1)) { psi[QW * i + j] = 1.0; continue; }
-            double x = qi[j], mx = x, mn = x;
-            for (int k = k0; k < k1; ++k) {
-                int code = m.cf_list[k];
-                double xo;
-                if (code < m.Fi) { int o = m.own[code]; xo = q[QW * (o == i ? m.nei[code] : o) + j]; }
-                else xo = qb[QW * (code - m.Fi) + j];
-                mx = fmax(mx, xo); mn = fmin(mn, xo);
-            }
-            double dmax = mx - x, dmin = mn - x, p = 1.0;
-            V3 gj = mk(acc[3 * j], acc[3 * j + 1], acc[3 * j + 2]);
-            for (int k = k0; k < k1; ++k) {
-                int code = m.cf_list[k];
-                V3 Cf = code < m.Fi ? ldv3(m.Cf, m.Fi, code) : ldv3(m.bCf, m.NB, code - m.Fi);
-                double d2 = dot3(gj, sub3(Cf, Ci));
+        for (int j = 0; j < 7; ++j) { mx[j] -= qi[j]; mn[j] -= qi[j]; p[j] = 1.0; }
+        for (int k = k0; k < k1; ++k) {
+            const int code = m.cf_list[k];
+            const V3 Cf = code < m.Fi ? ldv3(m.Cf, m.Fi, code) : ldv3(m.bCf, m.NB, code - m.Fi);
+            const V3 d = sub3(Cf, Ci);
+#pragma unroll
+            for (int j = 0; j < 7; ++j) {
+                if (!((venkat_mask >> j) & 1)) continue;
+                const double dmax = mx[j], dmin = mn[j];
+                const double d2 = dot3(mk(acc[3 * j], acc[3 * j + 1], acc[3 * j + 2]), d);
                 double ph;
                 if (d2 > 0) ph = ((dmax * dmax + eps2) * d2 + 2 * d2 * d2 * dmax) / (dmax * dmax + 2 * d2 * d2 + dmax * d2 + eps2) / d2;
                 else if (d2 < 0) ph = ((dmin * dmin + eps2) * d2 + 2 * d2 * d2 * dmin) / (dmin * dmin + 2 * d2 * d2 + dmin * d2 + eps2) / d2;
                 else ph = 1.0;
-                p = fmin(p, ph);
+                p[j] = fmin(p[j], ph);
             }
-            psi[QW * i + j] = p;
         }
+#pragma unroll
+        for (int j = 0; j < 7; ++j) psi[QW * i + j] = p[j];
     }
 }
 

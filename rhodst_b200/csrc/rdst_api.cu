@@ -1224,8 +1224,9 @@ struct Ops {
         k_recon<<<nblk(m.N + m.NB, TPB), TPB, 0, s>>>(m, c.th, c.tr, use_c, c.W.p, c.prim.p, c.bs.p, c.mut.p, c.mut_b.p,
                                                      c.q.p, c.qb.p);
         CKL();
-        k_grad<<<nblk(m.N, 128), 128, 0, s>>>(m, c.venkat_mask, o.venkat_K, c.q.p, c.qb.p, c.prim.p, c.g.p, c.psi.p,
-                                             c.fcell.p, o.flux == FLUX_HLLCP, c.bs.p, visc ? c.gU.p : nullptr);
+        auto* grad = c.venkat_mask ? k_grad<true> : k_grad<false>;
+        grad<<<nblk(m.N, 128), 128, 0, s>>>(m, c.venkat_mask, o.venkat_K, c.q.p, c.qb.p, c.prim.p, c.g.p, c.psi.p,
+                                            c.fcell.p, o.flux == FLUX_HLLCP, c.bs.p, visc ? c.gU.p : nullptr);
         CKL();
         if (visc && o.grad_U_limit > 0) {
             k_limit_gradU<<<nblk(m.N, 128), 128, 0, s>>>(m, o.grad_U_limit, c.prim.p, c.bs.p, c.gU.p);
