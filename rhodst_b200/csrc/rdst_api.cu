@@ -245,7 +245,8 @@ struct rdst_ctx {
     // fields
     DBuf<double> W, prim, bs, q, qb, g, psi, fcell, fl, bfl, R, rhs, partial;
     DBuf<double> bjac;             // boundary Jacobian blocks of the active boundary faces
-    DBuf<double> rdt, courantF, rhoOld, eOld, eNew;
+    DBuf<double> rdt, courantF, rhoOld, eOld;
+    DBuf<unsigned char> drop;      // cells whose density or energy fell (CFL cut)
     // viscous: grad U, face Up, viscous face terms, turbulent viscosity
     DBuf<double> gU, up, bup, vf, bvf, mut, mut_b;
     Transport tr{};
@@ -286,7 +287,7 @@ struct rdst_ctx {
     DBuf<int4> fr_desc;
     bool ilu_direct = false;
     // Krylov
-    DBuf<double> dx, r, t, Vb, s2, sh, ph, pv, xbar, Ax, pA;
+    DBuf<double> dx, r, t, Vb, s2, sh, ph, pv, xbar;
     DBuf<double> gs_r, gs_z;        // residual and correction of Gauss-Seidel sweeps after the first
     // block AMG: coarse levels 1.. (level 0 is the step's matrix)
     struct AmgDev {
@@ -1069,7 +1070,7 @@ void build(rdst_ctx& c, const rdst_mesh* mh) {
         c.gU.alloc(9L * N); c.up.alloc(3L * std::max(Fi, 1)); c.bup.alloc(3L * std::max(NB, 1));
         c.vf.alloc(8L * std::max(Fi, 1)); c.bvf.alloc(8L * std::max(NB, 1));
     }
-    c.rdt.alloc(N); c.courantF.alloc(N); c.rhoOld.alloc(N); c.eOld.alloc(N); c.eNew.alloc(N);
+    c.rdt.alloc(N); c.courantF.alloc(N); c.rhoOld.alloc(N); c.eOld.alloc(N); c.drop.alloc(N);
     c.sc.alloc(1); c.sc.zero(s);
     c.reps.alloc(rdst_ctx::REP_CAP);
     int nbmax = std::max(nblk(std::max(N, Fi), TPB), red_blocks(5L * N));
@@ -1094,7 +1095,7 @@ void build(rdst_ctx& c, const rdst_mesh* mh) {
     if (o.precon == PRECON_GAUSS_SEIDEL && o.n_sweeps > 1) { c.gs_r.alloc(5L * N); c.gs_z.alloc(5L * N); }
     // ---- Krylov
     const long n5 = 5L * N;
-    c.r.alloc(n5); c.t.alloc(n5); c.Ax.alloc(n5); c.pA.alloc(n5); c.xbar.alloc(8);
+    c.r.alloc(n5); c.t.alloc(n5); c.xbar.alloc(8);
     // basis vectors 64-entry aligned (the orthogonalisation reads 4 entries per 16-byte load)
     c.ldv = (n5 + 63) / 64 * 64;
     // (with zeros past the end, which the orthogonalisation reads along)
@@ -1430,18 +1431,17 @@ struct Ops {
         const int N = c.N;
         int nb = red_blocks(N);
         if (c.o.dependent_W) {
-            spmv(c, c.W.p, c.Ax.p, nullptr, nullptr);
             k_sum5<<<nb, RED_TPB, 0, s>>>(N, c.W.p, c.partial.p); CKL();
             k_mean5_finalize<<<1, RED_TPB, 0, s>>>(c.partial.p, nb, N, c.xbar.p); CKL();
-            k_spmv_const<MT><<<nblk(N, 256), 256, 0, s>>>(c.mat<MT>(c.Aval), c.xbar.p, c.pA.p); CKL();
         }
-        k_normfactor<<<nb, RED_TPB, 0, s>>>(N, c.Ax.p, c.rhs.p, c.pA.p, c.o.dependent_W ? 1 : 0, c.partial.p); CKL();
-        k_nf_finalize<<<1, RED_TPB, 0, s>>>(c.partial.p, nb, c.sc.p); CKL();
-        k_abs5<<<nb, RED_TPB, 0, s>>>(N, c.rhs.p, c.partial.p); CKL();
-        k_linres_finalize<<<1, RED_TPB, 0, s>>>(c.partial.p, nb, c.sc.p, 1); CKL();
+        const int nbi = std::min(nblk(N, 256), 8 * c.sms);
+        {
+            Timed tm(c, KS_SPMV);       // the product A W
+            k_solve_init<MT><<<nbi, 256, 0, s>>>(c.mat<MT>(c.Aval), c.o.dependent_W ? 1 : 0, c.W.p, c.xbar.p, c.rhs.p,
+                                                 c.partial.p); CKL();
+        }
+        k_solve_start<<<1, RED_TPB, 0, s>>>(c.partial.p, nbi, c.sc.p, criteria(c)); CKL();
         CK(cudaMemsetAsync(c.dx.p, 0, sizeof(double) * c.nvec(), s));
-        CK(cudaMemsetAsync(&c.sc.p->lin_iterations, 0, sizeof(int), s));
-        k_check<<<1, 1, 0, s>>>(c.sc.p, criteria(c), 0); CKL();
         if (c.o.solver == SOLVER_BICGSTAB) {
             Scalars* sc = c.sc.p;
             double *rw = c.Vb.p, *part = c.orth_part.p;
@@ -1510,7 +1510,7 @@ struct Ops {
         spmv(c, c.dx.p, c.r.p, c.rhs.p, nullptr);
         int nb = red_blocks(c.N);
         k_abs5<<<nb, RED_TPB, 0, c.s>>>(c.N, c.r.p, c.partial.p); CKL();
-        k_linres_finalize<<<1, RED_TPB, 0, c.s>>>(c.partial.p, nb, c.sc.p, 0); CKL();
+        k_linres_finalize<<<1, RED_TPB, 0, c.s>>>(c.partial.p, nb, c.sc.p); CKL();
         k_check<<<1, 1, 0, c.s>>>(c.sc.p, criteria(c), 1); CKL();
     }
     // one BiCGStab iteration (van der Vorst, right preconditioned)
@@ -1652,9 +1652,8 @@ void post_update(rdst_ctx& c) {
     if (c.turb && !c.o.frozen_turbulence) sa_correct(c);   // turbulence_.correct(); frozen: mu_t held
     k_courant_scalar<<<1, 1, 0, s>>>(c.sc.p, (!c.steady && c.o.adjust_time_step) ? 1 : 0, c.o.min_co, c.o.max_co); CKL();
     if (c.steady) {
-        k_courant_cells<<<nblk(c.N, TPB), TPB, 0, s>>>(c.m, c.W.p, c.rhoOld.p, c.eOld.p, c.courantF.p, c.sc.p,
-                                                      c.o.min_co, c.o.max_co, c.eNew.p); CKL();
-        k_store_old<<<nblk(c.N, TPB), TPB, 0, s>>>(c.N, c.W.p, c.eNew.p, c.rhoOld.p, c.eOld.p); CKL();
+        k_courant_drop<<<nblk(c.N, TPB), TPB, 0, s>>>(c.N, c.W.p, c.rhoOld.p, c.eOld.p, c.drop.p); CKL();
+        k_courant_cells<<<nblk(c.N, TPB), TPB, 0, s>>>(c.m, c.drop.p, c.courantF.p, c.sc.p, c.o.min_co, c.o.max_co); CKL();
         set_steady_dt(c);
     } else if (c.o.adjust_time_step) {
         set_transient_dt(c);
@@ -1989,10 +1988,9 @@ void run_dual_steps(rdst_ctx& c, int n, rdst_step_report* host_reps) {
                                                    o.min_co, o.max_co);
                 CKL();
                 if (pseudo) {
-                    k_courant_cells<<<nblk(c.N, TPB), TPB, 0, s>>>(c.m, c.W.p, c.rhoOld.p, c.eOld.p, c.courantF.p,
-                                                                  c.sc.p, o.min_co, o.max_co, c.eNew.p);
+                    k_courant_drop<<<nblk(c.N, TPB), TPB, 0, s>>>(c.N, c.W.p, c.rhoOld.p, c.eOld.p, c.drop.p); CKL();
+                    k_courant_cells<<<nblk(c.N, TPB), TPB, 0, s>>>(c.m, c.drop.p, c.courantF.p, c.sc.p, o.min_co, o.max_co);
                     CKL();
-                    k_store_old<<<nblk(c.N, TPB), TPB, 0, s>>>(c.N, c.W.p, c.eNew.p, c.rhoOld.p, c.eOld.p); CKL();
                     set_steady_dt(c);
                 } else if (o.adjust_time_step) {
                     set_transient_dt(c);
