@@ -171,12 +171,14 @@ def algorithmic_bytes(kind: str, N: int, F: int, S: int, precon: str, vb: int = 
     if kind == "factor":
         return 2 * (25 * S * Bk + 4 * Bk) + 25 * S * N
     if kind == "orth":
-        # one GMRES direction of CGS2 at the mean basis size J = (m+1)/2:
-        # three passes over the J basis vectors (dots; axpy fused with the
-        # second dots; axpy fused with the norm) and five passes over w
-        # (read; read+write; read+write), w in fp64
-        J = (m + 1) / 2.0
-        return N * (3 * J * 5 * vb + 5 * 40)
+        # one launch of the orthogonalisation at the mean basis size J (the
+        # cycle's start and m directions): two passes over the J basis
+        # vectors with an fp64 basis, three with an fp32 one, and over w (fp64)
+        # a read for the dots, a read and a write per update, and the scaled
+        # copy into the basis
+        J = m / 2.0
+        passes, updates = (2, 1) if vb == 8 else (3, 2)
+        return N * 5 * (passes * J * vb + 8 + 16 * updates + 8 + vb)
     return 0.0
 
 
