@@ -700,12 +700,14 @@ __global__ void __launch_bounds__(32) k_ilu_factor_direct(SellMat<MT> A, MT* __r
 // when they are needed (EXT).
 //
 // TIGHT: three compute warps (two with FP64) and the registers of six CTAs an
-// SM.  Every
-// mbarrier wait is bounded (2 s of globaltimer): on expiry the warp raises
-// bit 2 of *flags (reported as a timeout by the host), takes part in the
-// sweep's remaining level barriers, so that no other warp stays in one, and
-// ends; they find their own waits expired in turn, and the producer waits,
-// again bounded, for its copies in flight.
+// SM.
+//
+// Every mbarrier wait is bounded (2 s of globaltimer).  A compute warp whose
+// wait expires raises bit 2 of *flags (reported as a timeout by the host) and
+// computes no more, but takes all that is left of the level barriers of both
+// sweeps (rec_give_up): bar.sync has no bound of its own, so no barrier may
+// miss a warp.  The others find their own waits expired in turn, and the
+// producer waits, again bounded, for its copies in flight.
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -1135,6 +1137,30 @@ __global__ void __launch_bounds__(TIGHT ? 96 : 256, TIGHT ? 6 : 2)
     while (arrived < nlev - 1) arrive();
 }
 
+// The level barriers of the W compute warps.  An SM has 64 barriers and a kernel
+// that names one in a register reserves all 16, which would leave four CTAs an
+// SM: the tight instance names its four.
+template <bool TIGHT>
+__device__ __forceinline__ void level_arrive(int id, int W) {
+    if (!TIGHT) asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(W * 32) : "memory");
+    else if (id == 1) asm volatile("bar.arrive 1, %0;" ::"r"(W * 32) : "memory");
+    else if (id == 2) asm volatile("bar.arrive 2, %0;" ::"r"(W * 32) : "memory");
+    else if (id == 3) asm volatile("bar.arrive 3, %0;" ::"r"(W * 32) : "memory");
+    else asm volatile("bar.arrive 4, %0;" ::"r"(W * 32) : "memory");
+}
+template <bool TIGHT>
+__device__ __forceinline__ void level_sync(int id, int W) {
+    if (!TIGHT) asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(W * 32) : "memory");
+    else if (id == 1) asm volatile("bar.sync 1, %0;" ::"r"(W * 32) : "memory");
+    else if (id == 2) asm volatile("bar.sync 2, %0;" ::"r"(W * 32) : "memory");
+    else if (id == 3) asm volatile("bar.sync 3, %0;" ::"r"(W * 32) : "memory");
+    else asm volatile("bar.sync 4, %0;" ::"r"(W * 32) : "memory");
+}
+template <bool TIGHT>
+__device__ __forceinline__ void level_give_up(RecBarriers<TIGHT> bar, int nlev, bool back, int W) {
+    rec_give_up(bar, nlev, back, [&] { level_sync<TIGHT>(bar.id, W); bar.next(); });
+}
+
 template <typename MT, int NB, bool EXT, bool TIGHT>
 __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TIGHT ? 6 : 2)
     k_ilu_apply_rec(IluDev P, const double* __restrict__ b, double* x, const int* __restrict__ active,
@@ -1230,10 +1256,6 @@ __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TI
 
     // ---------------- compute warps
     constexpr unsigned LRB = lb_row_bytes<CT>();
-    // ids of the level barriers: more than the W levels a warp can be ahead of
-    // the slowest.  An SM has 64 barriers and a kernel that names one in a
-    // register reserves all 16, which would leave four CTAs an SM.
-    constexpr int NBAR = TIGHT ? 4 : 15;
     const int rsub = lane / 5, comp = lane - 5 * rsub;
     const int pos0 = lane < 30 ? rsub : 0x7fffffff;       // position in the task
     const int sbase = lane < 30 ? 5 * rsub : 0;
@@ -1246,42 +1268,20 @@ __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TI
     __syncwarp();
     int s = 0;                  // stage of the group the warp is in
     unsigned ph = 0;
-    auto sweep = [&](auto back_tag) -> bool {
+    auto sweep = [&](auto back_tag, RecBarriers<TIGHT>& bar) -> bool {
         constexpr bool BACK = decltype(back_tag)::value;
         const int ngrp = BACK ? ngb : ngf;
-        int grp = 0, arrived = 0, bid = 1;      // group in the sweep; level barriers arrived on, the next one's id
+        int grp = 0;                            // group in the sweep
         unsigned gn = 0;                        // the group's address
         bool held = false;                      // the group is not returned yet
-        auto arrive = [&] {                     // end of a level on which nobody here waits
-            if (TIGHT) {
-                if (bid == 1) asm volatile("bar.arrive 1, %0;" ::"r"(W * 32) : "memory");
-                else if (bid == 2) asm volatile("bar.arrive 2, %0;" ::"r"(W * 32) : "memory");
-                else if (bid == 3) asm volatile("bar.arrive 3, %0;" ::"r"(W * 32) : "memory");
-                else asm volatile("bar.arrive 4, %0;" ::"r"(W * 32) : "memory");
-            } else {
-                asm volatile("bar.arrive %0, %1;" ::"r"(bid), "r"(W * 32) : "memory");
-            }
-            bid = bid == NBAR ? 1 : bid + 1;
-            ++arrived;
-        };
-        auto await = [&] {                      // end of the level before the next task's
-            if (TIGHT) {
-                if (bid == 1) asm volatile("bar.sync 1, %0;" ::"r"(W * 32) : "memory");
-                else if (bid == 2) asm volatile("bar.sync 2, %0;" ::"r"(W * 32) : "memory");
-                else if (bid == 3) asm volatile("bar.sync 3, %0;" ::"r"(W * 32) : "memory");
-                else asm volatile("bar.sync 4, %0;" ::"r"(W * 32) : "memory");
-            } else {
-                asm volatile("bar.sync %0, %1;" ::"r"(bid), "r"(W * 32) : "memory");
-            }
-            bid = bid == NBAR ? 1 : bid + 1;
-            ++arrived;
-        };
+        // end of a level on which nobody here waits, of the one before the next task's
+        auto arrive = [&] { level_arrive<TIGHT>(bar.id, W); bar.next(); };
+        auto await = [&] { level_sync<TIGHT>(bar.id, W); bar.next(); };
         auto enter = [&] {                      // the group in stage s has landed
             gn = dyn + (unsigned)(s * stage_bytes);
             held = true;
             if (__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, ph))) return true;
             if (lane == 0) atomicOr(flags, 4);
-            while (arrived < nlev - 1) await();      // in step with the others, who may still run
             return false;
         };
         auto release = [&] {
@@ -1354,8 +1354,8 @@ __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TI
                 if (!next_group()) return false;
             }
             const int level = load(first);
-            while (arrived < level - 1) arrive();
-            if (arrived < level) await();
+            while (bar.taken < level - 1) arrive();
+            if (bar.taken < level) await();
             for (;;) {
                 // ---- the chain: x of the level before, products, hand on
                 CT part_k[NB];
@@ -1407,7 +1407,7 @@ __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TI
                 if (dl > 0) await();
             }
         }
-        while (arrived < nlev - 1) arrive();
+        while (bar.taken < nlev - 1) arrive();
         if (!BACK) {
             __syncwarp();
             if (lane == 0) mbar_arrive(fdone);
@@ -1419,8 +1419,11 @@ __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TI
         if (++s == REC_STAGES) { s = 0; ph ^= 1u; }
         return true;
     };
-    if (!sweep(std::false_type{})) return;
-    sweep(std::true_type{});
+    // a warp that gave up stays in step with the others, who may still run
+    RecBarriers<TIGHT> forward(nlev, false);
+    if (!sweep(std::false_type{}, forward)) { level_give_up(forward, nlev, false, W); return; }
+    RecBarriers<TIGHT> backward(nlev, true);
+    if (!sweep(std::true_type{}, backward)) level_give_up(backward, nlev, true, W);
 }
 
 // ---------------------------------------------------------------- vectors

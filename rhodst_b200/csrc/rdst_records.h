@@ -46,6 +46,12 @@
 #include <thread>
 #include <vector>
 
+#ifdef __CUDACC__
+#define RDST_HD __host__ __device__ __forceinline__
+#else
+#define RDST_HD inline
+#endif
+
 namespace rdst {
 
 constexpr int REC_ROWS = 6;             // rows of a task
@@ -60,6 +66,32 @@ constexpr int REC_STAGES = 2;
 constexpr size_t REC_STAGE_CAP = 65536, REC_RAMP0 = 8192, REC_RAMP1 = 20480;
 constexpr int REC_WARP_LAST = 1;        // the warp's last task of the sweep
 constexpr int REC_FAR = 2;              // some column lies in the global vector
+
+// The level barriers of a sweep: nlev - 1, taken by every compute warp in the
+// same order, waiting on it or not, and also by a warp that has given up, since
+// the others may be waiting in one.  A warp goes past at most W - 1 of them
+// without waiting (its next task is at most W levels on), so with more than W
+// ids in turn none is used again before its last use is complete.  For that to
+// hold at the turn too, where a warp that gave up does not wait for the others'
+// forward sweep, the backward sweep goes on with the id after the forward one's.
+template <bool TIGHT> struct RecBarriers {
+    static constexpr int ids = TIGHT ? 4 : 15;
+    int id, taken = 0;      // the next barrier's; of this sweep
+    RDST_HD RecBarriers(int nlev, bool back) : id(back ? 1 + (nlev - 1) % ids : 1) {}
+    RDST_HD void next() { id = id == ids ? 1 : id + 1; ++taken; }
+};
+
+// What a warp still has to take once its wait for a group has expired: the rest
+// of this sweep's barriers and, from the forward sweep, the backward one's.  The
+// others go on into that sweep and give up there (this warp's arrivals are
+// missing) or compute on; either way they take all of its barriers.
+template <typename Bar, typename Await>
+RDST_HD void rec_give_up(Bar& bar, int nlev, bool back, Await&& await) {
+    while (bar.taken < nlev - 1) await();
+    if (back) return;
+    bar.taken = 0;
+    while (bar.taken < nlev - 1) await();
+}
 
 struct RecGroup { uint32_t off16; uint32_t bytes; int32_t row0; int32_t nrows; };
 struct RecTask { uint32_t head16; uint32_t group16; };   // a task's header and its group, from the records' start / 16
