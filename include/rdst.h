@@ -333,6 +333,14 @@ double rdst_last_step_ms(const rdst_ctx* ctx);
 rdst_status rdst_kernel_stats(rdst_ctx* ctx, const char* kernel, int64_t* launches, double* total_ms);
 rdst_status rdst_set_profile(rdst_ctx* ctx, int32_t on);
 
+/* Limit of the solver kernels' device waits (no reference counterpart), 0 to
+ * 3600 s, 2 s in a new context; 0: every such wait gives up at once.  When one
+ * runs out rdst_step and rdst_adjoint return RDST_ERR_TIMEOUT.  The fields and
+ * the time control that a step leaves then are not to be used, and the calls go
+ * on to report it until rdst_set_primitive starts anew.  An adjoint call leaves
+ * the state as it was. */
+rdst_status rdst_set_wait_limit(rdst_ctx* ctx, double seconds);
+
 /* Allocation-free residual norms (no counterpart in the reference; an
  * addition for callers that may not allocate device memory: code running
  * during CUDA stream capture, where cudaMalloc is not capturable, hosts

@@ -134,6 +134,7 @@ def declare(lib: ctypes.CDLL, prefix: str) -> None:
         f("last_step_ms", c_double, [vp])
         f("kernel_stats", c_int32, [vp, c_char_p, POINTER(ctypes.c_int64), POINTER(c_double)])
         f("set_profile", c_int32, [vp, c_int32])
+        f("set_wait_limit", c_int32, [vp, c_double])
         f("get_cells_device", c_int32, [vp, c_int32, POINTER(c_int32), c_void_p])
         f("set_cells_device", c_int32, [vp, c_int32, POINTER(c_int32), c_void_p])
     if hasattr(lib, prefix + "adjoint"):
@@ -350,6 +351,9 @@ class Solver:
 
     def set_profile(self, on: bool) -> None:
         self._check(self._fn("set_profile")(self._h, 1 if on else 0), "set_profile")
+
+    def set_wait_limit(self, seconds: float) -> None:
+        self._check(self._fn("set_wait_limit")(self._h, seconds), "set_wait_limit")
 
     def kernel_stats(self, kernel: str):
         n = ctypes.c_int64()

@@ -702,12 +702,12 @@ __global__ void __launch_bounds__(32) k_ilu_factor_direct(SellMat<MT> A, MT* __r
 // TIGHT: three compute warps (two with FP64) and the registers of six CTAs an
 // SM.
 //
-// Every mbarrier wait is bounded (2 s of globaltimer).  A compute warp whose
-// wait expires raises bit 2 of *flags (reported as a timeout by the host) and
+// Every mbarrier wait is bounded (wait_ms of globaltimer).  A compute warp whose
+// wait expires raises bit 2 of the flags (reported as a timeout by the host) and
 // computes no more, but takes all that is left of the level barriers of both
 // sweeps (rec_give_up): bar.sync has no bound of its own, so no barrier may
 // miss a warp.  The others find their own waits expired in turn, and the
-// producer waits, again bounded, for its copies in flight.
+// producer waits, bounded by 2 s, for its copies in flight.
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -733,17 +733,33 @@ __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// true once the phase of parity `parity` has completed; false after 2 s
-__device__ __noinline__ bool mbar_wait_slow(unsigned bar, unsigned parity) {
+// true once the phase of parity `parity` has completed; false after wait_ms
+// (0: at once)
+__device__ __noinline__ bool mbar_wait_for(unsigned bar, unsigned parity, unsigned wait_ms) {
     const unsigned long long t0 = globaltimer_ns();
-    for (;;) {
+    while (wait_ms) {
         for (int it = 0; it < 64; ++it)
             if (mbar_try(bar, parity)) return true;
-        if (globaltimer_ns() - t0 > 2000000000ull) return false;
+        if (globaltimer_ns() - t0 > wait_ms * 1000000ull) break;
     }
+    return false;
+}
+// the CTA's limit: kept here, since an argument more of the call below would
+// cost the compute warps a register that the tight instances do not have
+__shared__ unsigned s_wait_ms;
+__device__ __noinline__ bool mbar_wait_slow(unsigned bar, unsigned parity) {
+    return mbar_wait_for(bar, parity, s_wait_ms);
 }
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
     return mbar_try(bar, parity) || mbar_wait_slow(bar, parity);
+}
+// A bounded wait of a solver kernel has expired: bit 2 of the flags, which the
+// host reports, and nothing left to do for the rest of the solve (the launches
+// that follow would wait out the limit in turn, or go on with half sums).
+__device__ __forceinline__ void wait_expired(Scalars* sc) {
+    atomicOr(&sc->flags, 4);
+    sc->gm_active = sc->gm_used = sc->bi_active = 0;
+    sc->converged = 1;
 }
 __device__ __forceinline__ void cpa8(unsigned dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
@@ -1157,14 +1173,15 @@ __device__ __forceinline__ void level_sync(int id, int W) {
     else asm volatile("bar.sync 4, %0;" ::"r"(W * 32) : "memory");
 }
 template <bool TIGHT>
-__device__ __forceinline__ void level_give_up(RecBarriers<TIGHT> bar, int nlev, bool back, int W) {
+__device__ __forceinline__ void level_give_up(RecBarriers<TIGHT> bar, int nlev, bool back, int W, Scalars* sc) {
+    if ((threadIdx.x & 31) == 0) wait_expired(sc);
     rec_give_up(bar, nlev, back, [&] { level_sync<TIGHT>(bar.id, W); bar.next(); });
 }
 
 template <typename MT, int NB, bool EXT, bool TIGHT>
 __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TIGHT ? 6 : 2)
     k_ilu_apply_rec(IluDev P, const double* __restrict__ b, double* x, const int* __restrict__ active,
-                    int stage_bytes, int y0_rows, int lb_rows, int* flags) {
+                    int stage_bytes, int y0_rows, int lb_rows, Scalars* sc, unsigned wait_ms) {
     using CT = typename IluCT<MT>::T;
     if (active && !*active) return;
     __shared__ __align__(8) unsigned long long s_bar[2 * REC_STAGES + 1];     // full, empty, forward done
@@ -1182,6 +1199,7 @@ __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TI
             mbar_init(empty0 + 8 * k, W);
         }
         mbar_init(fdone, W);
+        s_wait_ms = wait_ms;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -1194,7 +1212,7 @@ __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TI
         int s = 0;
         unsigned ph = 0;                           // parity of the next fill of stage s
         unsigned used = 0, lastp = 0;              // stages that took a copy, parity of the last one
-        bool ok = true;
+        bool ok = wait_ms != 0;                    // 0: no wait is granted
         auto record = [&](const RecGroup& g, const unsigned char* rec) {
             ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1u));
             if (!ok) return;
@@ -1247,9 +1265,9 @@ __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TI
         }
         // abandoned: copies still in flight land before the CTA's shared memory goes
         if (!ok && lane == 0) {
-            atomicOr(flags, 4);
+            wait_expired(sc);
             for (int d = 0; d < REC_STAGES; ++d)
-                if ((used >> d) & 1u) mbar_wait(full0 + 8 * d, (lastp >> d) & 1u);
+                if ((used >> d) & 1u) mbar_wait_for(full0 + 8 * d, (lastp >> d) & 1u, 2000);
         }
         return;
     }
@@ -1280,9 +1298,7 @@ __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TI
         auto enter = [&] {                      // the group in stage s has landed
             gn = dyn + (unsigned)(s * stage_bytes);
             held = true;
-            if (__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, ph))) return true;
-            if (lane == 0) atomicOr(flags, 4);
-            return false;
+            return __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, ph)) != 0;
         };
         auto release = [&] {
             __syncwarp();
@@ -1421,9 +1437,9 @@ __global__ void __launch_bounds__(TIGHT ? (sizeof(MT) == 8 ? 96 : 128) : 288, TI
     };
     // a warp that gave up stays in step with the others, who may still run
     RecBarriers<TIGHT> forward(nlev, false);
-    if (!sweep(std::false_type{}, forward)) { level_give_up(forward, nlev, false, W); return; }
+    if (!sweep(std::false_type{}, forward)) { level_give_up(forward, nlev, false, W, sc); return; }
     RecBarriers<TIGHT> backward(nlev, true);
-    if (!sweep(std::true_type{}, backward)) level_give_up(backward, nlev, true, W);
+    if (!sweep(std::true_type{}, backward)) level_give_up(backward, nlev, true, W, sc);
 }
 
 // ---------------------------------------------------------------- vectors
@@ -1509,7 +1525,8 @@ __device__ __forceinline__ void solver_check(Scalars* sc, const Criteria& k, int
         if (!(sc->lin_final[c] < tol)) t = false;
         if (!(sc->lin_final[c] < relTol * sc->lin_initial[c])) r = false;
     }
-    sc->converged = (it >= minIter) && (t || r || it >= maxIter);
+    // (or a wait has expired: no iteration will change anything)
+    sc->converged = ((it >= minIter) && (t || r || it >= maxIter)) || (sc->flags & 4);
     if (sc->converged) sc->flags = (t || r) ? (sc->flags & ~8) : (sc->flags | 8);
 }
 __global__ void k_check(Scalars* sc, Criteria k, int count) {
@@ -1595,8 +1612,13 @@ __device__ __forceinline__ double warp_sum16(double (&a)[16]) {
     return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
 }
 
-// all blocks of a cooperative launch; false after 2 s (bit 2 of *flags)
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, int* flags) {
+// All blocks of a cooperative launch, the round-th time in it (from 1); false
+// after wait_ms (0: at once).  A launch that gave up leaves the counter as it is,
+// so the solver kernels do nothing more (wait_expired) until the host has cleared
+// it (k_clear_expired, k_init_scalars).
+__device__ __forceinline__ bool grid_barrier(Scalars* sc, unsigned round, unsigned wait_ms) {
+    unsigned* bar = &sc->orth_bar;
+    const unsigned target = round * gridDim.x;
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1604,15 +1626,16 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, int
         unsigned v;
         unsigned long long t0 = 0;
         int ok = 0;
-        for (unsigned it = 0;; ++it) {
+        for (unsigned it = 0; wait_ms; ++it) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
             if (v >= target) { ok = 1; break; }
             if ((it & 255u) == 255u) {
                 const unsigned long long now = globaltimer_ns();
                 if (t0 == 0) t0 = now;
-                else if (now - t0 > 2000000000ull) { atomicOr(flags, 4); break; }
+                else if (now - t0 > wait_ms * 1000000ull) break;
             }
         }
+        if (!ok) wait_expired(sc);
         s_ok = ok;
     }
     __syncthreads();
@@ -1733,8 +1756,9 @@ __device__ __forceinline__ void grid_leave(Scalars* sc) {
 // (FP64 basis).  partial: ORTH_COLS columns of gridDim.x doubles.
 template <typename VT>
 __global__ void __launch_bounds__(ORTH_TPB, 1)
-    k_orth(long n, int nv, const VT* V, long ldv, double* w, VT* vout, double* partial, Scalars* sc, int m) {
-    if (nv > 0 && !sc->gm_active) return;
+    k_orth(long n, int nv, const VT* V, long ldv, double* w, VT* vout, double* partial, Scalars* sc, int m,
+           unsigned wait_ms) {
+    if (nv > 0 ? !sc->gm_active : (sc->flags & 4) != 0) return;
     constexpr int NW = ORTH_TPB / 32;
     __shared__ double s_red[NW][17];
     __shared__ double s_col[2 * ORTH_MAXV + 1], s_c[ORTH_MAXV], s_b[2];
@@ -1746,7 +1770,7 @@ __global__ void __launch_bounds__(ORTH_TPB, 1)
     const int i = nv - 1;
     for (int q = tid; q < i * i; q += ORTH_TPB) s_G[(q / i) * nv + q % i] = sc->G[(q / i) * ORTH_MAXV + q % i];
     unsigned round = 0;
-    auto barrier = [&] { return grid_barrier(&sc->orth_bar, ++round * (unsigned)nb, &sc->flags); };
+    auto barrier = [&] { return grid_barrier(sc, ++round, wait_ms); };
     // sum of x over the block into column col
     auto block_col = [&](double x, int col) {
         x = warp_sum(x);
@@ -1929,8 +1953,9 @@ __device__ __forceinline__ double sum_as_block(const double* part, int nb) {
 
 template <typename VT>
 __global__ void __launch_bounds__(CGS_TPB, 1)
-    k_orth_cgs2(long n, int nv, const VT* V, long ldv, double* w, VT* vout, double* partial, Scalars* sc, int m, int nbv) {
-    if (nv > 0 && !sc->gm_active) return;
+    k_orth_cgs2(long n, int nv, const VT* V, long ldv, double* w, VT* vout, double* partial, Scalars* sc, int m, int nbv,
+                unsigned wait_ms) {
+    if (nv > 0 ? !sc->gm_active : (sc->flags & 4) != 0) return;
     constexpr int NWB = RED_TPB / 32;               // warps of a virtual block
     __shared__ double s_red[CGS_TPB / 32][CGS_NV];
     __shared__ double s_h[2][ORTH_MAXV], s_rot[2][ORTH_MAXV], s_b;
@@ -1938,7 +1963,7 @@ __global__ void __launch_bounds__(CGS_TPB, 1)
     const int i = nv - 1;
     const long nc = (n + 3) / 4, stride = (long)nbv * RED_TPB;
     unsigned round = 0;
-    auto barrier = [&] { return grid_barrier(&sc->orth_bar, ++round * gridDim.x, &sc->flags); };
+    auto barrier = [&] { return grid_barrier(sc, ++round, wait_ms); };
     // every virtual block of this CTA, two at a time (f is called by all
     // threads, with a block past the end for a CTA's odd last one)
     auto blocks = [&](auto f) {
@@ -2186,7 +2211,9 @@ __device__ __forceinline__ void bi_columns(double (&x)[K], double* partial, int 
 // r = rw = p = rhs, v = 0, rho = rw . r
 __global__ void __launch_bounds__(BI_TPB) k_bi_start(int N, const double* __restrict__ rhs, double* __restrict__ r,
                                                      double* __restrict__ rw, double* __restrict__ p,
-                                                     double* __restrict__ v, double* partial, Scalars* sc) {
+                                                     double* __restrict__ v, double* partial, Scalars* sc,
+                                                     unsigned wait_ms) {
+    if (sc->flags & 4) return;
     __shared__ double s_sum[1];
     double d[1] = {0.0};
     for (long i = (long)blockIdx.x * BI_TPB + threadIdx.x; i < N; i += (long)gridDim.x * BI_TPB)
@@ -2200,7 +2227,7 @@ __global__ void __launch_bounds__(BI_TPB) k_bi_start(int N, const double* __rest
             d[0] += a * a;
         }
     bi_columns(d, partial, 0);
-    if (!grid_barrier(&sc->orth_bar, gridDim.x, &sc->flags)) return;
+    if (!grid_barrier(sc, 1, wait_ms)) return;
     if (blockIdx.x == 0) {
         sum_columns<BI_TPB>(partial, 1, gridDim.x, s_sum);
         if (threadIdx.x == 0) {
@@ -2214,7 +2241,7 @@ __global__ void __launch_bounds__(BI_TPB) k_bi_start(int N, const double* __rest
 // alpha = rho / (rw . v); s = r - alpha v
 __global__ void __launch_bounds__(BI_TPB) k_bi_alpha(int N, const double* __restrict__ rw, const double* __restrict__ r,
                                                      const double* __restrict__ v, double* __restrict__ s,
-                                                     double* partial, Scalars* sc) {
+                                                     double* partial, Scalars* sc, unsigned wait_ms) {
     if (!sc->bi_active) return;
     __shared__ double s_sum[1];
     const double rho = sc->bi_rho;
@@ -2223,7 +2250,7 @@ __global__ void __launch_bounds__(BI_TPB) k_bi_alpha(int N, const double* __rest
 #pragma unroll
         for (int c = 0; c < 5; ++c) d[0] += rw[5 * i + c] * v[5 * i + c];
     bi_columns(d, partial, 0);
-    if (!grid_barrier(&sc->orth_bar, gridDim.x, &sc->flags)) return;
+    if (!grid_barrier(sc, 1, wait_ms)) return;
     sum_columns<BI_TPB>(partial, 1, gridDim.x, s_sum);
     const double alpha = rho / s_sum[0];
     for (long i = (long)blockIdx.x * BI_TPB + threadIdx.x; i < N; i += (long)gridDim.x * BI_TPB)
@@ -2239,7 +2266,8 @@ __global__ void __launch_bounds__(BI_TPB) k_bi_omega(int N, double* __restrict__
                                                      const double* __restrict__ ph, const double* __restrict__ sh,
                                                      const double* __restrict__ s, const double* __restrict__ t,
                                                      const double* __restrict__ rw, const double* __restrict__ v,
-                                                     double* __restrict__ p, double* partial, Scalars* sc, Criteria k) {
+                                                     double* __restrict__ p, double* partial, Scalars* sc, Criteria k,
+                                                     unsigned wait_ms) {
     if (!sc->bi_active) return;
     __shared__ double s_sum[BI_COLS];
     const double alpha = sc->bi_alpha, rho0 = sc->bi_rho;
@@ -2253,7 +2281,7 @@ __global__ void __launch_bounds__(BI_TPB) k_bi_omega(int N, double* __restrict__
             d[1] += tc * s[5 * i + c];
         }
     bi_columns(d, partial, 0);
-    if (!grid_barrier(&sc->orth_bar, gridDim.x, &sc->flags)) return;
+    if (!grid_barrier(sc, 1, wait_ms)) return;
     sum_columns<BI_TPB>(partial, 2, gridDim.x, s_sum);
     const double omega = s_sum[0] > 0 ? s_sum[1] / s_sum[0] : 0.0;
     double a[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -2269,7 +2297,7 @@ __global__ void __launch_bounds__(BI_TPB) k_bi_omega(int N, double* __restrict__
         }
     double* part2 = partial + 2 * (size_t)gridDim.x;
     bi_columns(a, part2, 0);
-    if (!grid_barrier(&sc->orth_bar, 2 * gridDim.x, &sc->flags)) return;
+    if (!grid_barrier(sc, 2, wait_ms)) return;
     sum_columns<BI_TPB>(part2, 6, gridDim.x, s_sum);
     const double rho = s_sum[5], beta = rho / rho0 * (alpha / omega);
     for (long i = i0; i < N; i += stride)

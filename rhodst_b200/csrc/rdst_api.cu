@@ -306,6 +306,8 @@ struct rdst_ctx {
     long ldv = 0;                   // stride between basis vectors (entries)
     DBuf<double> orth_part;         // partial sums of k_orth's blocks
     int orth_blocks = 0, sms = 0;   // blocks of k_orth that are resident together
+    unsigned wait_ms = 2000;        // limit of the solver kernels' waits
+    bool expired = false;           // one ran out in a step; until rdst_set_primitive
     DBuf<double> wv;                // FP64 Arnoldi vector that is orthogonalised before it is stored in Vf
     // discrete adjoint (allocated on first use)
     DBuf<double> a_fbar, a_qbbar, a_qbar, a_gbar, a_vval, a_hval, a_wbar, a_wbarb, a_ubarb, a_pbar;
@@ -1176,7 +1178,7 @@ static void ilu_apply_rec(rdst_ctx& c, const IluDev& P, const double* in, double
     const int threads = 32 * (c.rec_warps + 1);
     ilu_rec_instance<MT>(std::max(c.ilu_ml, c.ilu_mu), c.rec_tight, [&](auto* k) {
         k<<<c.n_parts, threads, c.rec_smem_bytes, c.s>>>(P, in, out, active, c.rec_stage_bytes, c.rec_y0_rows,
-                                                         c.rec_lb_rows, &c.sc.p->flags);
+                                                         c.rec_lb_rows, c.sc.p, c.wait_ms);
     });
 }
 // blocks of the fresh factors -> the records (the backward ones alone after
@@ -1446,7 +1448,8 @@ struct Ops {
             Scalars* sc = c.sc.p;
             double *rw = c.Vb.p, *part = c.orth_part.p;
             int n = N;
-            void* args[] = {&n, &c.rhs.p, &c.r.p, &rw, &c.t.p, &c.pv.p, &part, &sc};
+            unsigned wait_ms = c.wait_ms;
+            void* args[] = {&n, &c.rhs.p, &c.r.p, &rw, &c.t.p, &c.pv.p, &part, &sc, &wait_ms};
             coop(c, (const void*)k_bi_start, args);
         } else if (c.o.solver != SOLVER_GMRES) {
             CK(cudaMemcpyAsync(c.r.p, c.rhs.p, sizeof(double) * c.nvec(), cudaMemcpyDeviceToDevice, s));
@@ -1459,15 +1462,16 @@ struct Ops {
         Timed tm(c, KS_ORTH);
         long n = c.nvec(), ldv = c.ldv;
         double* part = c.orth_part.p;
+        unsigned wait_ms = c.wait_ms;
         if constexpr (std::is_same<VT, double>::value) {
             const int nb = (int)std::min<long>(c.orth_blocks, nblk((n + 3) / 4, ORTH_PIECES));
-            void* args[] = {&n, &nv, &V, &ldv, &w, &vout, &part, &sc, &m};
+            void* args[] = {&n, &nv, &V, &ldv, &w, &vout, &part, &sc, &m, &wait_ms};
             CK(cudaLaunchCooperativeKernel((const void*)k_orth<VT>, dim3(nb), dim3(ORTH_TPB), args,
                                            sizeof(double) * nv * nv, c.s));
         } else {
             int nbv = red_blocks(n);
             const int nb = std::min(c.orth_blocks, (nbv + 1) / 2);
-            void* args[] = {&n, &nv, &V, &ldv, &w, &vout, &part, &sc, &m, &nbv};
+            void* args[] = {&n, &nv, &V, &ldv, &w, &vout, &part, &sc, &m, &nbv, &wait_ms};
             CK(cudaLaunchCooperativeKernel((const void*)k_orth_cgs2<VT>, dim3(nb), dim3(CGS_TPB), args, 0, c.s));
         }
         count_launch();
@@ -1522,11 +1526,12 @@ struct Ops {
         Criteria k = criteria(c);
         precond(c, c.t.p, c.ph.p, act);                       // t holds p
         spmv(c, c.ph.p, c.pv.p, nullptr, act);                // v = A ph
-        void* a1[] = {&N, &rw, &c.r.p, &c.pv.p, &c.s2.p, &part, &sc};
+        unsigned wait_ms = c.wait_ms;
+        void* a1[] = {&N, &rw, &c.r.p, &c.pv.p, &c.s2.p, &part, &sc, &wait_ms};
         coop(c, (const void*)k_bi_alpha, a1);
         precond(c, c.s2.p, c.sh.p, act);
         spmv(c, c.sh.p, t2, nullptr, act);
-        void* a2[] = {&N, &c.dx.p, &c.r.p, &c.ph.p, &c.sh.p, &c.s2.p, &t2, &rw, &c.pv.p, &c.t.p, &part, &sc, &k};
+        void* a2[] = {&N, &c.dx.p, &c.r.p, &c.ph.p, &c.sh.p, &c.s2.p, &t2, &rw, &c.pv.p, &c.t.p, &part, &sc, &k, &wait_ms};
         coop(c, (const void*)k_bi_omega, a2);
     }
     static Criteria criteria(const rdst_ctx& c) {
@@ -1680,8 +1685,19 @@ __global__ void k_init_scalars(Scalars* sc, double time, double dt, double co) {
     sc->orth_bar = sc->orth_out = 0;     // left behind by a launch whose barrier expired
 }
 
+__global__ void k_clear_expired(Scalars* sc) {
+    if (threadIdx.x != 0) return;
+    sc->flags &= ~4;
+    sc->orth_bar = sc->orth_out = 0;
+}
+void clear_expired(rdst_ctx& c, Scalars* sc) {
+    k_clear_expired<<<1, 1, 0, c.s>>>(sc);
+    CKL();
+}
+
 // timeDST::initialize (timeDST.C:67-208) on the freshly set state
 void initialize_time(rdst_ctx& c) {
+    c.expired = false;
     k_init_time<<<nblk(c.N, TPB), TPB, 0, c.s>>>(c.N, c.prim.p, c.th, c.rhoOld.p, c.eOld.p, c.courantF.p, c.o.initial_co);
     CKL();
     k_init_scalars<<<1, 1, 0, c.s>>>(c.sc.p, c.o.start_time, c.o.delta_t, c.o.initial_co);
@@ -1768,6 +1784,14 @@ void launch_graph(rdst_ctx& c, rdst_ctx::Graph& g) {
     c.launches += g.launches;
 }
 
+const char* const EXPIRED_MSG =
+    "a bounded device wait expired (a copy of the ILU apply, or a grid barrier of the orthogonalisation or of BiCGStab)";
+void report_expired(rdst_ctx& c, int flags) {
+    if (!(flags & 4)) return;
+    c.expired = true;
+    throw TimeoutError(EXPIRED_MSG);
+}
+
 template <typename MT>
 void run_steps(rdst_ctx& c, int n, rdst_step_report* host_reps) {
     cudaStream_t s = c.s;
@@ -1851,7 +1875,7 @@ void run_steps(rdst_ctx& c, int n, rdst_step_report* host_reps) {
     CK(cudaMemcpyAsync(&flags, &c.sc.p->flags, sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     c.collect_events();
-    if (flags & 4) throw TimeoutError("a bounded wait of the ILU apply expired (bulk copy not completed)");
+    report_expired(c, flags);
     if (flags & 2) throw std::domain_error("non-physical state (NaN or non-positive rho/p) after the update");
 }
 
@@ -2023,7 +2047,7 @@ void run_dual_steps(rdst_ctx& c, int n, rdst_step_report* host_reps) {
     CK(cudaMemcpyAsync(&flags, &c.sc.p->flags, sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     c.collect_events();
-    if (flags & 4) throw TimeoutError("a bounded wait of the ILU apply expired (bulk copy not completed)");
+    report_expired(c, flags);
     if (flags & 2) throw std::domain_error("non-physical state (NaN or non-positive rho/p) after the update");
 }
 
@@ -2253,6 +2277,15 @@ void adj_prec(rdst_ctx& c, const double* in, double* out) {
     CKL();
 }
 
+// flags of the outer solve and of the inner cycles and applies
+int adj_flags(rdst_ctx& c) {
+    int f[2] = {0, 0};
+    CK(cudaMemcpyAsync(&f[0], &c.a_sc.p->flags, sizeof(int), cudaMemcpyDeviceToHost, c.s));
+    CK(cudaMemcpyAsync(&f[1], &c.sc.p->flags, sizeof(int), cudaMemcpyDeviceToHost, c.s));
+    CK(cudaStreamSynchronize(c.s));
+    return f[0] | f[1];
+}
+
 // Flexible GMRES(m), right preconditioned by adj_prec, for
 // (dR/dW)^T psi = rhs; its Hessenberg lives in its own Scalars (the inner
 // cycles use the step's).  Returns the number of outer iterations; res0 /
@@ -2266,6 +2299,7 @@ int adj_solve(rdst_ctx& c, const double* rhs, double* psi, double rel_tol, int m
     double* Vb = c.a_V.p;
     double* Zb = c.a_Z.p;
     CK(cudaMemsetAsync(psi, 0, sizeof(double) * n, s));
+    clear_expired(c, sc);
     int iters = 0;
     res0 = 0.0;
     res = 0.0;
@@ -2277,7 +2311,7 @@ int adj_solve(rdst_ctx& c, const double* rhs, double* psi, double rel_tol, int m
         Ops<MT>::template orth<double>(c, sc, Vb, 0, Vb, Vb, m);
         double beta = 0.0;
         CK(cudaMemcpyAsync(&beta, &sc->beta, sizeof(double), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
+        if (adj_flags(c) & 4) break;
         res = beta;
         if (cyc == 0) res0 = res;
         if (res <= rel_tol * res0 || res == 0.0) break;
@@ -2841,6 +2875,18 @@ RDST_API rdst_status rdst_set_profile(rdst_ctx* c, int32_t on) {
     }
 }
 
+RDST_API rdst_status rdst_set_wait_limit(rdst_ctx* c, double seconds) {
+    if (!c || !(seconds >= 0.0 && seconds <= 3600.0)) return RDST_ERR_ARG;
+    return guarded(c, [&] {
+        CK(cudaStreamSynchronize(c->s));
+        c->collect_events();
+        const unsigned ms = (unsigned)std::ceil(seconds * 1e3);
+        if (ms == c->wait_ms) return;
+        c->wait_ms = ms;
+        c->reset_graphs();      // the limit is an argument of the captured kernels
+    });
+}
+
 RDST_API rdst_status rdst_objective_gradient(rdst_ctx* c, const rdst_objective* ob, double* J, double force[3],
                                              double* dJdW, double dJdU[3]) {
     if (!c || !ob || !c->state_set) return RDST_ERR_ARG;
@@ -2932,11 +2978,16 @@ RDST_API rdst_status rdst_adjoint(rdst_ctx* c, const rdst_objective* ob, double 
         });
         CK(cudaMemcpyAsync(usum, c->a_u3.p + 8, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->s));
         CK(cudaEventRecord(e1, c->s));
-        CK(cudaStreamSynchronize(c->s));
+        const int flags = adj_flags(*c);
         float ms = 0;
         CK(cudaEventElapsedTime(&ms, e0, e1));
         c->ev_pool.push_back(e0);
         c->ev_pool.push_back(e1);
+        if (flags & 4) {
+            // the state is as it was: only a step's expired wait stays
+            if (!c->expired) { clear_expired(*c, c->sc.p); CK(cudaStreamSynchronize(c->s)); }
+            throw TimeoutError(EXPIRED_MSG);
+        }
         if (psi) field_to_caller(*c, c->a_psi.p, psi);
         if (rep) {
             rep->J = out[0];

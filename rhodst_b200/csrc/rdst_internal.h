@@ -77,7 +77,8 @@ struct Scalars {
     double nf;                 // linear solver normFactor
     double lin_initial[5], lin_final[5];
     int lin_iterations;
-    int flags;                 // bit0 bounding active, bit1 non-physical state
+    int flags;                 // bit0 bounding active, bit1 non-physical state, bit2 a bounded wait expired,
+                               // bit3 the solve stopped on maxIter
     int step_idx;              // report slot of the current step
     int converged;
     double rdt_min, rdt_max, dt_face_min;
@@ -86,7 +87,7 @@ struct Scalars {
     int gm_active, gm_used;
     double H[64 * 65], bh[65], cs[64], sn[64];
     double G[64 * 64];                  // V^T V of the cycle's basis
-    unsigned orth_bar, orth_out;        // grid barrier of k_orth (zero between launches)
+    unsigned orth_bar, orth_out;        // grid barrier of the cooperative kernels (zero between launches)
     // BiCGStab
     double bi_rho, bi_alpha;
     int bi_active;                      // 0 after the converged iteration
