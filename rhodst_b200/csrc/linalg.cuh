@@ -1458,10 +1458,7 @@ __device__ __forceinline__ void load4(const double* p, double (&o)[4]) {
     const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
     o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
 }
-__device__ __forceinline__ void load4(const float* p, double (&o)[4]) {
-    const float4 a = *reinterpret_cast<const float4*>(p);
-    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
-}
+
 // per-component sum |r_c| and the foam normFactor pieces
 __global__ void __launch_bounds__(RED_TPB) k_abs5(int N, const double* __restrict__ r, double* __restrict__ partial) {
     double a[5] = {0, 0, 0, 0, 0};
@@ -1549,39 +1546,37 @@ __global__ void k_solve_start(const double* __restrict__ partial, int nb, Scalar
 }
 
 // ---------------------------------------------------------------- GMRES
-// One Arnoldi vector's orthogonalisation in one cooperative launch (FP64
-// basis; k_orth_cgs2 for FP32).
-//
-// The basis is what this path reads (V: nv vectors, 4 or 8 bytes an entry),
-// so it is read twice, not three times as two classical Gram-Schmidt passes
-// with their own dot products would: the first pass takes h = V^T w and, in
-// the same read, e = V^T v of the newest basis vector v, the new column of
-// the Gram matrix G = V^T V.  The coefficients that a second pass would add,
-// V^T (w - V h), are then h - G h without touching V, which takes out what
-// the basis itself lacks in orthogonality; the second read subtracts c = 2 h - G h.  Rounding of w - V c
-// is amplified by |w| / |w - V c|, so where that ratio exceeds 100 a true
-// second pass follows (a branch that all blocks take together).
+// One Arnoldi vector's orthogonalisation in one cooperative launch: two
+// classical Gram-Schmidt passes, each with dots of its own (the coefficients of
+// the second formed from the Gram matrix of the basis instead would save a read
+// of it, but leave the basis less orthogonal, by |w| / |w - V h|: 4e-14 where two
+// passes leave 5e-16 at a ratio of 86).
 //
 // A launch per pass and one per sum costs more than the passes themselves up
 // to about 1e5 unknowns; the passes are therefore separated by a grid-wide
 // barrier (all blocks resident: cooperative launch), each block adding up
-// the blocks' partial sums by itself in the same order.  The second read
-// runs through the vectors backwards: what the first read last is still in
-// L2 (126 MB).  In the dot pass a thread takes four consecutive entries of
-// eight vectors, two groups of warps sharing the sixteen of a round (that
-// leaves registers for loads in flight); in the others two entries of all
-// vectors.  Vectors are padded to 64 entries of
-// zeros, so no load needs a test for the end.
+// the blocks' partial sums by itself in the same order.
 //
-// Per direction, mean of 20 (before: dots, update and dots, update and norm,
-// each with its own sum, then the Givens rotation and the scaling, ten
-// launches): 4 k cells 45 -> 13 us, 442 k 170 -> 88.
+// With a basis in FP32 (FP32 and BF16 Jacobians) the Arnoldi vector is rounded
+// to FP32 after every direction and in every preconditioner application, so a
+// last-bit difference in a coefficient is a difference of 1e-7 in the solve.
+// The kernel therefore keeps the sums of the separate launches it replaces to the
+// order of every addition, for both storages: red_blocks(n) "blocks" of 256
+// threads (a CTA takes two at a time, all of one SM's in turn), four entries a
+// thread per piece, the pieces in ascending order, the warps' tree, the eight
+// warps one after the other, then the blocks' sums as one block of 256 threads
+// adds them up.  Vectors are padded to 64 entries of zeros, so no load needs a
+// test for the end.  The loads of eight vectors at a time are issued together,
+// whatever their number (FP32, 1.2 M cells, mean of 20 directions: 230 -> 203 us;
+// keeping sixteen vectors in registers between the two uses spilled and was
+// slower).  It is bound by the three reads of the basis, on small meshes by the
+// barriers and the chain of loads between them.  Per direction, mean of 20,
+// FP64, against the ten launches of before (dots, update and dots, update and
+// norm, each with its own sum, then the rotation and the scaling): 4 k cells
+// 45 -> 20 us, 442 k 170 -> 124.
 constexpr int ORTH_TPB = 512;
-constexpr int ORTH_PIECES = ORTH_TPB / 2;       // four-entry pieces a block takes at a time
-constexpr int ORTH_NV = 8;                      // basis vectors whose dots a thread holds at once
+constexpr int ORTH_NV = 16;                     // basis vectors whose dots a thread holds at once
 constexpr int ORTH_MAXV = 64;                   // GMRES directions at most
-constexpr int ORTH_COLS = 3 * ORTH_MAXV + 3;    // partial sums per block: h, e, |w|^2, |w|^2 after each pass, h of the second
-constexpr double ORTH_AGAIN = 1.0e-4;           // |w - V c|^2 below this part of |w|^2: a second pass
 
 // f(integral_constant<cnt>) for 1 <= cnt <= MAXC: the loads of a round are all
 // issued before the first is used only if their number is known
@@ -1595,7 +1590,12 @@ __device__ __forceinline__ void with_count(int cnt, F&& f) {
 // four consecutive entries as they are stored
 template <typename VT> struct Raw4;
 template <> struct Raw4<float> { using T = float4; };
+struct __align__(16) Doubles4 { double2 a, b; };
+template <> struct Raw4<double> { using T = Doubles4; };
 __device__ __forceinline__ void raw4(const float4& a, double (&o)[4]) { o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; }
+__device__ __forceinline__ void raw4(const Doubles4& v, double (&o)[4]) { o[0] = v.a.x; o[1] = v.a.y; o[2] = v.b.x; o[3] = v.b.y; }
+
+__device__ __forceinline__ void copy4(const double (&a)[4], double (&o)[4]) { o[0] = a[0]; o[1] = a[1]; o[2] = a[2]; o[3] = a[3]; }
 
 // the warp's sums of 16 values: lane l gets that of a[l / 2]
 __device__ __forceinline__ double warp_sum16(double (&a)[16]) {
@@ -1750,171 +1750,6 @@ __device__ __forceinline__ void grid_leave(Scalars* sc) {
     if (threadIdx.x == 0 && atomicAdd(&sc->orth_out, 1u) == gridDim.x - 1) { sc->orth_bar = 0; sc->orth_out = 0; }
 }
 
-// Orthogonalise w against V_0 .. V_{nv-1}, beta = |w|, and (vout) V_nv =
-// w / beta; H(:, nv-1), its Givens rotation and bh by the first block.  nv 0
-// starts a cycle: beta = |w|, V_0 = w / beta, bh = beta e_0.  w may be vout
-// (FP64 basis).  partial: ORTH_COLS columns of gridDim.x doubles.
-template <typename VT>
-__global__ void __launch_bounds__(ORTH_TPB, 1)
-    k_orth(long n, int nv, const VT* V, long ldv, double* w, VT* vout, double* partial, Scalars* sc, int m,
-           unsigned wait_ms) {
-    if (nv > 0 ? !sc->gm_active : (sc->flags & 4) != 0) return;
-    constexpr int NW = ORTH_TPB / 32;
-    __shared__ double s_red[NW][17];
-    __shared__ double s_col[2 * ORTH_MAXV + 1], s_c[ORTH_MAXV], s_b[2];
-    extern __shared__ double s_G[];                 // [nv][nv]
-    const int nb = gridDim.x, blk = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int group = tid / ORTH_PIECES;            // which eight vectors of sixteen, which half of a piece
-    const long nc = (n + 3) / 4, stride = (long)nb * ORTH_PIECES, c0 = (long)blk * ORTH_PIECES + tid % ORTH_PIECES;
-    const bool single = nc <= stride;               // one piece a thread pair: w stays in registers
-    const int i = nv - 1;
-    for (int q = tid; q < i * i; q += ORTH_TPB) s_G[(q / i) * nv + q % i] = sc->G[(q / i) * ORTH_MAXV + q % i];
-    unsigned round = 0;
-    auto barrier = [&] { return grid_barrier(sc, ++round, wait_ms); };
-    // sum of x over the block into column col
-    auto block_col = [&](double x, int col) {
-        x = warp_sum(x);
-        if (lane == 0) s_red[wid][16] = x;
-        __syncthreads();
-        if (tid == 0) {
-            double s = 0;
-            for (int q = 0; q < NW; ++q) s += s_red[q][16];
-            partial[(size_t)col * nb + blk] = s;
-        }
-        __syncthreads();
-    };
-    double keep[2] = {0, 0};                        // single: this thread's half of w
-    // V^T w into columns col.., V^T V_i into columns ecol.. (if >= 0)
-    auto dots = [&](int col, int ecol) {
-        for (int jb = 0; jb < nv; jb += 2 * ORTH_NV) {
-            const int j0 = jb + ORTH_NV * group, cnt = min(ORTH_NV, nv - j0);
-            double acc[16];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) acc[q] = 0.0;
-            auto piece = [&](long i0, auto full) {
-                double wv[4], vi[4];
-                load4(w + i0, wv);
-                load4(V + i * ldv + i0, vi);
-#pragma unroll
-                for (int j = 0; j < ORTH_NV; ++j)
-                    if (decltype(full)::value || j < cnt) {
-                        double v[4];
-                        load4(V + (j0 + j) * ldv + i0, v);
-                        acc[j] += v[0] * wv[0] + v[1] * wv[1] + v[2] * wv[2] + v[3] * wv[3];
-                        acc[8 + j] += v[0] * vi[0] + v[1] * vi[1] + v[2] * vi[2] + v[3] * vi[3];
-                    }
-            };
-            if (cnt >= ORTH_NV) for (long c = c0; c < nc; c += stride) piece(4 * c, std::true_type{});
-            else if (cnt > 0) for (long c = c0; c < nc; c += stride) piece(4 * c, std::false_type{});
-            const double s = warp_sum16(acc);
-            if ((lane & 1) == 0) s_red[wid][lane >> 1] = s;
-            __syncthreads();
-            if (tid < 32) {
-                const int g = tid >> 4, q = tid & 15, j = jb + ORTH_NV * g + (q & 7);
-                if (j < nv && (q < 8 || ecol >= 0)) {
-                    double t = 0;
-                    for (int k = 0; k < NW / 2; ++k) t += s_red[g * (NW / 2) + k][q];
-                    partial[(size_t)((q < 8 ? col : ecol) + j) * nb + blk] = t;
-                }
-            }
-            __syncthreads();
-        }
-    };
-    // w -= V c, pieces in descending order; |w|^2 into column col
-    auto subtract = [&](const double* c, int col) {
-        double nrm = 0.0;
-        for (long p = c0 < nc ? c0 + (nc - 1 - c0) / stride * stride : -1; p >= 0; p -= stride) {
-            const long i0 = 4 * p + 2 * group;
-            double a[2];
-            if (single) { a[0] = keep[0]; a[1] = keep[1]; }
-            else load2(w + i0, a);
-            orth_subtract(V, ldv, nv, c, i0, a);
-            nrm += a[0] * a[0] + a[1] * a[1];
-            if (single) { keep[0] = a[0]; keep[1] = a[1]; }
-            store2(w, i0, n, a);
-        }
-        block_col(nrm, col);
-    };
-    // ---- dots: h, e and |w|^2
-    {
-        double ww = 0.0;
-        for (long c = c0; c < nc; c += stride) {
-            double a[2];
-            load2(w + 4 * c + 2 * group, a);
-            ww += a[0] * a[0] + a[1] * a[1];
-            if (single) { keep[0] = a[0]; keep[1] = a[1]; }
-        }
-        block_col(ww, 2 * nv);
-        dots(0, nv);
-    }
-    if (!barrier()) return;
-    sum_columns<ORTH_TPB>(partial, 2 * nv + 1, nb, s_col);
-    double beta2 = s_col[2 * nv];
-    const double ww = beta2;
-    if (nv > 0) {
-        if (tid < nv) {
-            const double e = s_col[nv + tid];
-            s_G[tid * nv + i] = e;
-            s_G[i * nv + tid] = e;
-            if (blk == 0) { sc->G[tid * ORTH_MAXV + i] = e; sc->G[i * ORTH_MAXV + tid] = e; }
-        }
-        __syncthreads();
-        if (tid < nv) {
-            double s = 2.0 * s_col[tid];
-            for (int k = 0; k < nv; ++k) s -= s_G[tid * nv + k] * s_col[k];
-            s_c[tid] = s;
-        }
-        __syncthreads();
-        subtract(s_c, 2 * nv + 1);
-        if (!barrier()) return;
-        sum_columns<ORTH_TPB>(partial + (size_t)(2 * nv + 1) * nb, 1, nb, s_b);
-        beta2 = s_b[0];
-        if (beta2 < ORTH_AGAIN * ww) {
-            // w lay almost in the basis: a second pass with dots of its own
-            dots(2 * nv + 2, -1);
-            if (!barrier()) return;
-            sum_columns<ORTH_TPB>(partial + (size_t)(2 * nv + 2) * nb, nv, nb, s_col);
-            subtract(s_col, 3 * nv + 2);
-            if (tid < nv) s_c[tid] += s_col[tid];
-            if (!barrier()) return;
-            sum_columns<ORTH_TPB>(partial + (size_t)(3 * nv + 2) * nb, 1, nb, s_b + 1);
-            beta2 = s_b[1];
-        }
-    }
-    const double beta = sqrt(beta2);
-    if (vout && beta != 0.0) {
-        for (long c = c0; c < nc; c += stride) {
-            const long i0 = 4 * c + 2 * group;
-            double a[2];
-            if (single) { a[0] = keep[0]; a[1] = keep[1]; }
-            else load2(w + i0, a);
-            a[0] /= beta;
-            a[1] /= beta;
-            store2(vout, i0, n, a);
-        }
-    }
-    if (blk == 0) {
-        if (nv == 0) gm_start(sc, beta);
-        else gm_rotate(sc, s_c, s_col, s_col + ORTH_MAXV, i, m, beta);
-    }
-    grid_leave(sc);
-}
-
-// The same for a basis stored in FP32 (FP32 and BF16 Jacobians), by two
-// classical passes with dots of their own: there the Arnoldi vector is rounded
-// to FP32 after every direction and in every preconditioner application, so a
-// last-bit difference in a coefficient is a difference of 1e-7 in the solve.
-// This kernel therefore keeps the sums of the launches it replaces to the
-// order of every addition: red_blocks(n) "blocks" of 256 threads (a CTA takes
-// two at a time, all of one SM's in turn), four entries a thread per piece,
-// the pieces in ascending order, the warps' tree, the eight warps one after
-// the other, then the blocks' sums as one block of 256 threads adds them up.
-// The loads of eight vectors at a time are issued together, whatever their
-// number (1.2 M cells, mean of 20 directions: 230 -> 203 us; keeping sixteen
-// vectors in registers between the two uses spilled and was slower).
-constexpr int CGS_TPB = 512;
-constexpr int CGS_NV = 16;                      // basis vectors whose dots a thread holds at once
-
 // sum of part[0..nb) as one block of RED_TPB threads takes it: thread t the
 // entries t, t + RED_TPB, .., a tree over each warp, a tree over the warps;
 // by one warp, all lanes the result
@@ -1951,13 +1786,22 @@ __device__ __forceinline__ double sum_as_block(const double* part, int nb) {
     return v;
 }
 
-template <typename VT>
-__global__ void __launch_bounds__(CGS_TPB, 1)
+// Orthogonalise w against V_0 .. V_{nv-1}, beta = |w|, and (vout) V_nv =
+// w / beta; H(:, nv-1), its Givens rotation and bh by the first block.  nv 0
+// starts a cycle: beta = |w|, V_0 = w / beta, bh = beta e_0.  w may be vout
+// (FP64 basis).  nbv: red_blocks(n); partial: 2 nv + 1 columns of nbv doubles.
+//
+// SPLIT, where every "block" can have a CTA of its own (then a thread has at most
+// one piece): both halves of the CTA hold the same pieces of w, in registers from
+// the first pass to the last, and share the basis vectors of the dots between
+// them; w is not written (FP64, 4 k cells: 23.3 -> 20.4 us, 17 k: 29.3 -> 25.5).
+template <typename VT, bool SPLIT>
+__global__ void __launch_bounds__(ORTH_TPB, 1)
     k_orth_cgs2(long n, int nv, const VT* V, long ldv, double* w, VT* vout, double* partial, Scalars* sc, int m, int nbv,
                 unsigned wait_ms) {
     if (nv > 0 ? !sc->gm_active : (sc->flags & 4) != 0) return;
     constexpr int NWB = RED_TPB / 32;               // warps of a virtual block
-    __shared__ double s_red[CGS_TPB / 32][CGS_NV];
+    __shared__ double s_red[ORTH_TPB / 32][ORTH_NV];
     __shared__ double s_h[2][ORTH_MAXV], s_rot[2][ORTH_MAXV], s_b;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = tid / RED_TPB, t = tid % RED_TPB;
     const int i = nv - 1;
@@ -1967,11 +1811,12 @@ __global__ void __launch_bounds__(CGS_TPB, 1)
     // every virtual block of this CTA, two at a time (f is called by all
     // threads, with a block past the end for a CTA's odd last one)
     auto blocks = [&](auto f) {
-        for (int b0 = 2 * blockIdx.x; b0 < nbv; b0 += 2 * gridDim.x) f(b0 + g);
+        if (SPLIT) f((int)blockIdx.x);
+        else for (int b0 = 2 * blockIdx.x; b0 < nbv; b0 += 2 * gridDim.x) f(b0 + g);
     };
     // the block's sums of cnt values into columns col.. : a tree over each
     // warp, the warps one after the other
-    auto block_sums = [&](double (&acc)[CGS_NV], int cnt, int col, int vb) {
+    auto block_sums = [&](double (&acc)[ORTH_NV], int cnt, int col, int vb) {
         const double s = warp_sum16(acc);
         if ((lane & 1) == 0) s_red[wid][lane >> 1] = s;
         __syncthreads();
@@ -1993,6 +1838,11 @@ __global__ void __launch_bounds__(CGS_TPB, 1)
             for (int e = 0; e < 4 && i0 + e < n; ++e) w[i0 + e] = a[e];
         }
     };
+    double keep[4] = {0, 0, 0, 0};                  // SPLIT: the thread's piece of w
+    if (SPLIT && nv > 0) {
+        const long c = (long)blockIdx.x * RED_TPB + t;
+        if (c < nc) load4(w + 4 * c, keep);
+    }
     // entries k.. of C vectors from V_j on, as they are stored
     auto fetch = [&](int j, long k, auto& x, auto cnt) {
 #pragma unroll
@@ -2020,19 +1870,26 @@ __global__ void __launch_bounds__(CGS_TPB, 1)
     // dots with vectors jb.. < nv into columns col + jb..; with `coef` the
     // vector is first reduced by coef_j V_j over all j (once, jb 0)
     auto dots = [&](int col, const double* coef) {
-        for (int jb = 0; jb < nv; jb += CGS_NV) {
-            const int cnt = min(CGS_NV, nv - jb);
+        const int per = SPLIT && nv <= ORTH_NV ? ORTH_NV / 2 : ORTH_NV;      // vectors of a group at once
+        for (int j0 = 0; j0 < nv; j0 += SPLIT ? 2 * per : per) {
+            const int jb = SPLIT ? j0 + per * g : j0;
+            const int cnt = min(per, nv - jb);
             blocks([&](int vb) {
-                double acc[CGS_NV];
+                double acc[ORTH_NV];
 #pragma unroll
-                for (int q = 0; q < CGS_NV; ++q) acc[q] = 0.0;
+                for (int q = 0; q < ORTH_NV; ++q) acc[q] = 0.0;
                 if (vb < nbv)
                     for (long c = (long)vb * RED_TPB + t; c < nc; c += stride) {
                         double a[4];
-                        load4(w + 4 * c, a);
-                        if (coef && jb == 0) {
-                            reduce(coef, 4 * c, a);
-                            store4(4 * c, a);
+                        if (SPLIT) {
+                            if (coef && j0 == 0) reduce(coef, 4 * c, keep);
+                            copy4(keep, a);
+                        } else {
+                            load4(w + 4 * c, a);
+                            if (coef && j0 == 0) {
+                                reduce(coef, 4 * c, a);
+                                store4(4 * c, a);
+                            }
                         }
                         auto some = [&](auto from, auto tag) {
                             constexpr int F = decltype(from)::value, C = decltype(tag)::value;
@@ -2046,13 +1903,13 @@ __global__ void __launch_bounds__(CGS_TPB, 1)
                             }
                         };
                         using Zero = std::integral_constant<int, 0>;
-                        using Half = std::integral_constant<int, CGS_NV / 2>;
-                        if (cnt >= CGS_NV / 2) {
+                        using Half = std::integral_constant<int, ORTH_NV / 2>;
+                        if (cnt >= ORTH_NV / 2) {
                             some(Zero(), Half());
-                            if (cnt > CGS_NV / 2)
-                                with_count<CGS_NV / 2>(cnt - CGS_NV / 2, [&](auto tag) { some(Half(), tag); });
-                        } else {
-                            with_count<CGS_NV / 2>(cnt, [&](auto tag) { some(Zero(), tag); });
+                            if (cnt > ORTH_NV / 2)
+                                with_count<ORTH_NV / 2>(cnt - ORTH_NV / 2, [&](auto tag) { some(Half(), tag); });
+                        } else if (cnt > 0) {
+                            with_count<ORTH_NV / 2>(cnt, [&](auto tag) { some(Zero(), tag); });
                         }
                     }
                 block_sums(acc, cnt, col + jb, vb);
@@ -2062,7 +1919,8 @@ __global__ void __launch_bounds__(CGS_TPB, 1)
     double beta;
     if (nv == 0) {
         // |w|^2 entry by entry, the warps' sums by a tree
-        blocks([&](int vb) {
+        blocks([&](int block) {
+            const int vb = SPLIT && g ? nbv : block;
             double acc = 0.0;
             if (vb < nbv)
                 for (long k = (long)vb * RED_TPB + t; k < n; k += stride) {
@@ -2088,7 +1946,7 @@ __global__ void __launch_bounds__(CGS_TPB, 1)
         double* part1 = partial + (size_t)nv * nbv;
         double* part2 = partial + 2 * (size_t)nv * nbv;
         auto sums = [&](const double* part, double* out) {
-            for (int j = wid; j < nv; j += CGS_TPB / 32) {
+            for (int j = wid; j < nv; j += ORTH_TPB / 32) {
                 const double s = sum_as_block(part + (size_t)j * nbv, nbv);
                 if (lane == 0) out[j] = s;
             }
@@ -2101,18 +1959,23 @@ __global__ void __launch_bounds__(CGS_TPB, 1)
         if (!barrier()) return;
         sums(part1, s_h[1]);
         blocks([&](int vb) {
-            double acc[CGS_NV];
+            double acc[ORTH_NV];
 #pragma unroll
-            for (int q = 0; q < CGS_NV; ++q) acc[q] = 0.0;
+            for (int q = 0; q < ORTH_NV; ++q) acc[q] = 0.0;
             if (vb < nbv)
                 for (long c = (long)vb * RED_TPB + t; c < nc; c += stride) {
                     double a[4];
-                    load4(w + 4 * c, a);
-                    reduce(s_h[1], 4 * c, a);
-                    store4(4 * c, a);
+                    if (SPLIT) {
+                        reduce(s_h[1], 4 * c, keep);
+                        copy4(keep, a);
+                    } else {
+                        load4(w + 4 * c, a);
+                        reduce(s_h[1], 4 * c, a);
+                        store4(4 * c, a);
+                    }
                     acc[0] += a[0] * a[0] + a[1] * a[1] + a[2] * a[2] + a[3] * a[3];
                 }
-            block_sums(acc, 1, 2 * nv, vb);
+            block_sums(acc, SPLIT && g ? 0 : 1, 2 * nv, vb);
         });
         if (!barrier()) return;
         if (wid == 0) {
@@ -2126,10 +1989,11 @@ __global__ void __launch_bounds__(CGS_TPB, 1)
         blocks([&](int vb) {
             if (vb < nbv)
                 for (long c = (long)vb * RED_TPB + t; c < nc; c += stride)
-                    for (int hf = 0; hf < 2; ++hf) {
+                    for (int hf = SPLIT ? g : 0; hf < (SPLIT ? g + 1 : 2); ++hf) {
                         const long i0 = 4 * c + 2 * hf;
                         double a[2];
-                        load2(w + i0, a);
+                        if (SPLIT && nv > 0) { a[0] = hf ? keep[2] : keep[0]; a[1] = hf ? keep[3] : keep[1]; }
+                        else load2(w + i0, a);
                         a[0] /= beta;
                         a[1] /= beta;
                         store2(vout, i0, n, a);
@@ -2181,14 +2045,14 @@ __global__ void __launch_bounds__(ORTH_TPB, 2) k_gm_update(long n, int m, const 
 // ---------------------------------------------------------------- BiCGStab
 // The vector work between the preconditioner and matrix applications of an
 // iteration, in cooperative launches (a thread per cell, the sums over a
-// bounded grid barrier as in k_orth): two launches an iteration where dots,
+// bounded grid barrier as in k_orth_cgs2): two launches an iteration where dots,
 // their sums, the scalars, the updates, the residual sum and the check took
 // seventeen, each a few us on the meshes this solver is used on.  An iteration
 // after the converged one (bi_active 0) does nothing, so the host need not
 // wait for each check before it launches the next (run_steps).  RAE2822, 23,552
 // cells, steps of 7 to 12 iterations, a run of six: 12.2 -> 11.5 ms.
 constexpr int BI_TPB = 256;
-constexpr int BI_COLS = 6;
+constexpr int BI_COLS = 8;          // columns of partial sums
 
 template <int K>
 __device__ __forceinline__ void bi_columns(double (&x)[K], double* partial, int col) {
@@ -2269,7 +2133,7 @@ __global__ void __launch_bounds__(BI_TPB) k_bi_omega(int N, double* __restrict__
                                                      double* __restrict__ p, double* partial, Scalars* sc, Criteria k,
                                                      unsigned wait_ms) {
     if (!sc->bi_active) return;
-    __shared__ double s_sum[BI_COLS];
+    __shared__ double s_sum[6];
     const double alpha = sc->bi_alpha, rho0 = sc->bi_rho;
     const long i0 = (long)blockIdx.x * BI_TPB + threadIdx.x, stride = (long)gridDim.x * BI_TPB;
     double d[2] = {0.0, 0.0};

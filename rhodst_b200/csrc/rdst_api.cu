@@ -304,8 +304,8 @@ struct rdst_ctx {
     DBuf<unsigned char> rmask;      // held cells (internal order): zero residual, identity rows; empty: none
     DBuf<float> Vf;                 // GMRES basis when it is kept in FP32
     long ldv = 0;                   // stride between basis vectors (entries)
-    DBuf<double> orth_part;         // partial sums of k_orth's blocks
-    int orth_blocks = 0, sms = 0;   // blocks of k_orth that are resident together
+    DBuf<double> orth_part;         // partial sums of the cooperative kernels' blocks
+    int orth_blocks = 0, sms = 0;   // blocks of theirs that are resident together
     unsigned wait_ms = 2000;        // limit of the solver kernels' waits
     bool expired = false;           // one ran out in a step; until rdst_set_primitive
     DBuf<double> wv;                // FP64 Arnoldi vector that is orthogonalised before it is stored in Vf
@@ -1108,15 +1108,12 @@ void build(rdst_ctx& c, const rdst_mesh* mh) {
     } else if (o.solver == SOLVER_GMRES) { c.Vb.alloc((size_t)(o.n_directions + 1) * c.ldv); c.Vb.zero(s); }
     else { c.s2.alloc(n5); c.sh.alloc(n5); c.ph.alloc(n5); c.pv.alloc(n5); c.Vb.alloc(2 * n5); }
     {
-        int dev = 0, per = 0, per32 = 0;
+        int dev = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev));
-        const size_t sm = sizeof(double) * ORTH_MAXV * ORTH_MAXV;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_orth<double>, ORTH_TPB, sm));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per32, k_orth_cgs2<float>, CGS_TPB, 0));
-        c.orth_blocks = c.sms * std::max(1, std::min({1, per, per32}));
-        // partial sums: of k_orth's blocks, or two dots a direction and a norm of red_blocks(n)
-        c.orth_part.alloc(std::max((size_t)ORTH_COLS * c.orth_blocks, (size_t)(2 * ORTH_MAXV + 1) * red_blocks(n5)));
+        c.orth_blocks = c.sms;      // one an SM of every cooperative kernel (__launch_bounds__ at 512 and 256 threads)
+        // partial sums: two dots a direction and a norm of red_blocks(n), or of BiCGStab's blocks
+        c.orth_part.alloc(std::max((size_t)BI_COLS * c.orth_blocks, (size_t)(2 * ORTH_MAXV + 1) * red_blocks(n5)));
     }
     // limiter needs
     auto vk = [](Limiter l) { return l == LIM_VENKATAKRISHNAN; };
@@ -1456,24 +1453,19 @@ struct Ops {
         }
     }
     // w orthogonalised against V_0..V_{nv-1} and (vout) stored normalised, or
-    // (nv 0) the cycle's start; all blocks resident (k_orth)
+    // (nv 0) the cycle's start; all blocks resident (k_orth_cgs2)
     template <typename VT>
     static void orth(rdst_ctx& c, Scalars* sc, const VT* V, int nv, double* w, VT* vout, int m) {
         Timed tm(c, KS_ORTH);
         long n = c.nvec(), ldv = c.ldv;
         double* part = c.orth_part.p;
         unsigned wait_ms = c.wait_ms;
-        if constexpr (std::is_same<VT, double>::value) {
-            const int nb = (int)std::min<long>(c.orth_blocks, nblk((n + 3) / 4, ORTH_PIECES));
-            void* args[] = {&n, &nv, &V, &ldv, &w, &vout, &part, &sc, &m, &wait_ms};
-            CK(cudaLaunchCooperativeKernel((const void*)k_orth<VT>, dim3(nb), dim3(ORTH_TPB), args,
-                                           sizeof(double) * nv * nv, c.s));
-        } else {
-            int nbv = red_blocks(n);
-            const int nb = std::min(c.orth_blocks, (nbv + 1) / 2);
-            void* args[] = {&n, &nv, &V, &ldv, &w, &vout, &part, &sc, &m, &nbv, &wait_ms};
-            CK(cudaLaunchCooperativeKernel((const void*)k_orth_cgs2<VT>, dim3(nb), dim3(CGS_TPB), args, 0, c.s));
-        }
+        int nbv = red_blocks(n);
+        const bool split = nbv <= c.orth_blocks;
+        const int nb = split ? nbv : std::min(c.orth_blocks, (nbv + 1) / 2);
+        void* args[] = {&n, &nv, &V, &ldv, &w, &vout, &part, &sc, &m, &nbv, &wait_ms};
+        auto* k = split ? k_orth_cgs2<VT, true> : k_orth_cgs2<VT, false>;
+        CK(cudaLaunchCooperativeKernel((const void*)k, dim3(nb), dim3(ORTH_TPB), args, 0, c.s));
         count_launch();
     }
     // x += V y, H y = bh

@@ -86,7 +86,6 @@ struct Scalars {
     double beta;
     int gm_active, gm_used;
     double H[64 * 65], bh[65], cs[64], sn[64];
-    double G[64 * 64];                  // V^T V of the cycle's basis
     unsigned orth_bar, orth_out;        // grid barrier of the cooperative kernels (zero between launches)
     // BiCGStab
     double bi_rho, bi_alpha;
