@@ -863,7 +863,9 @@ __global__ void k_rec_meta(const RecGroup* __restrict__ grp, const RecMeta* __re
 // fills whole sectors of the record; the reads of the sliced stores are 6-row
 // pieces of lines that the neighbouring warps share.  L comes from the factor
 // store, U from A (from the factor store for rows whose own blocks take
-// updates, zero for a fill), backward first the pivot inverse.
+// updates, zero for a fill), backward first the pivot inverse.  There is no
+// factor store (lu null) after k_ilu_factor_rec: nf is 0 and no row's own blocks
+// take updates.
 template <typename MT>
 __global__ void __launch_bounds__(256) k_ilu_pack(int nf, int nb, SellMat<MT> A, const MT* __restrict__ lu,
                                                   const MT* __restrict__ dinv, IluDev P) {
@@ -895,12 +897,8 @@ __global__ void __launch_bounds__(256) k_ilu_pack(int nf, int nb, SellMat<MT> A,
         const int nk = k < 4 ? (int)((g.x >> (8 * k)) & 255u) : (int)nks[k];
         if (pos < nk) {
             const int f = lu_fid(r, back ? P.ml + k : k, ms);
-            const MT* src = lu + flat_e(f, 0);
-            if (back && !own_u) {
-                const int a = P.lu_src[f];
-                src = a >= 0 ? A.val + flat_e(a, 0) : nullptr;
-            }
-            copy(src, blk);
+            const int a = back && !own_u ? P.lu_src[f] : 0;
+            copy(back && !own_u ? (a >= 0 ? A.val + flat_e(a, 0) : nullptr) : lu + flat_e(f, 0), blk);
         }
         blk += nk;
     }

@@ -262,7 +262,7 @@ struct rdst_ctx {
     int n_slices = 0, n_slots = 0;
     DBuf<int> slice_off, slice_w, col;
     void* Aval = nullptr;
-    void* LUval = nullptr;
+    void* LUval = nullptr;              // sliced factor store (none with fac_rec)
     void* dinv = nullptr;
     size_t mt_size = 8;
     // ILU plan
@@ -627,8 +627,6 @@ void build_records(rdst_ctx& c, const Options& o, int nparts, const std::vector<
                 desc[i] = d;
             }
         if (ML <= ILU_FR_MAXQ) {
-            c.fr_trk.upload(trk, s);
-            c.fr_trt.upload(trt, s);
             c.fr_desc.upload(desc, s);
             c.ilu_direct = true;
             // every lower block in the matrix, and it updates the diagonal
@@ -642,6 +640,10 @@ void build_records(rdst_ctx& c, const Options& o, int nparts, const std::vector<
             c.fac_lbuf = c.fac_smem + 2 * (size_t)c.rec_lb_rows * row <= room;
             if (c.fac_lbuf) c.fac_smem += 2 * (size_t)c.rec_lb_rows * row;
             c.fac_rec = c.fac_rec && c.fac_smem <= (size_t)per_block - 256;
+            if (!c.fac_rec) {
+                c.fr_trk.upload(trk, s);
+                c.fr_trt.upload(trt, s);
+            }
         }
     }
     CK(cudaStreamSynchronize(s));
@@ -1083,7 +1085,7 @@ void build(rdst_ctx& c, const rdst_mesh* mh) {
     size_t mbytes = (size_t)c.n_slots * 32 * 25 * c.mt_size;
     CK(cudaMalloc(&c.Aval, mbytes));
     CK(cudaMemsetAsync(c.Aval, 0, mbytes, s));
-    if (factored) {
+    if (factored && !c.fac_rec) {       // k_ilu_factor_rec writes L into the records and reads U from A
         size_t lbytes = (size_t)c.n_slices * c.lu_slots * 32 * 25 * c.mt_size;
         CK(cudaMalloc(&c.LUval, lbytes));
         CK(cudaMemsetAsync(c.LUval, 0, lbytes, s));
