@@ -2048,7 +2048,10 @@ __global__ void __launch_bounds__(ORTH_TPB, 2) k_gm_update(long n, int m, const 
 // seventeen, each a few us on the meshes this solver is used on.  An iteration
 // after the converged one (bi_active 0) does nothing, so the host need not
 // wait for each check before it launches the next (run_steps).  RAE2822, 23,552
-// cells, steps of 7 to 12 iterations, a run of six: 12.2 -> 11.5 ms.
+// cells, steps of 7 to 12 iterations, a run of six: 12.2 -> 11.5 ms.  One CTA an
+// SM (the count shared with k_orth_cgs2) leaves bandwidth unused on large meshes,
+// but is still less than the launches it replaces took: 442 k cells 200 -> 134 us
+// an iteration, 1.2 M 436 -> 361.
 constexpr int BI_TPB = 256;
 constexpr int BI_COLS = 8;          // columns of partial sums
 

@@ -475,8 +475,12 @@ int lim_code(Limiter l) { return (int)l; }
 // holds at once the count is rounded to a whole number of such waves (a
 // partial last wave costs a whole extra chain: measured on the 1.2 M-cell
 // wing with the register apply, 784 parts took 23% longer than 592 or
-// 1184).  A wave is counted as eight CTAs an SM with the record apply (it
-// holds six, the rest follow as those end), four with the register apply.
+// 1184).  A wave is four CTAs an SM with the register apply.  With the record
+// apply it is counted as eight though six are resident: there a partial wave
+// costs little, since a CTA that ends makes room for the next one and the bytes
+// bound it (3.96 M cells FP32, us an apply: 1776 parts, two waves of six, 516;
+// 2072 524; 2368, the choice here, 495; 2664, three waves, 486; a step 40.9,
+// 42.1, 40.5, 40.2 ms), and another count is another preconditioner.
 int auto_ilu_parts(int N, Precision prec, bool bulk) {
     int dev = 0, sms = 0, per_sm = 0;
     CK(cudaGetDevice(&dev));
