@@ -172,13 +172,12 @@ def algorithmic_bytes(kind: str, N: int, F: int, S: int, precon: str, vb: int = 
         return 2 * (25 * S * Bk + 4 * Bk) + 25 * S * N
     if kind == "orth":
         # one launch of the orthogonalisation at the mean basis size J (the
-        # cycle's start and m directions): two passes over the J basis
-        # vectors with an fp64 basis, three with an fp32 one, and over w (fp64)
-        # a read for the dots, a read and a write per update, and the scaled
-        # copy into the basis
+        # cycle's start and m directions): three passes over the J basis
+        # vectors (dots, update and dots, update) and over w (fp64) a read for
+        # the dots, a read and a write per update, and the scaled copy into
+        # the basis
         J = m / 2.0
-        passes, updates = (2, 1) if vb == 8 else (3, 2)
-        return N * 5 * (passes * J * vb + 8 + 16 * updates + 8 + vb)
+        return N * 5 * (3 * J * vb + 8 + 16 * 2 + 8 + vb)
     return 0.0
 
 
