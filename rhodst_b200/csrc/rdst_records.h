@@ -42,7 +42,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -331,11 +331,12 @@ inline RecPlan rec_plan(int N, int nparts, const std::vector<int>& part_lvl0, co
             const int nt = (int)std::min<size_t>({8, std::max(1u, std::thread::hardware_concurrency()), ts.size() / 2048 + 1,
                                                   (size_t)nparts});
             std::vector<std::thread> th;
+            th.reserve(nt);             // nothing may throw past a running thread
             for (int k2 = 1; k2 < nt; ++k2) {
                 const int p0 = (int)((long)nparts * k2 / nt), p1 = (int)((long)nparts * (k2 + 1) / nt);
                 try {
                     th.emplace_back(fill, p0, p1);
-                } catch (const std::system_error&) {      // no thread to be had
+                } catch (const std::exception&) {         // no thread to be had, or no memory for one
                     fill(p0, p1);
                 }
             }
