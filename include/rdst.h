@@ -323,7 +323,9 @@ rdst_status rdst_partition_graph(int32_t n_cells, int32_t n_internal_faces,
  * rdst_kernel_stats: with the option "profile" "true", the library records
  * CUDA events around every launch of the named kernel class inside
  * rdst_step ("spmv", "precond", "flux", "assemble", "factor", "orth",
- * "update") and returns its launch count and summed device time.
+ * "update") and returns its launch count and summed device time (GMRES
+ * applies a "diagonal" preconditioner in the product's own launch, which
+ * counts as "spmv").
  * rdst_set_profile: switches that recording on or off for later steps
  * (the event records add device time of their own, so steps are timed
  * with it off).  No counterpart in the reference (instrumentation). */
