@@ -32,3 +32,21 @@ def test_routes_agree_on_prisms_and_tetrahedra(dims, parts, prec, tol):
         s.close()
     for a, b in zip(*out):
         assert np.abs(a - b).max() <= tol * np.abs(b).max()
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-11), ("fp32", 1e-5), ("bf16", 1e-5)])
+@pytest.mark.parametrize("fill,parts", [(1, 1), (1, 8), (2, 8)])
+def test_routes_agree_with_fill(fill, parts, prec, tol):
+    """Fill of one and two faces more (up to 6 and 12 blocks a side on quads):
+    rows that update blocks of their own, so the factorisations beside the record
+    one, their L and U packed into the records; chains of up to 160 levels."""
+    base = cases.forward_step_c1(preconditioner="ILUCp", n_directions=8).with_options(
+        **{"precision": prec, "ilu.parts": parts, "solvers.W.fillInLevel": fill})
+    out = []
+    for bulk in (True, False):
+        s = rhodst_b200.solver_for(base.with_options(**{"ilu.bulk": bulk}))
+        s.step(2)
+        out.append(s.conservative())
+        s.close()
+    for a, b in zip(*out):
+        assert np.abs(a - b).max() <= tol * np.abs(b).max()
