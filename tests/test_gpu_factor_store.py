@@ -6,6 +6,8 @@ and columns (an eighth more at the most: 32 bytes a block of 200), so against a
 context with the store and the register apply at most the records of the
 inverses and that eighth come on top: a store that is kept too is another six
 blocks a row."""
+import gc
+
 import pytest
 
 import rhodst_b200
@@ -20,6 +22,7 @@ def test_no_store_beside_the_records(prec, size):
     case = cases.swept_wing_c3(128, 40, 32, 16, precision=prec)
     used = {}
     for bulk in (False, True, False, True):     # the second pair: with the library's own memory in place
+        gc.collect()                            # contexts of earlier tests
         free = torch.cuda.mem_get_info()[0]
         s = rhodst_b200.solver_for(case.with_options(**{"ilu.bulk": bulk}))
         used[bulk] = free - torch.cuda.mem_get_info()[0]
